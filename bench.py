@@ -104,27 +104,29 @@ def make_inputs(gen, cfg, velocities=False):
 def m2l_flops_per_translation(p: int, kernel: str) -> float:
     """Flops (FMA = 2) of one directed M2L translation as the kernel runs it.
 
-    rotation (warp kernel, m >= 0 half basis): per degree k (K = k+1 terms)
-    four real swap products, each 2 flops per structurally nonzero entry of
-    its two (K x K) half-basis matrices (about half the entries: Pm[r][q] != 0
-    needs r + q + k even, Qm[r][q] != 0 needs r, q >= 1 and r + q + k odd),
-    plus 25K for phases and scaling; the axial translation 4 per (n, m, k)
-    term plus 4 per output; the lane reduction 2 per output; phases and
+    rotation (warp kernel, m >= 0 half basis): per degree k four real swap
+    products, 2 flops per structurally nonzero entry of their two half-basis
+    matrices (Pm[r][q] != 0 needs r + q + k even, Qm[r][q] != 0 needs r, q >= 1
+    and r + q + k odd), the second one on the rows and the third on the columns
+    m <= min(k, p - k) that the axial step couples; four phase products (6 per
+    order m >= 1), the two scalings of the coupled orders, the axial
+    translation 2 per real term, the column sums 2 per output; phases and
     geometry about 12(p+1) + 50.
     naive: 8 per complex term of sum_{n,m} (p-n+1)^2 (translate.rs:47-136).
     """
     if kernel == "naive":
         return 8.0 * sum((2 * n + 1) * (p - n + 1) ** 2 for n in range(p + 1))
-    h = (p + 1) * (p + 2) // 2
 
-    def nz(k):  # structural nonzeros of Pm and Qm of degree k
-        r = range(k + 1)
-        return (sum(1 for a in r for b in r if (a + b + k) % 2 == 0)
-                + sum(1 for a in r for b in r if a >= 1 and b >= 1 and (a + b + k) % 2 == 1))
+    def nz(k, rows, cols):  # structural nonzeros of Pm and Qm of degree k in rows < rows, columns < cols
+        return (sum(1 for a in range(rows) for b in range(cols) if (a + b + k) % 2 == 0)
+                + sum(1 for a in range(1, rows) for b in range(1, cols) if (a + b + k) % 2 == 1))
 
-    rot = sum(8 * nz(k) + 25 * (k + 1) for k in range(p + 1))
-    axial = sum(max(0, p - n - m + 1) for m in range(p + 1) for n in range(m, p + 1))
-    return rot + 4 * axial + 6 * h + 12 * (p + 1) + 50
+    fl = 12.0 * (p + 1) + 50
+    for k in range(p + 1):
+        n, c = k + 1, min(k, p - k) + 1
+        fl += 2 * (2 * nz(k, n, n) + nz(k, c, n) + nz(k, n, c)) + 24 * k + 2 * (2 * c - 1) + 2 * (2 * k + 1)
+        fl += sum(2 * (1 if m == 0 else 2) for m in range(c) for _ in range(m, p - k + 1))
+    return fl
 
 
 def p2p_flops(interactions: int) -> float:

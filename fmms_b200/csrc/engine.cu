@@ -117,8 +117,6 @@ struct BudgetScope {
     ~BudgetScope() { tl_budget = prev; }
 };
 
-int rot_moff_host(int k) { return 4 * (k * (k + 1) * (2 * k + 1) / 6); }
-
 int bits_for(uint64_t v) {
     int b = 0;
     while (b < 64 && (v >> b) != 0) ++b;
@@ -353,66 +351,6 @@ void build_swap(int p, std::vector<double>& sw) {
 }
 
 }  // namespace
-
-// Real half-basis forms of the swap matrices for the warp rotation M2L.
-void fmmx::make_rotw_tables(RotwTables& t) {
-    const int P = kRotwMaxP;
-    std::vector<double> sw;
-    build_swap(P, sw);
-    auto boff = [](int j) { return j == 0 ? 0 : j * (4 * j * j - 1) / 3; };
-    t.mats.assign(rot_moff_host(P + 1), 0.0);
-    for (int k = 0; k <= P; ++k) {
-        const int nb = 2 * k + 1, off = boff(k), kk = (k + 1) * (k + 1);
-        auto B = [&](int r, int c) { return sw[off + (r + k) * nb + (c + k)]; };
-        double* Pm = t.mats.data() + rot_moff_host(k);
-        double* Qm = Pm + kk;
-        double* PT = Qm + kk;
-        double* QT = PT + kk;
-        for (int r = 0; r <= k; ++r)
-            for (int c = 0; c <= k; ++c) {
-                const double sg = (c & 1) ? -1.0 : 1.0;
-                if (c == 0) {
-                    Pm[r * (k + 1)] = B(r, 0);
-                    Qm[r * (k + 1)] = B(r, 0);
-                    PT[r * (k + 1)] = B(0, r);
-                    QT[r * (k + 1)] = B(0, r);
-                } else {
-                    Pm[r * (k + 1) + c] = B(r, c) + sg * B(r, -c);
-                    Qm[r * (k + 1) + c] = B(r, c) - sg * B(r, -c);
-                    PT[r * (k + 1) + c] = B(c, r) + sg * B(-c, r);
-                    QT[r * (k + 1) + c] = B(c, r) - sg * B(-c, r);
-                }
-            }
-    }
-    std::vector<double> f(2 * P + 1, 1.0);
-    for (int i = 1; i <= 2 * P; ++i) f[i] = f[i - 1] * (double)i;
-    t.fact = f;
-    const int nh = P * (P + 1) / 2 + P + 1;
-    t.fm.assign(nh, 0.0);
-    t.ifm.assign(nh, 0.0);
-    for (int n = 0; n <= P; ++n)
-        for (int m = 0; m <= n; ++m) {
-            const int h = n * (n + 1) / 2 + m;
-            t.fm[h] = f[n - m] * f[n + m];
-            t.ifm[h] = 1.0 / t.fm[h];
-        }
-}
-
-bool fmmx::rotw_tables_check(const RotwTables& t) {
-    for (int k = 0; k <= kRotwMaxP; ++k) {
-        const int n = k + 1;
-        const double* m = t.mats.data() + rot_moff_host(k);  // P, Q, PT, QT
-        for (int r = 0; r < n; ++r)
-            for (int q = 0; q < n; ++q) {
-                const bool p_nz = ((r + q + k) & 1) == 0;
-                const bool q_nz = r >= 1 && q >= 1 && ((r + q + k) & 1) == 1;
-                if (!p_nz && (m[r * n + q] != 0.0 || m[2 * n * n + r * n + q] != 0.0)) return false;
-                if (q >= 1 && !q_nz && (m[n * n + r * n + q] != 0.0 || m[3 * n * n + r * n + q] != 0.0))
-                    return false;
-            }
-    }
-    return true;
-}
 
 namespace {
 
@@ -1197,16 +1135,6 @@ fmmx_status fmmx_create(const fmmx_config* cfg, fmmx_ctx** out) {
     if (ctx->nsm < 1) ctx->nsm = 1;
     g_nsm = ctx->nsm;
     make_tables(ctx->tab);
-    {
-        RotwTables rt;
-        make_rotw_tables(rt);
-        if (!rotw_tables_check(rt)) {  // cannot happen: the tables are fixed numbers
-            fmmx_destroy(ctx);
-            return FMMX_DEVICE_ERROR;
-        }
-        rotw_upload_f64(rt, ctx->stream);
-        rotw_upload_f32(rt, ctx->stream);
-    }
     upload_tables_exact(ctx->tab, ctx->stream);
     upload_tables_m2l(ctx->tab, ctx->stream);
     upload_tables_sweeps(ctx->tab, ctx->stream);

@@ -6,26 +6,16 @@
 
 namespace fmmx {
 
-void rotw_upload_f32(const RotwTables& t, cudaStream_t s) {
-    std::vector<float> mats(t.mats.begin(), t.mats.end()), fm(t.fm.begin(), t.fm.end()),
-        ifm(t.ifm.begin(), t.ifm.end()), fact(t.fact.begin(), t.fact.end());
-    cudaMemcpyToSymbolAsync(c_rot, mats.data(), sizeof(float) * ROTW_MATS, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_fm, fm.data(), sizeof(float) * ROTW_NH, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_ifm, ifm.data(), sizeof(float) * ROTW_NH, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_fact, fact.data(), sizeof(float) * (2 * ROTW_MAXP + 1), 0, cudaMemcpyHostToDevice, s);
-    cudaStreamSynchronize(s);  // the staging vectors die here
-}
-
 template <int P>
 static cudaError_t launch_p(DirList L, int nc, CellsView cv, const float* scale, const zf* mom, zf* loc, int* work,
                             int nsm, cudaStream_t s) {
-    constexpr size_t smem = rotw_smem_per_warp<float, P>();
-    auto kern = k_m2l_rotw<float, P, true, false>;
+    constexpr int W = rotw_block_warps<float, P>();
+    constexpr size_t smem = W * rotw_smem_per_warp<float, P>();
+    auto kern = k_m2l_rotw<float, P, true, false, W>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int per_sm = (int)std::min<size_t>(32, (220 * 1024) / smem);
-    if (per_sm < 1) per_sm = 1;
-    kern<<<work ? nsm * per_sm : (unsigned)nc, 32, smem, s>>>(L, nc, cv, scale, mom, loc, work);
+    constexpr int per_sm = rotw_warps_per_sm<float, P>() / W;
+    kern<<<work ? nsm * per_sm : (unsigned)((nc + W - 1) / W), 32 * W, smem, s>>>(L, nc, cv, scale, mom, loc, work);
     return cudaGetLastError();
 }
 

@@ -6,24 +6,16 @@
 
 namespace fmmx {
 
-void rotw_upload_f64(const RotwTables& t, cudaStream_t s) {
-    cudaMemcpyToSymbolAsync(c_rot, t.mats.data(), sizeof(double) * ROTW_MATS, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_fm, t.fm.data(), sizeof(double) * ROTW_NH, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_ifm, t.ifm.data(), sizeof(double) * ROTW_NH, 0, cudaMemcpyHostToDevice, s);
-    cudaMemcpyToSymbolAsync(c_fact, t.fact.data(), sizeof(double) * (2 * ROTW_MAXP + 1), 0, cudaMemcpyHostToDevice,
-                            s);
-}
-
 template <int P>
 static cudaError_t launch_p(DirList L, int nc, CellsView cv, const zd* mom, zd* loc, int* work, int nsm,
                             cudaStream_t s) {
-    constexpr size_t smem = rotw_smem_per_warp<double, P>();
-    auto kern = k_m2l_rotw<double, P, false, true>;
+    constexpr int W = rotw_block_warps<double, P>();
+    constexpr size_t smem = W * rotw_smem_per_warp<double, P>();
+    auto kern = k_m2l_rotw<double, P, false, true, W>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int per_sm = (int)std::min<size_t>(32, (220 * 1024) / smem);
-    if (per_sm < 1) per_sm = 1;
-    kern<<<work ? nsm * per_sm : (unsigned)nc, 32, smem, s>>>(L, nc, cv, nullptr, mom, loc, work);
+    constexpr int per_sm = rotw_warps_per_sm<double, P>() / W;
+    kern<<<work ? nsm * per_sm : (unsigned)((nc + W - 1) / W), 32 * W, smem, s>>>(L, nc, cv, nullptr, mom, loc, work);
     return cudaGetLastError();
 }
 
