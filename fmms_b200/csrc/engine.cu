@@ -128,6 +128,11 @@ struct Status {
     std::string msg;
 };
 
+// device flags and counters of the build: non-finite input, f pre-pass stack
+// overflow, cells per level and leaves, level-list cursors
+enum { TF_BAD = 0, TF_STACK = 1, TF_LEVELS = 2, TF_CURSOR = TF_LEVELS + FMMX_NLEVELS + 1,
+       TF_SIZE = TF_CURSOR + FMMX_NLEVELS };
+
 }  // namespace
 
 struct fmmx_ctx {
@@ -176,15 +181,11 @@ struct fmmx_ctx {
     DBuf<double> x, y, z, m, nax, nay, naz, npot;
     DBuf<char> cub_tmp;
 
-    // nodes before renumbering
-    DBuf<uint32_t> t_first, t_count;
-    DBuf<int32_t> t_parent;
-    DBuf<uint8_t> t_oct, t_level, t_leaf;
-    uint32_t tcap = 0;
-    DBuf<int> lvl;
-    DBuf<uint64_t> dfs_key, dfs_key_alt;
-    DBuf<uint32_t> dfs_val, dfs_val_alt;
-    DBuf<int32_t> new_id;
+    DBuf<uint32_t> cell_id0;  // n + 1: cells that start before each slot
+    DBuf<unsigned> geo_arrive;  // children of a cell whose geometry is done
+    DBuf<unsigned long long> bbox_enc;
+    DBuf<uint32_t> sort_sys, sort_sys_alt;  // a forest's second sort (by system)
+    DBuf<ulonglong2> sort_val, sort_val_alt;
 
     // cells (depth-first pre-order)
     DBuf<uint32_t> c_first, c_count;
@@ -272,7 +273,6 @@ fmmx_status finish(fmmx_ctx* ctx, fmmx_status st) {
     for (DBufBase* b : ctx->cache) b->release();
     ctx->built = ctx->evaluated = ctx->lists_valid = false;
     ctx->cap_front = ctx->cap_m2l = ctx->cap_p2p = 0;
-    ctx->tcap = 0;
     return st;
 }
 
@@ -400,7 +400,7 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     if (ctx->events) CK(cudaEventRecord(ctx->ev[0], s), "event");
     CK(ctx->keys.ensure(n), "alloc keys");
     CK(ctx->keys_sorted.ensure(n), "alloc keys");
-    CK(ctx->idx.ensure(n), "alloc idx");
+    CK(ctx->idx.ensure(n + 1), "alloc idx");
     CK(ctx->order.ensure(n), "alloc order");
     for (DBuf<double>* b : {&ctx->x, &ctx->y, &ctx->z, &ctx->m, &ctx->nax, &ctx->nay, &ctx->naz, &ctx->npot})
         CK(b->ensure(n), "alloc bodies");
@@ -413,101 +413,98 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     }
     const unsigned gb = std::min<unsigned>(grid_for(n, 256), 1024u);
     CK(ctx->bbox_part.ensure(gb * 6), "alloc box");
-    CK(ctx->flags.ensure(8), "alloc flags");
-    CK(cudaMemsetAsync(ctx->flags.p, 0, 8 * sizeof(int), s), "memset");
+    CK(ctx->flags.ensure(TF_SIZE), "alloc flags");
+    CK(cudaMemsetAsync(ctx->flags.p, 0, TF_SIZE * sizeof(int), s), "memset");
 
     ctx->launches = 0;
     const int nbits = 3 * FMMX_BITS;
     size_t tb;
     LCOUNT(5);  // bbox (2), keys, key sort (onesweep passes counted as 1), gather
+    int* bad = ctx->flags.p + TF_BAD;
+    uint64_t longest = n;  // the longest system
     if (nsys == 1) {
-        k_bbox_partial<<<gb, 256, 0, s>>>(d_pos, n, ctx->bbox_part.p, ctx->flags.p + 2);
+        k_bbox_partial<<<gb, 256, 0, s>>>(d_pos, n, ctx->bbox_part.p, bad);
         k_bbox_final<<<1, 32, 0, s>>>(ctx->bbox_part.p, (int)gb, ctx->box.p);
         k_keys<<<grid_for(n, 256), 256, 0, s>>>(d_pos, n, ctx->box.p, ctx->keys.p, ctx->idx.p);
-        CKL("keys");
-        tb = sort_pairs_u64_u32_temp((int)n, nbits);
-        CK(ctx->cub_tmp.ensure(tb), "alloc sort");
-        CK(sort_pairs_u64_u32(ctx->cub_tmp.p, tb, ctx->keys.p, ctx->keys_sorted.p, ctx->idx.p, ctx->order.p, (int)n,
-                              nbits, s),
-           "key sort");
     } else {
-        k_bbox_seg<<<nsys, 256, 0, s>>>(d_pos, ctx->sys_off.p, ctx->box.p, ctx->flags.p + 2);
+        longest = 0;
+        for (int q = 0; q < nsys; ++q) longest = std::max(longest, h_off[q + 1] - h_off[q]);
+        CK(ctx->bbox_enc.ensure(6 * (size_t)nsys), "alloc box");
+        CK(cudaMemsetAsync(ctx->bbox_enc.p, 0xff, 6 * (size_t)nsys * sizeof(unsigned long long), s), "memset");
+        k_bbox_seg<<<(unsigned)((n + BBOX_CHUNK - 1) / BBOX_CHUNK), 256, 0, s>>>(d_pos, n, ctx->sys_off.p, nsys,
+                                                                                 ctx->bbox_enc.p, bad);
+        k_bbox_seg_final<<<grid_for(nsys, 128), 128, 0, s>>>(ctx->bbox_enc.p, nsys, ctx->box.p);
         k_keys_seg<<<grid_for(n, 256), 256, 0, s>>>(d_pos, n, ctx->sys_off.p, nsys, ctx->box.p, ctx->keys.p,
                                                     ctx->idx.p);
-        CKL("keys");
+    }
+    CKL("keys");
+    // A forest of short systems is sorted a block per system. Where a system
+    // is longer than what a block sorts in a few steps, that block would run on
+    // alone (48 systems of together 10^6 bodies: 1.8 ms): one sort of all
+    // entries by key, then a stable one by system.
+    if (nsys > 1 && longest <= 4096) {
         tb = sort_pairs_seg_temp((int)n, nsys, ctx->sys_off.p, nbits);
         CK(ctx->cub_tmp.ensure(tb), "alloc sort");
         CK(sort_pairs_seg(ctx->cub_tmp.p, tb, ctx->keys.p, ctx->keys_sorted.p, ctx->idx.p, ctx->order.p, (int)n, nsys,
                           ctx->sys_off.p, nbits, s),
            "key sort");
+    } else {
+        tb = sort_pairs_u64_u32_temp((int)n, nbits);
+        CK(ctx->cub_tmp.ensure(tb), "alloc sort");
+        CK(sort_pairs_u64_u32(ctx->cub_tmp.p, tb, ctx->keys.p, ctx->keys_sorted.p, ctx->idx.p, ctx->order.p, (int)n,
+                              nbits, s),
+           "key sort");
+        if (nsys > 1) {
+            CK(ctx->sort_sys.ensure(n), "alloc sort");
+            CK(ctx->sort_sys_alt.ensure(n), "alloc sort");
+            CK(ctx->sort_val.ensure(n), "alloc sort");
+            CK(ctx->sort_val_alt.ensure(n), "alloc sort");
+            const int sbits = bits_for((uint64_t)(nsys - 1));
+            tb = sort_by_system_temp((int)n, sbits);
+            CK(ctx->cub_tmp.ensure(tb), "alloc sort");
+            k_pack_by_system<<<grid_for(n, 256), 256, 0, s>>>(ctx->keys_sorted.p, ctx->order.p, n, ctx->sys_off.p, nsys,
+                                                              ctx->sort_sys.p, ctx->sort_val.p);
+            CK(sort_by_system(ctx->cub_tmp.p, tb, ctx->sort_sys.p, ctx->sort_sys_alt.p, ctx->sort_val.p,
+                              ctx->sort_val_alt.p, (int)n, sbits, s),
+               "key sort");
+            k_unpack_by_system<<<grid_for(n, 256), 256, 0, s>>>(ctx->sort_val_alt.p, n, ctx->keys_sorted.p,
+                                                                ctx->order.p);
+            LCOUNT(3);
+        }
     }
     k_gather<<<grid_for(n, 256), 256, 0, s>>>(d_pos, d_mass, ctx->order.p, n, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p);
     CKL("gather");
 
-    // level-by-level node creation, retried with more room on overflow
-    CK(ctx->lvl.ensure(LV_SIZE), "alloc lvl");
-    if (ctx->tcap == 0 || ctx->tcap < (uint32_t)nsys) {
-        uint64_t est = 4ull * n / (uint64_t)std::max(ctx->cfg.n_leaf, 1) + 8ull * FMMX_NLEVELS * nsys + 64;
-        ctx->tcap = (uint32_t)std::min<uint64_t>(est, 0x7fffffffull);
-    }
-    int hl[LV_SIZE];
-    int hflags[8];
-    for (int attempt = 0;; ++attempt) {
-        const uint32_t cap = ctx->tcap;
-        CK(ctx->t_first.ensure(cap), "alloc nodes");
-        CK(ctx->t_count.ensure(cap), "alloc nodes");
-        CK(ctx->t_parent.ensure(cap), "alloc nodes");
-        CK(ctx->t_oct.ensure(cap), "alloc nodes");
-        CK(ctx->t_level.ensure(cap), "alloc nodes");
-        CK(ctx->t_leaf.ensure(cap), "alloc nodes");
-        TmpNodes tn{ctx->t_first.p, ctx->t_count.p, ctx->t_parent.p, ctx->t_oct.p, ctx->t_level.p, ctx->t_leaf.p};
-        CK(cudaMemsetAsync(ctx->lvl.p, 0, LV_SIZE * sizeof(int), s), "memset");
-        CK(cudaMemsetAsync(ctx->flags.p, 0, 2 * sizeof(int), s), "memset");
-        if (nsys == 1) k_tree_init<<<1, 32, 0, s>>>(tn, (uint32_t)n, ctx->lvl.p);
-        else k_tree_init_forest<<<grid_for(nsys, 128), 128, 0, s>>>(tn, ctx->sys_off.p, nsys, ctx->lvl.p);
-        LCOUNT(1 + FMMX_NLEVELS);
-        const unsigned gl = std::min<unsigned>(grid_for(cap, 256), 8u * (unsigned)ctx->nsm);
-        for (int L = 0; L < FMMX_NLEVELS; ++L)
-            k_build_level<<<gl, 256, 0, s>>>(tn, ctx->keys_sorted.p, L, (long long)ctx->cfg.n_leaf, cap, ctx->lvl.p,
-                                              ctx->flags.p);
-        CKL("build levels");
-        CK(cudaMemcpyAsync(hl, ctx->lvl.p, sizeof(hl), cudaMemcpyDeviceToHost, s), "copy");
-        CK(cudaMemcpyAsync(hflags, ctx->flags.p, sizeof(hflags), cudaMemcpyDeviceToHost, s), "copy");
-        CK(cudaStreamSynchronize(s), "tree build");
-        if (hflags[2]) return fail(ctx, FMMX_INVALID_ARG, "non-finite position");
-        if (!hflags[0]) break;
-        uint64_t total = 0;
-        for (int L = 0; L < FMMX_NLEVELS; ++L) total += (uint64_t)hl[LV_COUNT + L];
-        uint64_t want = std::max<uint64_t>(2ull * cap, total + total / 2 + 64);
-        if (want > 0x7fffffffull || attempt > 8) return fail(ctx, FMMX_OUT_OF_MEMORY, "node capacity");
-        ctx->tcap = (uint32_t)want;
-    }
-    int nc = 0, nlev = 0;
+    // the cells that start at each slot, and their numbers
+    const uint32_t n32 = (uint32_t)n, n_leaf = (uint32_t)ctx->cfg.n_leaf;
+    const unsigned gt = (unsigned)((n + 1 + TREE_BLOCK * TREE_PER_THREAD - 1) / (TREE_BLOCK * TREE_PER_THREAD));
+    CK(ctx->cell_id0.ensure(n + 1), "alloc cells");
+    tb = directed_list_temp(0, (int)n);
+    CK(ctx->cub_tmp.ensure(tb), "alloc scan");
+    k_cell_count<<<gt, TREE_BLOCK, 0, s>>>(ctx->keys_sorted.p, n32, ctx->sys_off.p, nsys, n_leaf, ctx->idx.p,
+                                           ctx->flags.p + TF_LEVELS);
+    CKL("tree cells");
+    CK(scan_u32(ctx->cub_tmp.p, ctx->cub_tmp.cap, ctx->idx.p, ctx->cell_id0.p, (int)(n + 1), s), "tree cells");
+    LCOUNT(3);
+    int hf[TF_SIZE];
+    CK(cudaMemcpyAsync(hf, ctx->flags.p, sizeof(hf), cudaMemcpyDeviceToHost, s), "copy");
+    CK(cudaStreamSynchronize(s), "tree build");
+    if (hf[TF_BAD]) return fail(ctx, FMMX_INVALID_ARG, "non-finite position");
+    uint64_t total = 0;
+    int nlev = 0;
+    LevelStarts ls;
     for (int L = 0; L < FMMX_NLEVELS; ++L) {
-        ctx->lvl_start[L] = nc;
-        ctx->lvl_count[L] = hl[LV_COUNT + L];
-        nc += hl[LV_COUNT + L];
-        if (hl[LV_COUNT + L] > 0) nlev = L + 1;
+        ctx->lvl_start[L] = ls.start[L] = (int)std::min<uint64_t>(total, 0x7fffffffull);
+        ctx->lvl_count[L] = hf[TF_LEVELS + L];
+        total += (uint64_t)hf[TF_LEVELS + L];
+        if (hf[TF_LEVELS + L] > 0) nlev = L + 1;
     }
+    if (total > 0x7fffffffull) return fail(ctx, FMMX_OUT_OF_MEMORY, "node capacity");
+    const int nc = (int)total;
     ctx->nc = nc;
     ctx->nlevels = nlev;
-    ctx->nleaves = hflags[1];
+    ctx->nleaves = hf[TF_LEVELS + FMMX_NLEVELS];
 
-    // depth-first renumbering: sort nodes by (first slot, level)
-    TmpNodes tn{ctx->t_first.p, ctx->t_count.p, ctx->t_parent.p, ctx->t_oct.p, ctx->t_level.p, ctx->t_leaf.p};
-    CK(ctx->dfs_key.ensure(nc), "alloc");
-    CK(ctx->dfs_key_alt.ensure(nc), "alloc");
-    CK(ctx->dfs_val.ensure(nc), "alloc");
-    CK(ctx->dfs_val_alt.ensure(nc), "alloc");
-    CK(ctx->new_id.ensure(nc), "alloc");
-    k_dfs_keys<<<grid_for(nc, 256), 256, 0, s>>>(tn, nc, ctx->dfs_key.p, ctx->dfs_val.p);
-    LCOUNT(5 + nlev);  // dfs keys, sort, finalize, link, body->leaf, geometry per level
-    const int dbits = 5 + bits_for(n);
-    tb = sort_pairs_u64_u32_temp(nc, dbits);
-    CK(ctx->cub_tmp.ensure(tb), "alloc sort");
-    CK(sort_pairs_u64_u32(ctx->cub_tmp.p, tb, ctx->dfs_key.p, ctx->dfs_key_alt.p, ctx->dfs_val.p, ctx->dfs_val_alt.p,
-                          nc, dbits, s),
-       "dfs sort");
     for (DBuf<uint32_t>* b : {&ctx->c_first, &ctx->c_count}) CK(b->ensure(nc), "alloc cells");
     CK(ctx->c_child.ensure(8 * (size_t)nc), "alloc cells");
     CK(ctx->c_parent.ensure(nc), "alloc cells");
@@ -515,31 +512,33 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     CK(ctx->body_leaf.ensure(n), "alloc cells");
     CK(ctx->c_leaf.ensure(nc), "alloc cells");
     CK(ctx->c_level.ensure(nc), "alloc cells");
-    for (DBuf<double>* b : {&ctx->c_cx, &ctx->c_cy, &ctx->c_cz, &ctx->c_mass, &ctx->c_rho})
+    for (DBuf<double>* b : {&ctx->c_cx, &ctx->c_cy, &ctx->c_cz, &ctx->c_mass, &ctx->c_rho, &ctx->c_h})
         CK(b->ensure(nc), "alloc cells");
+    CK(ctx->c_geo.ensure(nc), "alloc cells");
     CK(cudaMemsetAsync(ctx->c_child.p, 0xff, 8 * (size_t)nc * sizeof(int32_t), s), "memset");
-    k_finalize_cells<<<grid_for(nc, 256), 256, 0, s>>>(ctx->dfs_val_alt.p, nc, tn, ctx->new_id.p, view_mut(ctx));
-    k_link_cells<<<grid_for(nc, 256), 256, 0, s>>>(nc, tn, ctx->new_id.p, view_mut(ctx), ctx->level_cells.p);
-    k_body_leaf<<<grid_for((size_t)nc * 32, 256), 256, 0, s>>>(nc, ctx->c_first.p, ctx->c_count.p, ctx->c_leaf.p,
-                                                               ctx->body_leaf.p);
-    CKL("finalize cells");
-    for (int L = nlev - 1; L >= 0; --L) {
-        const int cnt = ctx->lvl_count[L];
-        k_geometry_level<<<grid_for(cnt, 128), 128, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt,
-                                                            view_mut(ctx), ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p,
-                                                            ctx->cfg.center_mode);
+    k_cell_emit<<<gt, TREE_BLOCK, 0, s>>>(ctx->keys_sorted.p, n32, ctx->sys_off.p, nsys, n_leaf, ctx->cell_id0.p, ls,
+                                          ctx->flags.p + TF_CURSOR, ctx->box.p, view_mut(ctx), ctx->level_cells.p,
+                                          ctx->body_leaf.p, ctx->c_h.p);
+    CKL("tree cells");
+    LCOUNT(2);  // cells, geometry
+    if (ctx->cfg.center_mode == FMMX_CENTER_COM) {
+        CK(ctx->geo_arrive.ensure(nc), "alloc cells");
+        CK(cudaMemsetAsync(ctx->geo_arrive.p, 0, (size_t)nc * sizeof(unsigned), s), "memset");
+        k_geometry_com<<<grid_for(nc, GEO_WARPS), 32 * GEO_WARPS, 0, s>>>(nc, view_mut(ctx), ctx->x.p, ctx->y.p,
+                                                                         ctx->z.p, ctx->m.p, ctx->geo_arrive.p,
+                                                                         ctx->c_geo.p);
+    } else {
+        for (int L = nlev - 1; L >= 0; --L) {
+            const int cnt = ctx->lvl_count[L];
+            k_geometry_level<<<grid_for(cnt, 128), 128, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt,
+                                                                view_mut(ctx), ctx->x.p, ctx->y.p, ctx->z.p,
+                                                                ctx->m.p, ctx->cfg.center_mode);
+        }
+        k_pack_geo<<<grid_for(nc, 256), 256, 0, s>>>(nc, ctx->c_cx.p, ctx->c_cy.p, ctx->c_cz.p, ctx->c_rho.p,
+                                                     ctx->c_geo.p);
+        LCOUNT(nlev);
     }
     CKL("geometry");
-    CK(ctx->c_h.ensure(nc), "alloc cells");
-    for (int L = 0; L < nlev; ++L) {
-        const int cnt = ctx->lvl_count[L];
-        k_cell_h<<<grid_for(cnt, 256), 256, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt, ctx->c_parent.p,
-                                                    ctx->box.p, ctx->c_h.p);
-    }
-    CK(ctx->c_geo.ensure(nc), "alloc cells");
-    k_pack_geo<<<grid_for(nc, 256), 256, 0, s>>>(nc, ctx->c_cx.p, ctx->c_cy.p, ctx->c_cz.p, ctx->c_rho.p, ctx->c_geo.p);
-    LCOUNT(nlev + 1);
-    CKL("cell sizes");
     if (ctx->events) CK(cudaEventRecord(ctx->ev[1], s), "event");
     CK(cudaStreamSynchronize(s), "build");
     if (ctx->events) {
@@ -854,9 +853,9 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         CK(cudaStreamWaitEvent(s2, ctx->fork[0], 0), "fork");
     }
     if (dehnen) {
-        CK(cudaMemsetAsync(ctx->flags.p + 3, 0, sizeof(int), s), "memset");
+        CK(cudaMemsetAsync(ctx->flags.p + TF_STACK, 0, sizeof(int), s), "memset");
         k_fprepass<<<grid_for(n, 128), 128, 0, s>>>(cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, n, ctx->sys_off.p,
-                                                    ctx->nsys, ctx->level_cells.p, ctx->f.p, ctx->flags.p + 3);
+                                                    ctx->nsys, ctx->level_cells.p, ctx->f.p, ctx->flags.p + TF_STACK);
         CKL("f pre-pass");
     }
     if (mixed && !dehnen) {
@@ -915,7 +914,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         if (st != FMMX_OK) return st;
         if (dehnen) {
             int bad = 0;
-            CK(cudaMemcpy(&bad, ctx->flags.p + 3, sizeof(int), cudaMemcpyDeviceToHost), "copy");
+            CK(cudaMemcpy(&bad, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost), "copy");
             if (bad) return fail(ctx, FMMX_DEVICE_ERROR, "f pre-pass stack overflow");
         }
     }

@@ -6,17 +6,9 @@
 
 namespace fmmx {
 
-// Level bookkeeping array: start and count of each level's nodes.
-enum { LV_START = 0, LV_COUNT = FMMX_NLEVELS + 1, LV_SIZE = 2 * (FMMX_NLEVELS + 1) };
-
-// Nodes as created level by level, before depth-first renumbering.
-struct TmpNodes {
-    uint32_t* first;
-    uint32_t* count;
-    int32_t* parent;
-    uint8_t* oct;
-    uint8_t* level;
-    uint8_t* leaf;
+// first position of each level in the level lists
+struct LevelStarts {
+    int start[FMMX_NLEVELS];
 };
 
 struct CellsMut {
@@ -71,21 +63,26 @@ __global__ void k_bbox_final(const double* part, int nparts, double* box);
 __global__ void k_keys(const double* pos, size_t n, const double* box, uint64_t* keys, uint32_t* idx);
 __global__ void k_gather(const double* pos, const double* mass, const uint32_t* order, size_t n, double* x,
                          double* y, double* z, double* m);
-__global__ void k_tree_init(TmpNodes t, uint32_t n, int* lvl);
-__global__ void k_bbox_seg(const double* pos, const uint64_t* off, double* box, int* bad);
+__global__ void k_bbox_seg(const double* pos, size_t n, const uint64_t* off, int nsys, unsigned long long* enc,
+                           int* bad);
+__global__ void k_bbox_seg_final(const unsigned long long* enc, int nsys, double* box);
+#define BBOX_CHUNK 2048  // bodies per block of k_bbox_seg
 __global__ void k_keys_seg(const double* pos, size_t n, const uint64_t* off, int nsys, const double* box,
                            uint64_t* keys, uint32_t* idx);
-__global__ void k_tree_init_forest(TmpNodes t, const uint64_t* off, int nsys, int* lvl);
-__global__ void k_cell_h(const int32_t* level_cells, int lstart, int lcnt, const int32_t* parent, const double* box,
-                         double* h);
+__global__ void k_pack_by_system(const uint64_t* keys, const uint32_t* order, size_t n, const uint64_t* off, int nsys,
+                                 uint32_t* sys, ulonglong2* val);
+__global__ void k_unpack_by_system(const ulonglong2* val, size_t n, uint64_t* keys, uint32_t* order);
 __global__ void k_walk_init(const int32_t* level_cells, int nroots, uint2* front);
-__global__ void k_build_level(TmpNodes t, const uint64_t* keys, int L, long long n_leaf, uint32_t cap, int* lvl,
-                              int* flags);
-__global__ void k_dfs_keys(TmpNodes t, int nc, uint64_t* key, uint32_t* val);
-__global__ void k_finalize_cells(const uint32_t* sorted_t, int nc, TmpNodes t, int32_t* new_id, CellsMut cells);
-__global__ void k_link_cells(int nc, TmpNodes t, const int32_t* new_id, CellsMut cells, int32_t* level_cells);
-__global__ void k_body_leaf(int nc, const uint32_t* first, const uint32_t* count, const uint8_t* leaf,
-                            int32_t* body_leaf);
+#define TREE_BLOCK 256
+#define TREE_PER_THREAD 4  // slots per thread of the two tree kernels
+__global__ void k_cell_count(const uint64_t* keys, uint32_t n, const uint64_t* off, int nsys, uint32_t n_leaf,
+                             uint32_t* count, int* lvl);
+__global__ void k_cell_emit(const uint64_t* keys, uint32_t n, const uint64_t* off, int nsys, uint32_t n_leaf,
+                            const uint32_t* id0, LevelStarts ls, int* cursor, const double* box, CellsMut cells,
+                            int32_t* level_cells, int32_t* body_leaf, double* h);
+#define GEO_WARPS 4
+__global__ void k_geometry_com(int nc, CellsMut cells, const double* x, const double* y, const double* z,
+                               const double* m, unsigned* arrive, double4* geo);
 __global__ void k_geometry_level(const int32_t* level_cells, int lstart, int lcnt, CellsMut cells, const double* x,
                                  const double* y, const double* z, const double* m, int center_mode);
 // bodies per round of the exact P2M (the lanes of a warp build that many Υ tables at once)

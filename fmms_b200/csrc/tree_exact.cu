@@ -90,47 +90,71 @@ __global__ void k_bbox_final(const double* __restrict__ part, int nparts, double
     box[7] = 1.0 / side;
 }
 
-// Forest of independent systems (segments [off[s], off[s+1]) of the input):
-// one block per system reduces its own box.
-__global__ void k_bbox_seg(const double* __restrict__ pos, const uint64_t* __restrict__ off,
-                           double* __restrict__ box, int* __restrict__ bad) {
-    const int sys = blockIdx.x;
-    const uint64_t b = off[sys], e = off[sys + 1];
-    double lo[3] = {INFINITY, INFINITY, INFINITY};
-    double hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    int nonfinite = 0;
-    for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            double v = pos[3 * i + d];
-            nonfinite |= !isfinite(v);
-            lo[d] = fmin(lo[d], v);
-            hi[d] = fmax(hi[d], v);
-        }
+// The system of a forest that holds input i: the last one with off[sys] <= i.
+__device__ __forceinline__ int system_of(const uint64_t* __restrict__ off, int nsys, size_t i) {
+    int lo = 0, hi = nsys;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (off[mid] <= i) lo = mid;
+        else hi = mid;
     }
-    __shared__ double sh[6][256];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        sh[d][threadIdx.x] = lo[d];
-        sh[3 + d][threadIdx.x] = hi[d];
-    }
-    if (nonfinite) atomicOr(bad, 1);
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
+    return lo;
+}
+
+// Order-preserving encoding of a double as an unsigned integer.
+__device__ __forceinline__ unsigned long long enc_order(double v) {
+    const long long b = __double_as_longlong(v);
+    return b < 0 ? ~(unsigned long long)b : (unsigned long long)b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double dec_order(unsigned long long u) {
+    return __longlong_as_double((long long)((u & 0x8000000000000000ull) ? u & 0x7fffffffffffffffull : ~u));
+}
+
+// Boxes of a forest of independent systems (segments [off[s], off[s+1]) of the
+// input): every block reduces BBOX_CHUNK consecutive bodies, system by system,
+// into enc[6 s ..] = minima of the encoded lo and -hi (all bits set at the
+// start); minima are exact, so the order does not matter. (One block per
+// system took 221 us for 48 systems of together 10^6 bodies: the largest
+// system's block ran alone.)
+__global__ void k_bbox_seg(const double* __restrict__ pos, size_t n, const uint64_t* __restrict__ off, int nsys,
+                           unsigned long long* __restrict__ enc, int* __restrict__ bad) {
+    const size_t b0 = (size_t)blockIdx.x * BBOX_CHUNK, e0 = min(n, b0 + BBOX_CHUNK);
+    __shared__ unsigned long long sh[6][8];
+    for (int sys = system_of(off, nsys, b0); sys < nsys && off[sys] < e0; ++sys) {
+        const size_t b = max((size_t)off[sys], b0), e = min((size_t)off[sys + 1], e0);
+        double v[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};
+        int nonfinite = 0;
+        for (size_t i = b + threadIdx.x; i < e; i += blockDim.x) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                sh[d][threadIdx.x] = fmin(sh[d][threadIdx.x], sh[d][threadIdx.x + w]);
-                sh[3 + d][threadIdx.x] = fmax(sh[3 + d][threadIdx.x], sh[3 + d][threadIdx.x + w]);
+                const double q = pos[3 * i + d];
+                nonfinite |= !isfinite(q);
+                v[d] = fmin(v[d], q);
+                v[3 + d] = fmin(v[3 + d], -q);
             }
+        }
+        if (nonfinite) atomicOr(bad, 1);
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int d = 0; d < 6; ++d) v[d] = fmin(v[d], __shfl_xor_sync(0xffffffffu, v[d], o));
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+            for (int d = 0; d < 6; ++d) sh[d][threadIdx.x >> 5] = enc_order(v[d]);
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            unsigned long long m = sh[threadIdx.x][0];
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = min(m, sh[threadIdx.x][w]);
+            atomicMin(enc + 6 * sys + threadIdx.x, m);
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
+}
+__global__ void k_bbox_seg_final(const unsigned long long* __restrict__ enc, int nsys, double* __restrict__ box) {
+    for (int sys = blockIdx.x * blockDim.x + threadIdx.x; sys < nsys; sys += gridDim.x * blockDim.x) {
         double* bx = box + 8 * sys;
         for (int d = 0; d < 3; ++d) {
-            bx[d] = sh[d][0];
-            bx[3 + d] = sh[3 + d][0];
+            bx[d] = dec_order(enc[6 * sys + d]);
+            bx[3 + d] = -dec_order(enc[6 * sys + 3 + d]);
         }
         const double side = fmax(fmax(fmax(bx[3] - bx[0], bx[4] - bx[1]), bx[5] - bx[2]), DBL_MIN);
         bx[6] = side;
@@ -173,13 +197,8 @@ __global__ void k_keys(const double* __restrict__ pos, size_t n, const double* _
 __global__ void k_keys_seg(const double* __restrict__ pos, size_t n, const uint64_t* __restrict__ off, int nsys,
                            const double* __restrict__ box, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        int lo = 0, hi = nsys;  // last system with off[sys] <= i
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (off[mid] <= i) lo = mid;
-            else hi = mid;
-        }
-        const double lo0 = box[8 * lo], inv = box[8 * lo + 7];
+        const int sys = system_of(off, nsys, i);
+        const double lo0 = box[8 * sys], inv = box[8 * sys + 7];
         uint64_t k = dilate21(quant(pos[3 * i + 2], lo0, inv));
         k |= dilate21(quant(pos[3 * i + 1], lo0, inv)) << 1;
         k |= dilate21(quant(pos[3 * i + 0], lo0, inv)) << 2;
@@ -201,47 +220,23 @@ __global__ void k_gather(const double* __restrict__ pos, const double* __restric
     }
 }
 
-// ------------------------------------------------------------ topology
-// The reference builds cells by depth-first recursion (build_rec,
-// tree.rs:404-445). Here nodes are created level by level from the sorted
-// keys (every node of a level in parallel, its octant ranges by binary search
-// on the key digit), then renumbered into depth-first pre-order: with ranges
-// nested or disjoint, pre-order is the order of (first slot, level).
-__global__ void k_tree_init(TmpNodes t, uint32_t n, int* __restrict__ lvl) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        t.first[0] = 0;
-        t.count[0] = n;
-        t.parent[0] = -1;
-        t.oct[0] = 0;
-        t.level[0] = 0;
-        lvl[LV_START + 0] = 0;
-        lvl[LV_COUNT + 0] = 1;
+// System of each entry of `order` (sorted by key over the whole forest), for
+// the second, stable sort by system; value: the key and the input index.
+__global__ void k_pack_by_system(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ order, size_t n,
+                                 const uint64_t* __restrict__ off, int nsys, uint32_t* __restrict__ sys,
+                                 ulonglong2* __restrict__ val) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t id = order[i];
+        sys[i] = (uint32_t)system_of(off, nsys, id);
+        val[i] = make_ulonglong2(keys[i], id);
     }
 }
-
-// One root per system.
-__global__ void k_tree_init_forest(TmpNodes t, const uint64_t* __restrict__ off, int nsys, int* __restrict__ lvl) {
-    for (int sys = blockIdx.x * blockDim.x + threadIdx.x; sys < nsys; sys += gridDim.x * blockDim.x) {
-        t.first[sys] = (uint32_t)off[sys];
-        t.count[sys] = (uint32_t)(off[sys + 1] - off[sys]);
-        t.parent[sys] = -1;
-        t.oct[sys] = 0;
-        t.level[sys] = 0;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        lvl[LV_START + 0] = 0;
-        lvl[LV_COUNT + 0] = nsys;
-    }
-}
-
-// Box size of every cell: a root gets its system's box side, a child half its
-// parent's. Level 0 lists the roots in system order.
-__global__ void k_cell_h(const int32_t* __restrict__ level_cells, int lstart, int lcnt, const int32_t* __restrict__ parent,
-                         const double* __restrict__ box, double* __restrict__ h) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < lcnt; j += gridDim.x * blockDim.x) {
-        const int c = level_cells[lstart + j];
-        const int par = parent[c];
-        h[c] = par < 0 ? box[8 * j + 6] : 0.5 * h[par];
+__global__ void k_unpack_by_system(const ulonglong2* __restrict__ val, size_t n, uint64_t* __restrict__ keys,
+                                   uint32_t* __restrict__ order) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const ulonglong2 v = val[i];
+        keys[i] = v.x;
+        order[i] = (uint32_t)v.y;
     }
 }
 
@@ -253,98 +248,182 @@ __global__ void k_walk_init(const int32_t* __restrict__ level_cells, int nroots,
     }
 }
 
-__global__ void k_build_level(TmpNodes t, const uint64_t* __restrict__ keys, int L, long long n_leaf, uint32_t cap,
-                              int* __restrict__ lvl, int* __restrict__ flags) {
-    const int start = lvl[LV_START + L];
-    const int cnt = lvl[LV_COUNT + L];
-    const int next_start = start + cnt;
-    if (blockIdx.x == 0 && threadIdx.x == 0) lvl[LV_START + L + 1] = next_start;
-    if (flags[0]) return;  // capacity exceeded earlier: the host retries larger
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-        const int tt = start + j;
-        if ((uint32_t)tt >= cap) break;
-        const uint32_t f = t.first[tt], c = t.count[tt];
-        const bool leaf = (long long)c <= n_leaf || L >= FMMX_MAXLEVEL;
-        t.leaf[tt] = leaf ? 1 : 0;
-        if (leaf) {
-            atomicAdd(&flags[1], 1);  // leaf count
-            continue;
-        }
-        const int shift = 3 * (FMMX_MAXLEVEL - (L + 1));
-        const uint32_t end = f + c;
-        uint32_t lo = f;
-        for (uint32_t oct = 0; oct < 8; ++oct) {
-            uint32_t a = lo, b = end;
-            while (a < b) {  // first slot whose octant digit exceeds oct
-                uint32_t mid = a + ((b - a) >> 1);
-                uint32_t d = (uint32_t)((keys[mid] >> shift) & 7ULL);
-                if (d <= oct) a = mid + 1;
-                else b = mid;
-            }
-            const uint32_t hi = a;
-            if (hi > lo) {
-                int slot = atomicAdd(&lvl[LV_COUNT + L + 1], 1);
-                uint32_t ct = (uint32_t)(next_start + slot);
-                if (ct < cap) {
-                    t.first[ct] = lo;
-                    t.count[ct] = hi - lo;
-                    t.parent[ct] = tt;
-                    t.oct[ct] = (uint8_t)oct;
-                    t.level[ct] = (uint8_t)(L + 1);
+// ------------------------------------------------------------ topology
+// The reference builds cells by depth-first recursion (build_rec,
+// tree.rs:404-445). Here every cell is found from the sorted keys alone, all
+// levels at once. A cell is a block of slots whose keys share their first L
+// octal digits; it exists if its parent (the block one digit shorter) holds
+// more than n_leaf bodies, and is split again while it does so itself, down to
+// level 21. With
+//   d_i = the digits slot i shares with slot i - 1 (-1 at a system's start) and
+//   w_i = the digits slot i shares with slot i + n_leaf (-1: another system),
+// the blocks that start at slot i are those of levels above d_i; one of them
+// holds more than n_leaf bodies up to level w_i, and the block of level d_i
+// around slot i, the parent of the first, is looked up where w_i does not
+// decide. So slot i starts the cells of levels d_i + 1 .. min(21, m_i + 1),
+// m_i the deepest level whose block around i is over-full, and the last of them
+// is a leaf. Depth-first pre-order is the order of (first slot, level): a
+// prefix sum of the counts numbers the cells, and body i's leaf is the last cell
+// that starts at or before it. (The build used to run a launch per level, a
+// binary search per octant and thread, and a radix sort into depth-first order:
+// N = 2e5, 10 levels, 0.46 ms for the levels and 0.1 ms for the order.)
+__device__ __forceinline__ int common_digits(uint64_t a, uint64_t b) {
+    const uint64_t x = a ^ b;
+    return x ? (__clzll((long long)x) - 1) / 3 : FMMX_MAXLEVEL;
+}
+
+// the slots [beg, end) of the system that holds slot i
+__device__ __forceinline__ void system_range(const uint64_t* __restrict__ off, int nsys, uint32_t n, uint32_t i,
+                                             uint32_t& beg, uint32_t& end) {
+    beg = 0;
+    end = n;
+    if (nsys > 1) {
+        const int s = system_of(off, nsys, i);
+        beg = (uint32_t)off[s];
+        end = (uint32_t)off[s + 1];
+    }
+}
+
+// first slot of [lo, i] that shares at least L digits with slot i
+__device__ __forceinline__ uint32_t block_begin(const uint64_t* __restrict__ keys, uint32_t lo, uint32_t i, int L) {
+    const uint64_t k = keys[i];
+    while (lo < i) {
+        const uint32_t mid = lo + ((i - lo) >> 1);
+        if (common_digits(keys[mid], k) >= L) i = mid;
+        else lo = mid + 1;
+    }
+    return i;
+}
+// first slot of (i, hi] that shares fewer than L digits with slot i (hi if none)
+__device__ __forceinline__ uint32_t block_end(const uint64_t* __restrict__ keys, uint64_t k, uint32_t lo, uint32_t hi,
+                                              int L) {
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (common_digits(keys[mid], k) >= L) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Cells that start at each slot (count[n] = 0 for the prefix sum), the cells
+// of each level and the number of leaves (lvl[0 .. 21] and lvl[22], zero at
+// the start).
+__global__ void __launch_bounds__(TREE_BLOCK) k_cell_count(const uint64_t* __restrict__ keys, uint32_t n,
+                                                           const uint64_t* __restrict__ off, int nsys,
+                                                           uint32_t n_leaf, uint32_t* __restrict__ count,
+                                                           int* __restrict__ lvl) {
+    __shared__ int hist[FMMX_NLEVELS + 1];
+    if (threadIdx.x <= FMMX_NLEVELS) hist[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * (uint32_t)(TREE_BLOCK * TREE_PER_THREAD) + threadIdx.x;
+    for (int q = 0; q < TREE_PER_THREAD; ++q) {
+        const uint32_t i = base + q * TREE_BLOCK;
+        if (i > n) break;
+        uint32_t c = 0;
+        if (i < n) {
+            uint32_t beg, end;
+            system_range(off, nsys, n, i, beg, end);
+            const uint64_t k = keys[i];
+            const int d = i == beg ? -1 : common_digits(keys[i - 1], k);
+            const int w = n_leaf < end - i ? common_digits(keys[i + n_leaf], k) : -1;
+            int m = w;  // deepest over-full block around i
+            if (w <= d) {
+                m = -2;
+                if (d < 0) {
+                    m = -1;  // a root exists whatever it holds
                 } else {
-                    atomicOr(&flags[0], 1);  // node capacity exceeded
+                    const uint32_t lo = i - beg > n_leaf ? i - n_leaf : beg;
+                    const uint32_t s = block_begin(keys, lo, i, d);
+                    // more than n_leaf bodies: the block begins before `lo`, or reaches slot s + n_leaf
+                    const bool over = n_leaf < end - s && common_digits(keys[s + n_leaf], k) >= d;
+                    if (over) m = d;
                 }
             }
-            lo = hi;
+            if (m >= d) {
+                const int last = min(FMMX_MAXLEVEL, m + 1);
+                c = (uint32_t)(last - d);
+                for (int L = d + 1; L <= last; ++L) atomicAdd(&hist[L], 1);
+                if (c) atomicAdd(&hist[FMMX_NLEVELS], 1);
+            }
         }
+        count[i] = c;
     }
+    __syncthreads();
+    if (threadIdx.x <= FMMX_NLEVELS && hist[threadIdx.x]) atomicAdd(&lvl[threadIdx.x], hist[threadIdx.x]);
 }
 
-__global__ void k_dfs_keys(TmpNodes t, int nc, uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-        key[i] = ((uint64_t)t.first[i] << 5) | (uint64_t)t.level[i];
-        val[i] = (uint32_t)i;
+// The cells in depth-first order (id0: the prefix sum of k_cell_count's
+// counts), the level lists (roots in system order, else arbitrary; cursor[22]
+// zero at the start), the bodies' leaves and the cells' box sizes.
+__global__ void __launch_bounds__(TREE_BLOCK) k_cell_emit(const uint64_t* __restrict__ keys, uint32_t n,
+                                                          const uint64_t* __restrict__ off, int nsys, uint32_t n_leaf,
+                                                          const uint32_t* __restrict__ id0, LevelStarts ls,
+                                                          int* __restrict__ cursor, const double* __restrict__ box,
+                                                          CellsMut cells, int32_t* __restrict__ level_cells,
+                                                          int32_t* __restrict__ body_leaf, double* __restrict__ h) {
+    __shared__ int hist[FMMX_NLEVELS], lbase[FMMX_NLEVELS];
+    if (threadIdx.x < FMMX_NLEVELS) hist[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * (uint32_t)(TREE_BLOCK * TREE_PER_THREAD) + threadIdx.x;
+    for (int q = 0; q < TREE_PER_THREAD; ++q) {  // this block's cells of each level
+        const uint32_t i = base + q * TREE_BLOCK;
+        if (i >= n) break;
+        const uint32_t c0 = id0[i], c1 = id0[i + 1];
+        body_leaf[i] = (int32_t)c1 - 1;
+        if (c0 == c1) continue;
+        uint32_t beg, end;
+        system_range(off, nsys, n, i, beg, end);
+        const int d = i == beg ? -1 : common_digits(keys[i - 1], keys[i]);
+        for (uint32_t c = c0; c < c1; ++c) atomicAdd(&hist[d + 1 + (int)(c - c0)], 1);
     }
-}
-
-__global__ void k_finalize_cells(const uint32_t* __restrict__ sorted_t, int nc, TmpNodes t,
-                                 int32_t* __restrict__ new_id, CellsMut cells) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-        uint32_t tt = sorted_t[i];
-        new_id[tt] = i;
-        cells.first[i] = t.first[tt];
-        cells.count[i] = t.count[tt];
-        cells.level[i] = t.level[tt];
-        cells.leaf[i] = t.leaf[tt];
+    __syncthreads();
+    if (threadIdx.x < FMMX_NLEVELS) {
+        const int v = hist[threadIdx.x];
+        lbase[threadIdx.x] = ls.start[threadIdx.x] + (v ? atomicAdd(&cursor[threadIdx.x], v) : 0);
+        hist[threadIdx.x] = 0;
     }
-}
-
-__global__ void k_link_cells(int nc, TmpNodes t, const int32_t* __restrict__ new_id, CellsMut cells,
-                             int32_t* __restrict__ level_cells) {
-    for (int tt = blockIdx.x * blockDim.x + threadIdx.x; tt < nc; tt += gridDim.x * blockDim.x) {
-        int c = new_id[tt];
-        level_cells[tt] = c;
-        int par = t.parent[tt];
-        if (par >= 0) {
-            int pc = new_id[par];
-            cells.child[8 * pc + t.oct[tt]] = c;
-            cells.parent[c] = pc;
-        } else {
-            cells.parent[c] = -1;
+    __syncthreads();
+    for (int q = 0; q < TREE_PER_THREAD; ++q) {
+        const uint32_t i = base + q * TREE_BLOCK;
+        if (i >= n) break;
+        const uint32_t c0 = id0[i], c1 = id0[i + 1];
+        if (c0 == c1) continue;
+        int sys = 0;
+        uint32_t beg = 0, end = n;
+        if (nsys > 1) {
+            sys = system_of(off, nsys, i);
+            beg = (uint32_t)off[sys];
+            end = (uint32_t)off[sys + 1];
         }
-    }
-}
-
-// slot -> leaf cell, for the L2P stage
-__global__ void k_body_leaf(int nc, const uint32_t* __restrict__ first, const uint32_t* __restrict__ count,
-                            const uint8_t* __restrict__ leaf, int32_t* __restrict__ body_leaf) {
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int c = warp; c < nc; c += nwarps) {
-        if (!leaf[c]) continue;
-        uint32_t f = first[c], e = first[c] + count[c];
-        for (uint32_t k = f + lane; k < e; k += 32) body_leaf[k] = c;
+        const uint64_t k = keys[i];
+        const int d = i == beg ? -1 : common_digits(keys[i - 1], k);
+        int par = -1;
+        if (d >= 0) {  // the block of level d around slot i
+            const uint32_t s = block_begin(keys, beg, i, d);
+            const int ds = s == beg ? -1 : common_digits(keys[s - 1], keys[s]);
+            par = (int)id0[s] + d - ds - 1;
+        }
+        const double side = box[8 * sys + 6];
+        uint32_t e = end;
+        for (uint32_t c = c0; c < c1; ++c) {
+            const int L = d + 1 + (int)(c - c0);
+            const bool leaf = c + 1 == c1;
+            // bounds of the block's end: a leaf above level 21 holds at most n_leaf bodies, an internal cell more
+            uint32_t lo = i + 1, hi = e;
+            if (leaf && L < FMMX_MAXLEVEL) hi = min(hi, i + max(n_leaf, 1u));
+            else if (!leaf) lo = i + n_leaf + 1;
+            e = block_end(keys, k, lo, hi, L);
+            cells.first[c] = i;
+            cells.count[c] = e - i;
+            cells.level[c] = (uint8_t)L;
+            cells.leaf[c] = leaf ? 1 : 0;
+            cells.parent[c] = par;
+            if (par >= 0) cells.child[8 * (size_t)par + ((k >> (3 * (FMMX_MAXLEVEL - L))) & 7)] = (int32_t)c;
+            h[c] = ldexp(side, -L);
+            if (L == 0) level_cells[sys] = (int32_t)c;
+            else level_cells[lbase[L] + atomicAdd(&hist[L], 1)] = (int32_t)c;
+            par = (int)c;
+        }
     }
 }
 
@@ -455,7 +534,9 @@ __device__ void ritter(const Items& it, double cen[3]) {
     }
 }
 
-// Octree::geometry, tree.rs:152-227, one level at a time from the deepest.
+// Octree::geometry, tree.rs:152-227, one level at a time from the deepest, a
+// thread per cell: the Ritter spheres (each a serial scan of its items), whose
+// centres of mass k_geometry_com does not serve.
 __global__ void k_geometry_level(const int32_t* __restrict__ level_cells, int lstart, int lcnt, CellsMut cells,
                                  const double* __restrict__ x, const double* __restrict__ y,
                                  const double* __restrict__ z, const double* __restrict__ m, int center_mode) {
@@ -518,6 +599,130 @@ __global__ void k_geometry_level(const int32_t* __restrict__ level_cells, int ls
         cells.cy[c] = cen[1];
         cells.cz[c] = cen[2];
         cells.rho[c] = rho;
+    }
+}
+
+// Octree::geometry with centres of mass, tree.rs:152-227, in one launch: a
+// warp per leaf, then up the tree -- the warp that finishes a cell's last child
+// goes on with the cell, so nobody waits. The sums run in the reference's order
+// (bodies in slot order, children in octant order): the lanes form the terms of
+// 32 bodies side by side and lanes 0..3 add one component each; rho is the
+// square root of the largest squared distance (the root is monotone and
+// correctly rounded, so it is the largest distance). Bound by the latency of
+// the FP64 add chains and of one L2 round trip per level. A thread per cell and
+// a launch per level took 0.27 ms at N = 2e5 (10 levels) and 0.11 ms at 2^20.
+// arrive: one zero per cell.
+__global__ void __launch_bounds__(32 * GEO_WARPS) k_geometry_com(int nc, CellsMut cells, const double* __restrict__ x,
+                                                                 const double* __restrict__ y,
+                                                                 const double* __restrict__ z,
+                                                                 const double* __restrict__ m,
+                                                                 unsigned* __restrict__ arrive,
+                                                                 double4* __restrict__ geo) {
+    __shared__ double buf_all[GEO_WARPS][4][33];
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    double(*buf)[33] = buf_all[threadIdx.x >> 5];
+    const int nwarps = gridDim.x * GEO_WARPS;
+    for (int c0 = blockIdx.x * GEO_WARPS + (threadIdx.x >> 5); c0 < nc; c0 += nwarps) {
+        if (!cells.leaf[c0]) continue;
+        int c = c0;
+        {
+            const uint32_t f = cells.first[c], cnt = cells.count[c];
+            double s = 0.0;  // lanes 0..3: mass, m x, m y, m z
+            double bx = 0, by = 0, bz = 0;
+            for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
+                const int nb = (int)min(32u, cnt - b0);
+                if (lane < nb) {
+                    const uint32_t k = f + b0 + lane;
+                    bx = x[k];
+                    by = y[k];
+                    bz = z[k];
+                    const double mk = m[k];
+                    buf[0][lane] = mk;
+                    buf[1][lane] = mk * bx;
+                    buf[2][lane] = mk * by;
+                    buf[3][lane] = mk * bz;
+                }
+                __syncwarp();
+                if (lane < 4)
+                    for (int k = 0; k < nb; ++k) s += buf[lane][k];
+                __syncwarp();
+            }
+            const double mass = __shfl_sync(FULL, s, 0);
+            const double q = s / mass;
+            const double cx = __shfl_sync(FULL, q, 1), cy = __shfl_sync(FULL, q, 2), cz = __shfl_sync(FULL, q, 3);
+            double d2 = 0.0;
+            for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
+                if (b0 + lane < cnt) {
+                    if (cnt > 32) {
+                        const uint32_t k = f + b0 + lane;
+                        bx = x[k];
+                        by = y[k];
+                        bz = z[k];
+                    }
+                    d2 = fmax(d2, dist2_3(bx, by, bz, cx, cy, cz));
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) d2 = fmax(d2, __shfl_xor_sync(FULL, d2, o));
+            if (lane == 0) {
+                const double rho = sqrt(d2);
+                cells.mass[c] = mass;
+                cells.cx[c] = cx;
+                cells.cy[c] = cy;
+                cells.cz[c] = cz;
+                cells.rho[c] = rho;
+                geo[c] = make_double4(cx, cy, cz, rho);
+            }
+        }
+        for (int par = cells.parent[c]; par >= 0; par = cells.parent[c]) {
+            const int ch = lane < 8 ? cells.child[8 * (size_t)par + lane] : -1;
+            const unsigned have = __ballot_sync(FULL, ch >= 0);
+            unsigned prev = 0;
+            if (lane == 0) {
+                __threadfence();  // this cell's values before the arrival
+                prev = atomicAdd(&arrive[par], 1u);
+            }
+            prev = __shfl_sync(FULL, prev, 0);
+            if (prev + 1 != (unsigned)__popc(have)) break;  // a sibling's warp goes on
+            __threadfence();
+            // the children's values come from other SMs: read past the L1
+            double cm = 0, cx = 0, cy = 0, cz = 0, cr = 0;
+            if (ch >= 0) {
+                cm = __ldcg(cells.mass + ch);
+                cx = __ldcg(cells.cx + ch);
+                cy = __ldcg(cells.cy + ch);
+                cz = __ldcg(cells.cz + ch);
+                cr = __ldcg(cells.rho + ch);
+            }
+            const double px = cm * cx, py = cm * cy, pz = cm * cz;
+            double mass = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                const double vm = __shfl_sync(FULL, cm, o), vx = __shfl_sync(FULL, px, o),
+                             vy = __shfl_sync(FULL, py, o), vz = __shfl_sync(FULL, pz, o);
+                if ((have >> o) & 1) {
+                    mass += vm;
+                    sx += vx;
+                    sy += vy;
+                    sz += vz;
+                }
+            }
+            sx /= mass;
+            sy /= mass;
+            sz /= mass;
+            double rho = ch >= 0 ? cr + dist3(cx, cy, cz, sx, sy, sz) : 0.0;
+            for (int o = 4; o > 0; o >>= 1) rho = fmax(rho, __shfl_xor_sync(FULL, rho, o));
+            c = par;
+            if (lane == 0) {
+                rho = fmax(rho, 0.0);
+                cells.mass[c] = mass;
+                cells.cx[c] = sx;
+                cells.cy[c] = sy;
+                cells.cz[c] = sz;
+                cells.rho[c] = rho;
+                geo[c] = make_double4(sx, sy, sz, rho);
+            }
+        }
     }
 }
 
