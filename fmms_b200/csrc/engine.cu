@@ -221,9 +221,10 @@ struct fmmx_ctx {
     DBuf<uint32_t> list_cnt2, long_bounds2;
     // near-field work units of the mixed P2P (per leaf: units, scratch bodies)
     DBuf<uint32_t> p2p_units, p2p_scr, p2p_uoff, p2p_soff;
-    DBuf<uint32_t> p2p_units_s, p2p_units_b, p2p_uoff_s, p2p_uoff_b;  // small-leaf units apart
+    DBuf<int32_t> p2p_ucell;
+    uint32_t p2p_nunits = 0;
     DBuf<double4> p2p_part;
-    DBuf<float4> body_loc;  // mixed near field: bodies relative to their leaf's centre, FP32, with the mass
+    DBuf<float4> body_pairs;  // mixed near field: bodies relative to their leaf's centre, FP32, with the mass, in pairs
     DBuf<unsigned> p2p_next;
 
     DBuf<int> work;  // persistent-kernel work counter
@@ -681,22 +682,16 @@ fmmx_status list_launch(fmmx_ctx* ctx, bool near, cudaStream_t s, DBuf<char>& tm
                            near ? ctx->c_count.p : nullptr, near ? ctx->inter.p : nullptr, cnt.p, off.p, src_u.p,
                            src.p, longs.p, grid_for(npairs, 256), s),
        near ? "p2p lists" : "m2l lists");
-    const bool units = near && ctx->cfg.precision == FMMX_MIXED;
-    if (units) {
-        // near-field work units: per leaf ceil(sources / P2P_UNIT_SRC), and the
-        // scratch for the partial sums of leaves with several units
-        for (DBuf<uint32_t>* b : {&ctx->p2p_units, &ctx->p2p_scr, &ctx->p2p_uoff, &ctx->p2p_soff, &ctx->p2p_units_s,
-                                   &ctx->p2p_units_b, &ctx->p2p_uoff_s, &ctx->p2p_uoff_b})
+    if (near) {
+        // near-field work units and the scratch for the partial sums of leaves with several shares
+        for (DBuf<uint32_t>* b : {&ctx->p2p_units, &ctx->p2p_scr, &ctx->p2p_uoff, &ctx->p2p_soff})
             CK(b->ensure(nc + 1), "alloc lists");
-        CK(ctx->p2p_next.ensure(2), "alloc lists");
+        CK(ctx->p2p_next.ensure(1), "alloc lists");
         const DirList lp{nullptr, ctx->p2p_src.p, ctx->p2p_off.p, ctx->p2p_off.p + 1, 32};
-        launch_p2p_plan(grid_for(nc + 1, 256), s, nc, lp, ctx->c_count.p, ctx->p2p_units.p, ctx->p2p_units_s.p,
-                        ctx->p2p_units_b.p, ctx->p2p_scr.p);
+        launch_p2p_plan(grid_for(nc + 1, 256), s, nc, lp, ctx->c_count.p, ctx->p2p_units.p, ctx->p2p_scr.p);
         CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_units.p, ctx->p2p_uoff.p, nc + 1, s), "p2p units");
-        CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_units_s.p, ctx->p2p_uoff_s.p, nc + 1, s), "p2p units");
-        CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_units_b.p, ctx->p2p_uoff_b.p, nc + 1, s), "p2p units");
         CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_scr.p, ctx->p2p_soff.p, nc + 1, s), "p2p units");
-        LCOUNT(9);
+        LCOUNT(5);
     }
     return FMMX_OK;
 }
@@ -709,14 +704,23 @@ fmmx_status list_finish(fmmx_ctx* ctx, bool near, cudaStream_t s, DBuf<char>& tm
     DBuf<uint32_t>& src_u = near ? ctx->p2p_src_u : ctx->m2l_src_u;
     DBuf<uint32_t>& src = near ? ctx->p2p_src : ctx->m2l_src;
     DBuf<int>& longs = near ? ctx->p2p_longs : ctx->m2l_longs;
-    const bool units = near && ctx->cfg.precision == FMMX_MIXED;
     // host read-back: the number of long segments (and the P2P scratch size)
     int nlong = 0;
-    uint32_t nscr = 0;
+    uint32_t nscr = 0, nunits = 0;
     CK(cudaMemcpyAsync(&nlong, longs.p, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
-    if (units) CK(cudaMemcpyAsync(&nscr, ctx->p2p_soff.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "copy");
+    if (near) {
+        CK(cudaMemcpyAsync(&nscr, ctx->p2p_soff.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "copy");
+        CK(cudaMemcpyAsync(&nunits, ctx->p2p_uoff.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "copy");
+    }
     CK(cudaStreamSynchronize(s), "lists");
-    if (units) CK(ctx->p2p_part.ensure(std::max<size_t>(nscr, 1)), "alloc p2p scratch");
+    if (near) {
+        CK(ctx->p2p_part.ensure(std::max<size_t>(nscr, 1)), "alloc p2p scratch");
+        CK(ctx->p2p_ucell.ensure(std::max<size_t>(nunits, 1)), "alloc p2p scratch");
+        ctx->p2p_nunits = nunits;
+        launch_p2p_unit_cells(s, nc, ctx->p2p_uoff.p, ctx->p2p_ucell.p);
+        CKL("p2p units");
+        LCOUNT(1);
+    }
     if (nlong > 0) {
         const int end_bit = bits_for((uint64_t)nc);
         CK(bounds.ensure(2 * (size_t)nlong), "alloc lists");
@@ -729,6 +733,12 @@ fmmx_status list_finish(fmmx_ctx* ctx, bool near, cudaStream_t s, DBuf<char>& tm
     return FMMX_OK;
 }
 
+// the near field's work units, as list_launch and list_finish left them
+P2pUnits near_units(fmmx_ctx* ctx) {
+    return P2pUnits{ctx->p2p_uoff.p, ctx->p2p_ucell.p, ctx->p2p_soff.p, ctx->p2p_part.p, ctx->p2p_next.p,
+                    ctx->p2p_nunits};
+}
+
 // Mixed form, near field: FP32 + double-single P2P on the second stream.
 fmmx_status near_mixed(fmmx_ctx* ctx, const DirList& lp, bool tm) {
     cudaStream_t s2 = ctx->cfg.overlap ? ctx->stream2 : ctx->stream;
@@ -738,11 +748,9 @@ fmmx_status near_mixed(fmmx_ctx* ctx, const DirList& lp, bool tm) {
     cudaEvent_t* ev = ctx->ev;
     if (tm) CK(cudaEventRecord(ev[12], s2), "event");
     const float soft2 = (float)(ctx->cfg.softening * ctx->cfg.softening);
-    CK(cudaMemsetAsync(ctx->p2p_next.p, 0, 2 * sizeof(unsigned), s2), "memset");
-    const P2pUnits units{ctx->p2p_uoff.p, ctx->p2p_uoff_s.p, ctx->p2p_uoff_b.p, ctx->p2p_soff.p, ctx->p2p_part.p,
-                         ctx->p2p_next.p};
-    launch_p2p_mixed(ctx->cfg.p2p_tile > 0 ? ctx->cfg.p2p_tile : 512, ctx->nsm, s2, lp, nc, cv, units, n,
-                     ctx->body_leaf.p, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, ctx->body_loc.p, soft2, ctx->nax.p,
+    CK(cudaMemsetAsync(ctx->p2p_next.p, 0, sizeof(unsigned), s2), "memset");
+    launch_p2p_mixed(ctx->cfg.p2p_tile > 0 ? ctx->cfg.p2p_tile : 512, ctx->nsm, s2, lp, nc, cv, near_units(ctx), n,
+                     ctx->body_leaf.p, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, ctx->body_pairs.p, soft2, ctx->nax.p,
                      ctx->nay.p, ctx->naz.p, ctx->npot.p);
     CKL("p2p (mixed)");
     if (tm) CK(cudaEventRecord(ev[8], s2), "event");
@@ -771,7 +779,7 @@ fmmx_status far_mixed(fmmx_ctx* ctx, const DirList& lm, double* d_acc, double* d
         CK(launch_rotw_f32(p, lm, nc, cv, ctx->ellf.p, ctx->mom_f.p, ctx->loc_f.p, work, ctx->nsm, s), "m2l");
     }
     if (tm) CK(cudaEventRecord(ev[6], s), "event");
-    LCOUNT((ctx->n_m2l > 0 ? 1 : 0) + (ctx->nlevels - 1) + 5);  // m2l, l2l per level, coords + p2p (2) + combine, l2p
+    LCOUNT((ctx->n_m2l > 0 ? 1 : 0) + (ctx->nlevels - 1) + 4);  // m2l, l2l per level, pairs + p2p + combine, l2p
     for (int L = 1; L < ctx->nlevels; ++L) {
         const int cnt = ctx->lvl_count[L];
         const unsigned g = std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm);
@@ -821,7 +829,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     const int H = (p + 1) * (p + 2) / 2;
     const CellsView cv = view(ctx);
     if (mixed) {
-        CK(ctx->body_loc.ensure(n), "alloc expansions");
+        CK(ctx->body_pairs.ensure(p2p_pairs_floats4(n, nc)), "alloc expansions");
         CK(ctx->mom_f.ensure((size_t)nc * half_stride(p)), "alloc expansions");
         CK(ctx->loc_f.ensure((size_t)nc * half_stride(p)), "alloc expansions");
         CK(ctx->ell.ensure(nc), "alloc expansions");
@@ -943,8 +951,9 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     } else {
         if (tm) CK(cudaEventRecord(ev[12], s2), "event");
         const double soft2 = ctx->cfg.softening * ctx->cfg.softening;
-        k_p2p_f64<<<(unsigned)nc, 128, 0, s2>>>(lp, nc, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, soft2,
-                                                ctx->nax.p, ctx->nay.p, ctx->naz.p, ctx->npot.p);
+        CK(cudaMemsetAsync(ctx->p2p_next.p, 0, sizeof(unsigned), s2), "memset");
+        launch_p2p_f64(ctx->nsm, s2, lp, nc, cv, near_units(ctx), ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, soft2,
+                       ctx->nax.p, ctx->nay.p, ctx->naz.p, ctx->npot.p);
         CKL("p2p");
         if (tm) CK(cudaEventRecord(ev[8], s2), "event");
         CK(cudaEventRecord(ctx->fork[2], s2), "event");
@@ -984,7 +993,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         CKL("m2l");
     }
     if (tm) CK(cudaEventRecord(ev[6], s), "event");
-    LCOUNT((ctx->n_m2l > 0 ? 1 : 0) + (ctx->nlevels - 1) + 2);  // m2l, l2l per level, p2p, l2p
+    LCOUNT((ctx->n_m2l > 0 ? 1 : 0) + (ctx->nlevels - 1) + 3);  // m2l, l2l per level, p2p + combine, l2p
     {
         const size_t smem = 2 * (size_t)dim * sizeof(zd);
         for (int L = 1; L < ctx->nlevels; ++L) {

@@ -138,6 +138,49 @@ __global__ void k_l2p_f64(size_t n, const int32_t* body_leaf, const uint32_t* or
                           const zd* locals, const double* x, const double* y, const double* z, const double* nax,
                           const double* nay, const double* naz, const double* npot, double* acc, double* pot);
 
+// p2p.cu
+// Near-field work units (both forms): up to P2P_NT targets of a leaf against a
+// share of its source leaves, a warp each. Units of cell c: uoff[c] ..
+// uoff[c+1], ucell[u] the cell of unit u; the partial sums of a leaf with
+// several shares at part[soff[c] + share * count + i].
+#define P2P_NT 32
+struct P2pUnits {
+    const uint32_t* uoff;  // ncells + 1
+    const int32_t* ucell;  // nunits
+    const uint32_t* soff;  // ncells + 1
+    double4* part;
+    unsigned* next;  // work counter, zero at launch
+    uint32_t nunits;
+};
+
+// Work units of the near field, a warp each: up to P2P_NT targets of a leaf
+// against an equal share of its source leaves, p2p_shares(targets, sources) of
+// them. The share depends on the leaf alone -- about the same work per unit,
+// 2048 target-source-leaf products -- so a leaf in a dense core with thousands
+// of neighbours, or one of few leaves of a small system, spreads over many warps
+// (the load-balancing aim of the reference's split_fat, crates/visual/src/
+// gpufmm.rs:1350-1414). A leaf with one share writes its bodies' sums directly;
+// the shares of the others write partial sums, which k_p2p_combine adds per
+// body in share order (a fixed order: the results do not depend on which warp
+// ran which unit).
+__host__ __device__ __forceinline__ uint32_t p2p_shares(uint32_t nt, uint32_t len) {
+    const uint32_t t = nt < P2P_NT ? nt : P2P_NT;
+    uint32_t per = 2048u / (t > 0 ? t : 1u);
+    per = per > 512u ? 512u : per;
+    uint32_t s = (len + per - 1) / per;
+    const uint32_t most = (1u << 22) / (nt > 0 ? nt : 1u) + 1u;  // bounds the partial sums of a very large leaf
+    return s < most ? s : most;
+}
+
+void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
+                     uint32_t* scratch);
+void launch_p2p_unit_cells(cudaStream_t s, int ncells, const uint32_t* uoff, int32_t* ucell);
+void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,
+                        double* az, double* pot);
+void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const double* x,
+                    const double* y, const double* z, const double* m, double soft2, double* ax, double* ay,
+                    double* az, double* pot);
+
 // mixed.cu
 void upload_tables_mixed(const OrderTables& t, cudaStream_t s);
 __global__ void k_cell_scale(int nc, const double* rho, const double* h, double* ell, float* ellf);
@@ -155,31 +198,11 @@ __global__ void k_l2p_mixed(size_t n, const int32_t* body_leaf, const uint32_t* 
                             const double* ell, int p, const zf* loc, const double* x, const double* y,
                             const double* z, const double* nax, const double* nay, const double* naz,
                             const double* npot, double* acc, double* pot);
-// Near-field work units: the sources of a leaf in units of P2P_UNIT_SRC
-// source leaves (uoff: units of cell c at uoff[c] .. uoff[c+1]; soff: the
-// partial sums of a leaf with several units at part[soff[c] + k * count + i]).
-// The units of leaves of at most P2P_SMALL_NT bodies are numbered apart
-// (uoff_s) and run a warp each; the others (uoff_b) a block each.
-#define P2P_UNIT_SRC 1024
-#define P2P_SMALL_NT 32
-struct P2pUnits {
-    const uint32_t* uoff;    // ncells + 1, all units
-    const uint32_t* uoff_s;  // ncells + 1, units of small leaves
-    const uint32_t* uoff_b;  // ncells + 1, units of the other leaves
-    const uint32_t* soff;    // ncells + 1
-    double4* part;
-    unsigned* next;  // two work counters (small, other), zero at launch
-};
-void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
-                     uint32_t* units_s, uint32_t* units_b, uint32_t* scratch);
-// loc: n float4 of scratch (bodies relative to their leaf's centre, with the mass)
+// pairs: p2p_pairs_floats4 float4 of scratch (the bodies relative to their leaf's centre, with the mass, in pairs)
+size_t p2p_pairs_floats4(size_t n, int ncells);
 void launch_p2p_mixed(int tile, int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, size_t n,
                       const int32_t* body_leaf, const double* x, const double* y, const double* z, const double* m,
-                      float4* loc, float soft2, double* ax, double* ay, double* az, double* pot);
-
-// p2p.cu
-__global__ void k_p2p_f64(DirList L, int ncells, CellsView cv, const double* x, const double* y, const double* z,
-                          const double* m, double soft2, double* ax, double* ay, double* az, double* pot);
+                      float4* pairs, float soft2, double* ax, double* ay, double* az, double* pot);
 
 // integrate.cu
 __global__ void k_kick(size_t n3, double* v, const double* a, double h);

@@ -510,107 +510,53 @@ __global__ void k_l2p_mixed(size_t n, const int32_t* __restrict__ body_leaf, con
 }
 
 // ------------------------------------------------------------------ P2P
-// FP32 P2P with compensated accumulation. Source bodies are staged in shared
-// memory relative to the target leaf's centre (the FP64 subtraction), so the
-// FP32 differences d = x_j - x_i keep their relative precision; each thread
-// sums at least P2PM_FLUSH source pairs (two partial sums per component) in
-// FP32 and adds them into a double-single (hi, lo) accumulator with an
-// error-free TwoSum. 1/r by the hardware rsqrt.
-#define P2PM_BLOCK 128
-#define P2PM_SRC_CHUNK 256
-
-struct DS {
-    float hi, lo;
-};
-__device__ __forceinline__ void ds_add(DS& a, float b) {
-    const float s = a.hi + b;
-    const float bb = s - a.hi;
-    const float err = (a.hi - (s - bb)) + (b - bb);
-    a.hi = s;
-    a.lo += err;
-}
+// FP32 near field with FP64 sums. Bodies are kept relative to their own leaf's
+// centre in FP32 (the FP64 subtraction, once per evaluation); a source body is
+// moved to the target leaf's frame by its leaf's offset from the target leaf's
+// centre (an FP64 difference rounded once per source leaf), so d = x_j - x_i
+// carries roundings of quantities no larger than the pair's leaf separation.
+// A lane sums a few dozen source pairs in FP32 (two partial sums per
+// component) and adds them into FP64. 1/r by the hardware rsqrt.
 
 // The hardware reciprocal square root (about 2^-22 relative error), flushing
 // subnormal inputs: r2 is a squared distance plus the squared softening, far
 // above the subnormal range whenever it is positive. No Newton step: its
-// error is of the order of the FP32 rounding of the per-tile partial sums,
-// which dominates the near-field error. Measured at N = 2^20 (uniform cube,
-// p = 10, theta 0.5, 4096 targets against the FP64 direct sum): p99 relative
-// force error 1.3787e-6 with a Newton step, 1.3773e-6 without, P2P 2.96 ->
-// 2.58 ms; theta 0.3, p = 12: 6.42e-7 and 6.49e-7, 12.64 -> 10.98 ms.
+// error is of the order of the FP32 rounding of the partial sums, which
+// dominates the near-field error. Measured at N = 2^20 (uniform cube, p = 10,
+// theta 0.5, 4096 targets against the FP64 direct sum): p99 relative force
+// error 1.3787e-6 with a Newton step, 1.3773e-6 without; theta 0.3, p = 12:
+// 6.42e-7 and 6.49e-7.
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
-// One source body against one target, FP32, d relative to the target leaf's
-// centre.
-__device__ __forceinline__ void p2p_term(const float4 s, float xi, float yi, float zi, float soft2, float& ax,
-                                         float& ay, float& az, float& pt) {
-    const float dx = s.x - xi, dy = s.y - yi, dz = s.z - zi;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
-    const float inv = rsqrt_approx(r2);
-    const float mi = s.w * inv;
-    const float f = mi * inv * inv;
-    ax = fmaf(f, dx, ax);
-    ay = fmaf(f, dy, ay);
-    az = fmaf(f, dz, az);
-    pt += mi;
+// Source bodies in pairs, leaf by leaf (an odd leaf's last pair is padded with
+// a massless body far away): pair q of leaf c at pairs[2 (pair_base(c) + q)] =
+// (x, x', y, y') and the next float4 (z, z', m, m'), relative to the leaf's
+// centre. The bases are disjoint without a prefix sum: the next leaf's first
+// slot plus cell id exceeds this one's by at least count + 1.
+__host__ __device__ __forceinline__ uint32_t pair_base(uint32_t first, uint32_t c) {
+    return (uint32_t)(((uint64_t)first + c + 1) >> 1);
 }
+size_t p2p_pairs_floats4(size_t n, int ncells) { return 2 * ((n + (size_t)ncells + 1) / 2 + 1); }
 
-// Work units of the near field: the sources of leaf c are cut into units of
-// P2P_UNIT_SRC source leaves, units[c] = ceil(len / P2P_UNIT_SRC), so a leaf
-// in a dense cluster core with thousands of neighbours spreads over many
-// blocks instead of holding one block to the end of the launch (the
-// load-balancing aim of the reference's split_fat, crates/visual/src/
-// gpufmm.rs:1350-1414). A leaf with one unit writes its bodies' sums
-// directly; the units of a leaf with several write partial sums, which
-// k_p2p_combine adds per body in unit order (a fixed order: the results do
-// not depend on which block ran which unit).
-__global__ void k_p2p_plan(int ncells, DirList L, const uint32_t* __restrict__ count, uint32_t* __restrict__ units,
-                           uint32_t* __restrict__ units_s, uint32_t* __restrict__ units_b,
-                           uint32_t* __restrict__ scratch) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x) {
-        uint32_t nu = 0;
-        bool small = false;
-        if (c < ncells) {
-            const uint32_t len = L.seg_end[c] - L.seg_begin[c];
-            nu = (len + P2P_UNIT_SRC - 1) / P2P_UNIT_SRC;
-            small = count[c] <= P2P_SMALL_NT;
-        }
-        units[c] = nu;
-        units_s[c] = small ? nu : 0;
-        units_b[c] = small ? 0 : nu;
-        scratch[c] = nu > 1 ? nu * count[c] : 0;
-    }
-}
-
-__device__ __forceinline__ int unit_cell(const uint32_t* __restrict__ uoff, int ncells, uint32_t u) {
-    int lo = 0, hi = ncells;  // the last c with uoff[c] <= u
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (uoff[mid] <= u) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Body coordinates relative to their own leaf's centre, FP32, with the mass:
-// computed once per evaluation (the FP64 subtraction), so that staging a
-// source body for the near field is one 16-byte load plus its leaf's offset
-// from the target leaf's centre (c_s - c_t, FP64 rounded to FP32 once per
-// source leaf). The difference d = x_j - x_i then carries three FP32
-// roundings of quantities no larger than the pair's leaf separation instead
-// of one: the same order of absolute error.
-__global__ void k_local_coords(size_t n, const int32_t* __restrict__ body_leaf, CellsView cv,
-                               const double* __restrict__ x, const double* __restrict__ y,
-                               const double* __restrict__ z, const double* __restrict__ m,
-                               float4* __restrict__ loc) {
+__global__ void k_local_pairs(size_t n, const int32_t* __restrict__ body_leaf, CellsView cv,
+                              const double* __restrict__ x, const double* __restrict__ y,
+                              const double* __restrict__ z, const double* __restrict__ m, float* __restrict__ pairs) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         const int c = body_leaf[k];
-        loc[k] = make_float4((float)(x[k] - cv.cx[c]), (float)(y[k] - cv.cy[c]), (float)(z[k] - cv.cz[c]),
-                             (float)m[k]);
+        const uint32_t f = cv.first[c], i = (uint32_t)k - f;
+        float* o = pairs + 8 * ((size_t)pair_base(f, (uint32_t)c) + (i >> 1)) + (i & 1);
+        o[0] = (float)(x[k] - cv.cx[c]);
+        o[2] = (float)(y[k] - cv.cy[c]);
+        o[4] = (float)(z[k] - cv.cz[c]);
+        o[6] = (float)m[k];
+        if ((i & 1) == 0 && i + 1 == cv.count[c]) {
+            o[1] = 1e18f;
+            o[3] = o[5] = o[7] = 0.f;
+        }
     }
 }
 
@@ -646,457 +592,196 @@ __device__ __forceinline__ void mask_self(float4& a, float4& b, int h, float x, 
     }
 }
 
-// TILE: source bodies staged per shared-memory tile (the tile shape the
-// autotuner picks), as pairs: ta[q] = (x_2q, x_2q+1, y_2q, y_2q+1),
-// tz[q] = (z_2q, z_2q+1, m_2q, m_2q+1), an odd tile padded with a massless
-// body far away. Each thread carries two targets, so every staged pair feeds
-// four interactions; groups of G threads cover the leaf's targets and
-// R = BLOCK / G groups split each tile's pairs. The target's own body is
-// masked only in the tiles that overlap the target leaf itself. Blocks are
-// persistent and take units from a counter.
-//
-// The sources are taken in chunks of at most P2PM_SRC_CHUNK source leaves and
-// P2PM_MAP bodies: a chunk's bodies are numbered consecutively and own[]
-// gives each body's leaf in the chunk, so staging a body is a table lookup
-// (a leaf of more than P2PM_MAP bodies is a chunk of its own, without the
-// table). A target chunk's sums over the R groups are reduced by all threads,
-// S threads per output in fixed strips and a fixed shuffle tree.
-#define P2PM_MAP 4096
+// A warp per work unit, persistent, no block barriers. Two targets per lane:
+// groups of G = ceil(nt / 2) lanes hold the targets and R = 32 / G groups split
+// the source pairs of each tile. The sources are taken in chunks of up to
+// P2PW_CHUNK leaves and P2PW_MAP pairs; a table gives each pair's leaf, so that
+// staging a pair is a lookup, two 16-byte loads, six additions and two 16-byte
+// stores, and the next tile's loads are in flight while a tile is computed. The
+// target's own body is masked only in the tiles that overlap the target leaf.
+// Bound by issue: per interaction 7.5 packed FP32x2 and MUFU instructions plus
+// staging shared by the unit's targets.
+#define P2PW_CHUNK 128
+#define P2PW_MAP 1024
+#define P2PW_WARPS 4
 #define P2PM_FLUSH 16
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Start copying the bodies of the tile [b0, b0 + nb) of a chunk to raw[]:
-// thread tid takes pairs tid, tid + BLOCK, ...; lq[] keeps each body's leaf
-// in the chunk (-1: padding past the tile's end).
-template <int PPT>
-__device__ __forceinline__ void stage_issue(uint32_t b0, uint32_t nb, int tid, bool mapped,
-                                            const uint8_t* own, const uint32_t* sbase,
-                                            const float4* __restrict__ loc, float4* raw, int* lq) {
-    const int npair = (int)(nb + 1) >> 1;
-#pragma unroll
-    for (int e = 0; e < PPT; ++e) {
-        const int q = tid + e * P2PM_BLOCK;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t gg = b0 + 2u * (uint32_t)q + (uint32_t)h;
-            lq[2 * e + h] = -1;
-            if (q < npair && gg < b0 + nb) {
-                const int l = mapped ? (int)own[gg] : 0;
-                lq[2 * e + h] = l;
-                cp_async16(raw + 2 * q + h, loc + (gg + sbase[l]));
-            }
-        }
-    }
-    cp_async_commit();
-}
-
-// Finish the bodies this thread copied: wait for its copies, add the leaf
-// offsets and write the pair layout.
-template <int PPT>
-__device__ __forceinline__ void stage_finish(int npair, int tid, const float4* raw, const float4* soff,
-                                             const int* lq, float4* ta, float4* tz) {
-    cp_async_wait_all();
-#pragma unroll
-    for (int e = 0; e < PPT; ++e) {
-        const int q = tid + e * P2PM_BLOCK;
-        if (q < npair) {
-            float4 s2[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int l = lq[2 * e + h];
-                if (l >= 0) {
-                    const float4 v = raw[2 * q + h];
-                    const float4 o = soff[l];
-                    s2[h] = make_float4(v.x + o.x, v.y + o.y, v.z + o.z, v.w);
-                } else {
-                    s2[h] = make_float4(1e18f, 0.f, 0.f, 0.f);  // massless padding
-                }
-            }
-            ta[q] = make_float4(s2[0].x, s2[1].x, s2[0].y, s2[1].y);
-            tz[q] = make_float4(s2[0].z, s2[1].z, s2[0].w, s2[1].w);
-        }
-    }
-}
-template <int P2PM_TILE>
-__global__ void __launch_bounds__(P2PM_BLOCK, 5) k_p2p_mixed(DirList L, int ncells, CellsView cv, P2pUnits U,
-                                                         const float4* __restrict__ loc, float soft2_1,
-                                                         double* __restrict__ ax, double* __restrict__ ay,
-                                                         double* __restrict__ az, double* __restrict__ pot) {
-    constexpr int NPAIR = P2PM_TILE / 2;
-    constexpr int PPT = (NPAIR + P2PM_BLOCK - 1) / P2PM_BLOCK;  // pairs staged per thread
-    __shared__ float4 ta[NPAIR];
-    __shared__ float4 tz[NPAIR];
-    // the next tile's bodies as copied (leaf-relative); also the per-group
-    // sums at the end of a target chunk, when no copy is in flight
-    __shared__ float4 raw[P2PM_TILE > 512 ? P2PM_TILE : 512];
-    float(*red)[P2PM_BLOCK] = reinterpret_cast<float(*)[P2PM_BLOCK]>(raw);
-    static_assert(sizeof(raw) >= 16 * P2PM_BLOCK * sizeof(float), "the group sums alias the copy buffer");
-    __shared__ uint32_t pre[P2PM_SRC_CHUNK + 1];
-    __shared__ uint32_t sbase[P2PM_SRC_CHUNK];  // first slot of the leaf - its first position in the chunk
-    __shared__ float4 soff[P2PM_SRC_CHUNK];     // source leaf centre - target leaf centre
-    __shared__ uint8_t own[P2PM_MAP];
-    __shared__ uint32_t wsum[P2PM_BLOCK / 32];
-    __shared__ int self_pos, nuse_sh;
-    __shared__ uint32_t unit_sh;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, wid = tid >> 5;
-    const uint32_t nunits = U.uoff_b[ncells];
-    const float2 soft2 = make_float2(soft2_1, soft2_1);
-    for (;;) {
-        if (tid == 0) unit_sh = atomicAdd(U.next + 1, 1u);
-        __syncthreads();
-        const uint32_t u = unit_sh;
-        __syncthreads();
-        if (u >= nunits) break;
-        const int c = unit_cell(U.uoff_b, ncells, u);
-        const uint32_t k = u - U.uoff_b[c], nu = U.uoff[c + 1] - U.uoff[c];
-        const uint32_t beg = L.seg_begin[c] + k * P2P_UNIT_SRC;
-        const uint32_t end = min(L.seg_end[c], beg + P2P_UNIT_SRC);
-        const double cx = cv.cx[c], cy = cv.cy[c], cz = cv.cz[c];
-        const uint32_t tf = cv.first[c], tn = cv.count[c];
-        for (uint32_t t0 = 0; t0 < tn; t0 += 2 * P2PM_BLOCK) {
-            const int nt = (int)min((uint32_t)(2 * P2PM_BLOCK), tn - t0);
-            const int G = (nt + 1) >> 1;
-            const int R = P2PM_BLOCK / G;
-            const int g = tid % G, rep = tid / G;
-            const bool active = rep < R;
-            const int i0 = g, i1 = g + G;
-            const bool has1 = active && i1 < nt;
-            float x0 = 0, y0 = 0, z0 = 0, x1 = 0, y1 = 0, z1 = 0;
-            if (active) {
-                const float4 v = loc[tf + t0 + i0];
-                x0 = v.x; y0 = v.y; z0 = v.z;
-            }
-            if (has1) {
-                const float4 v = loc[tf + t0 + i1];
-                x1 = v.x; y1 = v.y; z1 = v.z;
-            }
-            const float2 nx0 = make_float2(-x0, -x0), ny0 = make_float2(-y0, -y0), nz0 = make_float2(-z0, -z0);
-            const float2 nx1 = make_float2(-x1, -x1), ny1 = make_float2(-y1, -y1), nz1 = make_float2(-z1, -z1);
-            DS a0x{0, 0}, a0y{0, 0}, a0z{0, 0}, p0{0, 0}, a1x{0, 0}, a1y{0, 0}, a1z{0, 0}, p1{0, 0};
-            // FP32 partial sums, added into the double-single sums once they
-            // hold P2PM_FLUSH source pairs (and at the end)
-            float2 q0x{0, 0}, q0y{0, 0}, q0z{0, 0}, q0p{0, 0}, q1x{0, 0}, q1y{0, 0}, q1z{0, 0}, q1p{0, 0};
-            int held = 0;
-            auto flush = [&]() {
-                ds_add(a0x, q0x.x + q0x.y);
-                ds_add(a0y, q0y.x + q0y.y);
-                ds_add(a0z, q0z.x + q0z.y);
-                ds_add(p0, q0p.x + q0p.y);
-                ds_add(a1x, q1x.x + q1x.y);
-                ds_add(a1y, q1y.x + q1y.y);
-                ds_add(a1z, q1z.x + q1z.y);
-                ds_add(p1, q1p.x + q1p.y);
-                q0x = q0y = q0z = q0p = q1x = q1y = q1z = q1p = make_float2(0.f, 0.f);
-                held = 0;
-            };
-            for (uint32_t sc = beg; sc < end;) {
-                const int ns = (int)min((uint32_t)P2PM_SRC_CHUNK, end - sc);
-                __syncthreads();
-                if (tid == 0) self_pos = -1;
-                // exclusive prefix of source leaf sizes (warp scans, then warp totals)
-                int myq[2] = {-1, -1};
-                for (int q0 = 0, h = 0; q0 < ns; q0 += P2PM_BLOCK, ++h) {
-                    const int q = q0 + tid;
-                    uint32_t v = 0;
-                    int src = -1;
-                    if (q < ns) {
-                        src = (int)L.src(L.key(sc + q));
-                        v = cv.count[src];
-                        soff[q] = make_float4((float)(cv.cx[src] - cx), (float)(cv.cy[src] - cy),
-                                              (float)(cv.cz[src] - cz), 0.f);
-                        myq[h] = src;
-                    }
-                    uint32_t incl = v;
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += t;
-                    }
-                    if (lane == 31) wsum[wid] = incl;
-                    __syncthreads();
-                    uint32_t base = q0 == 0 ? 0 : pre[q0];
-                    for (int w = 0; w < wid; ++w) base += wsum[w];
-                    if (q < ns) {
-                        pre[q + 1] = base + incl;
-                        sbase[q] = cv.first[src] - (base + incl - v);
-                    }
-                    if (q0 == 0 && tid == 0) pre[0] = 0;
-                    __syncthreads();
-                }
-                // the leaves whose bodies fit in the table (at least one)
-                int fit = 0;
-                for (int q = tid; q < ns; q += P2PM_BLOCK) fit += pre[q + 1] <= P2PM_MAP ? 1 : 0;
-                if (tid == 0) nuse_sh = 0;
-                __syncthreads();
-                if (fit) atomicAdd(&nuse_sh, fit);
-                __syncthreads();
-                const int nl = max(1, nuse_sh);
-                const bool mapped = pre[nl] <= P2PM_MAP;
-                for (int h = 0; h < 2; ++h) {
-                    const int q = tid + h * P2PM_BLOCK;
-                    if (q < nl) {
-                        if (myq[h] == c) self_pos = (int)pre[q];
-                        if (mapped)
-                            for (uint32_t e = pre[q]; e < pre[q + 1]; ++e) own[e] = (uint8_t)q;
-                    }
-                }
-                __syncthreads();
-                const uint32_t total = pre[nl];
-                const int sp = self_pos;  // position of the target leaf in this chunk's sources, or -1
-                sc += nl;
-                // tile k + 1's bodies are copied to raw[] (cp.async) while tile k
-                // is computed; each thread later finishes the bodies it copied
-                // (its leaf's offset added, pair layout), so only the tile
-                // hand-over needs a block barrier
-                int lq_cur[2 * PPT], lq_nxt[2 * PPT];
-                stage_issue<PPT>(0, min((uint32_t)P2PM_TILE, total), tid, mapped, own, sbase, loc, raw, lq_cur);
-                for (uint32_t b0 = 0; b0 < total; b0 += P2PM_TILE) {
-                    const uint32_t nb = min((uint32_t)P2PM_TILE, total - b0);
-                    const int npair = (int)(nb + 1) >> 1;
-                    stage_finish<PPT>(npair, tid, raw, soff, lq_cur, ta, tz);
-                    __syncthreads();
-                    if (b0 + P2PM_TILE < total)
-                        stage_issue<PPT>(b0 + P2PM_TILE, min((uint32_t)P2PM_TILE, total - b0 - P2PM_TILE), tid,
-                                         mapped, own, sbase, loc, raw, lq_nxt);
-                    if (active) {
-                        const bool overlaps = sp >= 0 && (uint32_t)sp < b0 + nb && (uint32_t)sp + tn > b0;
-                        if (!overlaps) {
-#pragma unroll 2
-                            for (int j = rep; j < npair; j += R) {
-                                const float4 a = ta[j], b = tz[j];
-                                p2p_pair(a, b, nx0, ny0, nz0, soft2, q0x, q0y, q0z, q0p);
-                                p2p_pair(a, b, nx1, ny1, nz1, soft2, q1x, q1y, q1z, q1p);
-                            }
-                        } else {
-                            // the target's own body sits at position sp + t0 + i in the sources
-                            const int s0 = sp + (int)t0 + i0 - (int)b0, s1 = sp + (int)t0 + i1 - (int)b0;
-                            for (int j = rep; j < npair; j += R) {
-                                const float4 a = ta[j], b = tz[j];
-                                float4 a0 = a, b0v = b, a1 = a, b1v = b;
-                                if (s0 >= 0 && j == (s0 >> 1)) mask_self(a0, b0v, s0 & 1, x0, y0, z0);
-                                if (s1 >= 0 && j == (s1 >> 1)) mask_self(a1, b1v, s1 & 1, x1, y1, z1);
-                                p2p_pair(a0, b0v, nx0, ny0, nz0, soft2, q0x, q0y, q0z, q0p);
-                                p2p_pair(a1, b1v, nx1, ny1, nz1, soft2, q1x, q1y, q1z, q1p);
-                            }
-                        }
-                        held += (npair - rep + R - 1) / R;
-                        if (held >= P2PM_FLUSH) flush();
-                    }
-                    __syncthreads();
-#pragma unroll
-                    for (int e = 0; e < 2 * PPT; ++e) lq_cur[e] = lq_nxt[e];
-                }
-            }
-            flush();
-            red[0][tid] = a0x.hi; red[1][tid] = a0x.lo; red[2][tid] = a0y.hi; red[3][tid] = a0y.lo;
-            red[4][tid] = a0z.hi; red[5][tid] = a0z.lo; red[6][tid] = p0.hi; red[7][tid] = p0.lo;
-            red[8][tid] = a1x.hi; red[9][tid] = a1x.lo; red[10][tid] = a1y.hi; red[11][tid] = a1y.lo;
-            red[12][tid] = a1z.hi; red[13][tid] = a1z.lo; red[14][tid] = p1.hi; red[15][tid] = p1.lo;
-            __syncthreads();
-            // outputs: nt targets x 4 components; S threads per output (a power
-            // of two up to 32, so an output's threads share a warp)
-            const int nout = 4 * nt;
-            int S = 1;
-            while (S < 32 && 2 * S * nout <= P2PM_BLOCK) S <<= 1;
-            for (int o0 = 0; o0 < nout; o0 += P2PM_BLOCK / S) {
-                const int o = o0 + tid / S, st = tid % S;
-                double v = 0.0;
-                if (o < nout) {
-                    const int t = o >> 2, comp = o & 3;
-                    const int gi = t % G, half = t / G;  // target t = gi + half * G
-                    const int row = 8 * half + 2 * comp;
-                    for (int r = st; r < R; r += S) {
-                        const int q = r * G + gi;
-                        v += (double)red[row][q] + (double)red[row + 1][q];
-                    }
-                }
-                for (int w = S >> 1; w > 0; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w, S);
-                if (o < nout && st == 0) {
-                    const int t = o >> 2, comp = o & 3;
-                    if (nu == 1) {
-                        double* out = comp == 0 ? ax : comp == 1 ? ay : comp == 2 ? az : pot;
-                        out[tf + t0 + t] = v;
-                    } else {
-                        reinterpret_cast<double*>(U.part + U.soff[c] + k * tn + t0 + t)[comp] = v;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// Small target leaves (at most P2P_SMALL_NT bodies): a warp per work unit,
-// four independent warps per block, warp-synchronous (no block barriers).
-// With a few targets per leaf, a block per unit spends most of its
-// instructions on what every thread repeats per tile and per unit (the loop
-// setup, the barriers, the group reduction, finding the unit's leaf); a warp
-// pays them over a quarter of the threads. Same arithmetic as the block
-// kernel: two targets per lane, groups of G = ceil(nt / 2) lanes, R = 32 / G
-// groups over each tile's source pairs, packed FP32x2 interactions,
-// double-single sums, the leaf table for staging (chunks of at most
-// P2PW_CHUNK leaves and P2PW_MAP bodies), the target's own body masked.
-#define P2PW_TILE 128
-#define P2PW_CHUNK 128
-#define P2PW_MAP 2048
-#define P2PW_WARPS 4
+template <int TP>  // source pairs per tile
 struct P2pWarpSmem {
-    float4 ta[P2PW_TILE / 2];
-    float4 tz[P2PW_TILE / 2];
-    float4 soff[P2PW_CHUNK];
-    uint32_t pre[P2PW_CHUNK + 1];
-    uint32_t sbase[P2PW_CHUNK];
-    float red[16][32];
-    uint8_t own[P2PW_MAP];
+    union {
+        struct {
+            float4 ta[TP];  // (x, x', y, y')
+            float4 tz[TP];  // (z, z', m, m')
+        } t;
+        double red[8][32];  // the groups' sums at the end of a unit
+    };
+    float4 soff[P2PW_CHUNK];  // source leaf's centre - target leaf's centre; w: first pair of the leaf - its
+                              // first position in the chunk (as bits)
+    uint8_t own[P2PW_MAP];    // leaf of each pair of the chunk
 };
 
-__global__ void __launch_bounds__(32 * P2PW_WARPS) k_p2p_mixed_small(DirList L, int ncells, CellsView cv, P2pUnits U,
-                                                                     const float4* __restrict__ loc, float soft2_1,
-                                                                     double* __restrict__ ax, double* __restrict__ ay,
-                                                                     double* __restrict__ az,
-                                                                     double* __restrict__ pot) {
-    __shared__ P2pWarpSmem smem_w[P2PW_WARPS];
+template <int TP>
+__global__ void __launch_bounds__(32 * P2PW_WARPS, 5) k_p2p_mixed(DirList L, CellsView cv, P2pUnits U,
+                                                                const float4* __restrict__ pairs, float soft2_1,
+                                                                double* __restrict__ ax, double* __restrict__ ay,
+                                                                double* __restrict__ az, double* __restrict__ pot) {
+    constexpr int PPT = TP / 32;  // pairs staged per lane
+    __shared__ P2pWarpSmem<TP> smem_w[P2PW_WARPS];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    P2pWarpSmem& S = smem_w[threadIdx.x >> 5];
-    const uint32_t nunits = U.uoff_s[ncells];
+    P2pWarpSmem<TP>& S = smem_w[threadIdx.x >> 5];
     const float2 soft2 = make_float2(soft2_1, soft2_1);
     for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(U.next, 1u);
         u = __shfl_sync(FULL, u, 0);
-        if (u >= nunits) break;
-        const int c = unit_cell(U.uoff_s, ncells, u);
-        const uint32_t k = u - U.uoff_s[c], nu = U.uoff[c + 1] - U.uoff[c];
-        const uint32_t beg = L.seg_begin[c] + k * P2P_UNIT_SRC;
-        const uint32_t end = min(L.seg_end[c], beg + P2P_UNIT_SRC);
-        const double cx = cv.cx[c], cy = cv.cy[c], cz = cv.cz[c];
-        const uint32_t tf = cv.first[c];
-        const int nt = (int)cv.count[c];  // <= P2P_SMALL_NT (32) by the plan
+        if (u >= U.nunits) break;
+        const int c = U.ucell[u];
+        const uint32_t lb = L.seg_begin[c], len = L.seg_end[c] - lb;
+        const uint32_t tf = cv.first[c], tn = cv.count[c];
+        const uint32_t ns_all = p2p_shares(tn, len);
+        const uint32_t k = u - U.uoff[c], share = k % ns_all, t0 = (k / ns_all) * P2P_NT;
+        const uint32_t beg = lb + (uint32_t)((uint64_t)len * share / ns_all);
+        const uint32_t end = lb + (uint32_t)((uint64_t)len * (share + 1) / ns_all);
+        const double4 gc = cv.geo[c];
+        const int nt = (int)min((uint32_t)P2P_NT, tn - t0);
         const int G = (nt + 1) >> 1;
         const int R = 32 / G;
         const int g = lane % G, rep = lane / G;
         const bool active = rep < R;
-        const int i0 = g, i1 = g + G;
-        const bool has1 = active && i1 < nt;
-        float x0 = 0, y0 = 0, z0 = 0, x1 = 0, y1 = 0, z1 = 0;
-        if (active) {
-            const float4 v = loc[tf + i0];
-            x0 = v.x; y0 = v.y; z0 = v.z;
-        }
-        if (has1) {
-            const float4 v = loc[tf + i1];
-            x1 = v.x; y1 = v.y; z1 = v.z;
+        const int i0 = g, i1 = min(g + G, nt - 1);  // (an odd last target is computed twice, written once)
+        float x0, y0, z0, x1, y1, z1;
+        {
+            const float* tp = reinterpret_cast<const float*>(pairs) + 8 * (size_t)pair_base(tf, (uint32_t)c);
+            const uint32_t b0 = t0 + i0, b1 = t0 + i1;
+            const float* q0 = tp + 8 * (size_t)(b0 >> 1) + (b0 & 1);
+            const float* q1 = tp + 8 * (size_t)(b1 >> 1) + (b1 & 1);
+            x0 = q0[0]; y0 = q0[2]; z0 = q0[4];
+            x1 = q1[0]; y1 = q1[2]; z1 = q1[4];
         }
         const float2 nx0 = make_float2(-x0, -x0), ny0 = make_float2(-y0, -y0), nz0 = make_float2(-z0, -z0);
         const float2 nx1 = make_float2(-x1, -x1), ny1 = make_float2(-y1, -y1), nz1 = make_float2(-z1, -z1);
-        DS a0x{0, 0}, a0y{0, 0}, a0z{0, 0}, p0{0, 0}, a1x{0, 0}, a1y{0, 0}, a1z{0, 0}, p1{0, 0};
+        double a0x = 0, a0y = 0, a0z = 0, p0 = 0, a1x = 0, a1y = 0, a1z = 0, p1 = 0;
+        // FP32 partial sums, added into the FP64 sums once they hold
+        // P2PM_FLUSH source pairs (and at the end)
         float2 q0x{0, 0}, q0y{0, 0}, q0z{0, 0}, q0p{0, 0}, q1x{0, 0}, q1y{0, 0}, q1z{0, 0}, q1p{0, 0};
         int held = 0;
         auto flush = [&]() {
-            ds_add(a0x, q0x.x + q0x.y);
-            ds_add(a0y, q0y.x + q0y.y);
-            ds_add(a0z, q0z.x + q0z.y);
-            ds_add(p0, q0p.x + q0p.y);
-            ds_add(a1x, q1x.x + q1x.y);
-            ds_add(a1y, q1y.x + q1y.y);
-            ds_add(a1z, q1z.x + q1z.y);
-            ds_add(p1, q1p.x + q1p.y);
+            a0x += (double)(q0x.x + q0x.y);
+            a0y += (double)(q0y.x + q0y.y);
+            a0z += (double)(q0z.x + q0z.y);
+            p0 += (double)(q0p.x + q0p.y);
+            a1x += (double)(q1x.x + q1x.y);
+            a1y += (double)(q1y.x + q1y.y);
+            a1z += (double)(q1z.x + q1z.y);
+            p1 += (double)(q1p.x + q1p.y);
             q0x = q0y = q0z = q0p = q1x = q1y = q1z = q1p = make_float2(0.f, 0.f);
             held = 0;
         };
         for (uint32_t sc = beg; sc < end;) {
             const int ns = (int)min((uint32_t)P2PW_CHUNK, end - sc);
             __syncwarp();
-            // exclusive prefix of the chunk's source leaf sizes (one warp scan
-            // per 32 leaves, carried over); each lane remembers where the
-            // target leaf itself lies, if it holds it
-            uint32_t base = 0;
-            int self_q = P2PW_CHUNK, self_at = -1;
-            for (int q0 = 0; q0 < ns; q0 += 32) {
-                const int q = q0 + lane;
-                uint32_t v = 0;
-                int src = -1;
-                if (q < ns) {
-                    src = (int)L.src(L.key(sc + q));
-                    v = cv.count[src];
-                    S.soff[q] = make_float4((float)(cv.cx[src] - cx), (float)(cv.cy[src] - cy),
-                                            (float)(cv.cz[src] - cz), 0.f);
+            // the chunk's source leaves: all loads of a kind at once, then the
+            // positions of their pairs (one warp scan per 32 leaves)
+            int src[P2PW_CHUNK / 32];
+            uint32_t np[P2PW_CHUNK / 32], pb[P2PW_CHUNK / 32];
+#pragma unroll
+            for (int h = 0; h < P2PW_CHUNK / 32; ++h) {
+                const int q = lane + 32 * h;
+                src[h] = q < ns ? (int)L.keys32[sc + q] : -1;
+            }
+#pragma unroll
+            for (int h = 0; h < P2PW_CHUNK / 32; ++h) {
+                np[h] = 0;
+                pb[h] = 0;
+                if (src[h] >= 0) {
+                    np[h] = (cv.count[src[h]] + 1) >> 1;
+                    pb[h] = pair_base(cv.first[src[h]], (uint32_t)src[h]);
+                    const double4 gs = cv.geo[src[h]];
+                    S.soff[lane + 32 * h] = make_float4((float)(gs.x - gc.x), (float)(gs.y - gc.y),
+                                                        (float)(gs.z - gc.z), 0.f);
                 }
-                uint32_t incl = v;
+            }
+            uint32_t base = 0;
+            int nl = 0, self_at = -1;  // leaves whose pairs fit in the table; the target leaf's first position
+#pragma unroll
+            for (int h = 0; h < P2PW_CHUNK / 32; ++h) {
+                const int q = lane + 32 * h;
+                uint32_t incl = np[h];
+#pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(FULL, incl, o);
                     if (lane >= o) incl += t;
                 }
-                if (q < ns) {
-                    const uint32_t excl = base + incl - v;
-                    S.pre[q + 1] = excl + v;
-                    S.sbase[q] = cv.first[src] - excl;
-                    if (src == c) {
-                        self_q = q;
-                        self_at = (int)excl;
+                incl += base;
+                const uint32_t excl = incl - np[h];
+                const bool fits = src[h] >= 0 && (incl <= P2PW_MAP || (q == 0));
+                nl += __popc(__ballot_sync(FULL, fits));
+                if (fits) {
+                    S.soff[q].w = __uint_as_float(pb[h] - excl);
+                    if (src[h] == c) self_at = (int)excl;
+                    if (incl <= P2PW_MAP)
+                        for (uint32_t e = excl; e < incl; ++e) S.own[e] = (uint8_t)q;
+                }
+                if (fits) np[h] = incl;  // keeps the last leaf's end
+                base = __shfl_sync(FULL, incl, 31);
+            }
+            // pairs of the nl leaves: the end of the last one
+            uint32_t total = 0;
+#pragma unroll
+            for (int h = 0; h < P2PW_CHUNK / 32; ++h) {
+                const uint32_t v = __shfl_sync(FULL, np[h], (nl - 1) & 31);
+                if ((nl - 1) >> 5 == h) total = v;
+            }
+            const bool mapped = total <= P2PW_MAP;
+            const int sp = __reduce_max_sync(FULL, self_at);
+            __syncwarp();
+            sc += nl;
+            float4 ra[PPT], rz[PPT], ro[PPT];
+            auto issue = [&](uint32_t b0) {  // load the pairs of the tile at b0
+#pragma unroll
+                for (int e = 0; e < PPT; ++e) {
+                    const uint32_t p = b0 + lane + 32 * e;
+                    if (p < total) {
+                        ro[e] = S.soff[mapped ? S.own[p] : 0];
+                        const float4* s = pairs + 2 * (size_t)(p + __float_as_uint(ro[e].w));
+                        ra[e] = s[0];
+                        rz[e] = s[1];
                     }
                 }
-                base += __shfl_sync(FULL, incl, 31);
-            }
-            if (lane == 0) S.pre[0] = 0;
-            __syncwarp();
-            // the leaves whose bodies fit in the table (at least one)
-            unsigned fit = 0;
-            for (int q = lane; q < ns; q += 32) fit += S.pre[q + 1] <= P2PW_MAP ? 1u : 0u;
-            const int nl = max(1, (int)__reduce_add_sync(FULL, fit));
-            const bool mapped = S.pre[nl] <= P2PW_MAP;
-            const int sp = __reduce_max_sync(FULL, self_q < nl ? self_at : -1);
-            if (mapped)
-                for (int q = lane; q < nl; q += 32)
-                    for (uint32_t e = S.pre[q]; e < S.pre[q + 1]; ++e) S.own[e] = (uint8_t)q;
-            __syncwarp();
-            const uint32_t total = S.pre[nl];
-            sc += nl;
-            for (uint32_t b0 = 0; b0 < total; b0 += P2PW_TILE) {
-                const uint32_t nb = min((uint32_t)P2PW_TILE, total - b0);
-                const int npair = (int)(nb + 1) >> 1;
-                for (int q = lane; q < npair; q += 32) {
-                    float4 s2[2];
+            };
+            issue(0);
+            for (uint32_t b0 = 0; b0 < total; b0 += TP) {
+                const int npair = (int)min((uint32_t)TP, total - b0);
+                __syncwarp();
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t gg = b0 + 2u * (uint32_t)q + (uint32_t)h;
-                        if (gg < b0 + nb) {
-                            const int l = mapped ? (int)S.own[gg] : 0;
-                            const float4 v = loc[gg + S.sbase[l]];
-                            const float4 o = S.soff[l];
-                            s2[h] = make_float4(v.x + o.x, v.y + o.y, v.z + o.z, v.w);
-                        } else {
-                            s2[h] = make_float4(1e18f, 0.f, 0.f, 0.f);  // massless padding
-                        }
+                for (int e = 0; e < PPT; ++e) {
+                    const int p = lane + 32 * e;
+                    if (p < npair) {
+                        const float4 o = ro[e];
+                        S.t.ta[p] = make_float4(ra[e].x + o.x, ra[e].y + o.x, ra[e].z + o.y, ra[e].w + o.y);
+                        S.t.tz[p] = make_float4(rz[e].x + o.z, rz[e].y + o.z, rz[e].z, rz[e].w);
                     }
-                    S.ta[q] = make_float4(s2[0].x, s2[1].x, s2[0].y, s2[1].y);
-                    S.tz[q] = make_float4(s2[0].z, s2[1].z, s2[0].w, s2[1].w);
                 }
                 __syncwarp();
+                issue(b0 + TP);
                 if (active) {
-                    const bool overlaps = sp >= 0 && (uint32_t)sp < b0 + nb && (uint32_t)sp + (uint32_t)nt > b0;
-                    if (!overlaps) {
+                    const int last = sp + (int)((tn + 1) >> 1);  // the target leaf's own pairs: sp .. last - 1
+                    if (sp < 0 || sp >= (int)b0 + npair || last <= (int)b0) {
 #pragma unroll 2
                         for (int j = rep; j < npair; j += R) {
-                            const float4 a = S.ta[j], b = S.tz[j];
+                            const float4 a = S.t.ta[j], b = S.t.tz[j];
                             p2p_pair(a, b, nx0, ny0, nz0, soft2, q0x, q0y, q0z, q0p);
                             p2p_pair(a, b, nx1, ny1, nz1, soft2, q1x, q1y, q1z, q1p);
                         }
                     } else {
-                        // the target's own body sits at position sp + i in the sources
-                        const int s0 = sp + i0 - (int)b0, s1 = sp + i1 - (int)b0;
+                        // the target's own body is body t0 + i of the leaf
+                        const int s0 = 2 * (sp - (int)b0) + (int)t0 + i0, s1 = 2 * (sp - (int)b0) + (int)t0 + i1;
                         for (int j = rep; j < npair; j += R) {
-                            const float4 a = S.ta[j], b = S.tz[j];
+                            const float4 a = S.t.ta[j], b = S.t.tz[j];
                             float4 a0 = a, b0v = b, a1 = a, b1v = b;
-                            if (s0 >= 0 && j == (s0 >> 1)) mask_self(a0, b0v, s0 & 1, x0, y0, z0);
-                            if (s1 >= 0 && j == (s1 >> 1)) mask_self(a1, b1v, s1 & 1, x1, y1, z1);
+                            if (j == (s0 >> 1)) mask_self(a0, b0v, s0 & 1, x0, y0, z0);
+                            if (j == (s1 >> 1)) mask_self(a1, b1v, s1 & 1, x1, y1, z1);
                             p2p_pair(a0, b0v, nx0, ny0, nz0, soft2, q0x, q0y, q0z, q0p);
                             p2p_pair(a1, b1v, nx1, ny1, nz1, soft2, q1x, q1y, q1z, q1p);
                         }
@@ -1104,98 +789,54 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS) k_p2p_mixed_small(DirList L, 
                     held += (npair - rep + R - 1) / R;
                     if (held >= P2PM_FLUSH) flush();
                 }
-                __syncwarp();
             }
         }
         flush();
-        S.red[0][lane] = a0x.hi; S.red[1][lane] = a0x.lo; S.red[2][lane] = a0y.hi; S.red[3][lane] = a0y.lo;
-        S.red[4][lane] = a0z.hi; S.red[5][lane] = a0z.lo; S.red[6][lane] = p0.hi; S.red[7][lane] = p0.lo;
-        S.red[8][lane] = a1x.hi; S.red[9][lane] = a1x.lo; S.red[10][lane] = a1y.hi; S.red[11][lane] = a1y.lo;
-        S.red[12][lane] = a1z.hi; S.red[13][lane] = a1z.lo; S.red[14][lane] = p1.hi; S.red[15][lane] = p1.lo;
+        __syncwarp();
+        S.red[0][lane] = a0x; S.red[1][lane] = a0y; S.red[2][lane] = a0z; S.red[3][lane] = p0;
+        S.red[4][lane] = a1x; S.red[5][lane] = a1y; S.red[6][lane] = a1z; S.red[7][lane] = p1;
         __syncwarp();
         // outputs: nt targets x 4 components, each the sum over the R groups
         // in group order
         for (int o = lane; o < 4 * nt; o += 32) {
             const int t = o >> 2, comp = o & 3;
-            const int gi = t % G, half = t / G;  // target t = gi + half * G
-            const int row = 8 * half + 2 * comp;
+            const int gi = t < G ? t : t - G;  // target t = gi + half * G
+            const int row = (t < G ? 0 : 4) + comp;
             double v = 0.0;
-            for (int r = 0; r < R; ++r) v += (double)S.red[row][r * G + gi] + (double)S.red[row + 1][r * G + gi];
-            if (nu == 1) {
+            for (int r = 0; r < R; ++r) v += S.red[row][r * G + gi];
+            if (ns_all == 1) {
                 double* out = comp == 0 ? ax : comp == 1 ? ay : comp == 2 ? az : pot;
-                out[tf + t] = v;
+                out[tf + t0 + t] = v;
             } else {
-                reinterpret_cast<double*>(U.part + U.soff[c] + k * (uint32_t)nt + t)[comp] = v;
+                reinterpret_cast<double*>(U.part + U.soff[c] + (size_t)share * tn + t0 + t)[comp] = v;
             }
         }
         __syncwarp();
     }
 }
 
-// The bodies of the leaves with several units: the units' partial sums, in
-// unit order (one warp per leaf).
-__global__ void k_p2p_combine(int ncells, CellsView cv, P2pUnits U, double* __restrict__ ax, double* __restrict__ ay,
-                              double* __restrict__ az, double* __restrict__ pot) {
-    const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
-        const uint32_t nu = U.uoff[c + 1] - U.uoff[c];
-        if (nu <= 1) continue;
-        const uint32_t tn = cv.count[c], tf = cv.first[c];
-        const double4* pp = U.part + U.soff[c];
-        for (uint32_t i = lane; i < tn; i += 32) {
-            double4 s = pp[i];
-            for (uint32_t k = 1; k < nu; ++k) {
-                const double4 v = pp[k * tn + i];
-                s.x += v.x;
-                s.y += v.y;
-                s.z += v.z;
-                s.w += v.w;
-            }
-            ax[tf + i] = s.x;
-            ay[tf + i] = s.y;
-            az[tf + i] = s.z;
-            pot[tf + i] = s.w;
-        }
-    }
-}
-
-void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
-                     uint32_t* units_s, uint32_t* units_b, uint32_t* scratch) {
-    k_p2p_plan<<<grid, 256, 0, s>>>(ncells, L, count, units, units_s, units_b, scratch);
-}
-
-template <int TILE>
-static void launch_tile(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const float4* loc,
-                        float soft2, double* ax, double* ay, double* az, double* pot) {
-    // persistent blocks: as many as fit on an SM at once (capping them at four
-    // to leave room for the far field's list kernels beside the P2P was
-    // measured: the P2P lost more, 31.5 -> 35.8 ms at the clustered
-    // N = 2^22 workload, than the lists gained)
+template <int TP>
+static void launch_tile(int nsm, cudaStream_t s, DirList L, CellsView cv, P2pUnits U, const float4* pairs, float soft2,
+                        double* ax, double* ay, double* az, double* pot) {
+    // persistent blocks: as many as fit on an SM at once, no more than there are units
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p_mixed<TILE>, P2PM_BLOCK, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p_mixed<TP>, 32 * P2PW_WARPS, 0) != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
-    k_p2p_mixed<TILE><<<nsm * per_sm, P2PM_BLOCK, 0, s>>>(L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
+    const unsigned need = (unsigned)std::min<uint64_t>(((uint64_t)U.nunits + P2PW_WARPS - 1) / P2PW_WARPS, 1u << 30);
+    k_p2p_mixed<TP><<<std::max(1u, std::min(need, (unsigned)(nsm * per_sm))), 32 * P2PW_WARPS, 0, s>>>(
+        L, cv, U, pairs, soft2, ax, ay, az, pot);
 }
 
 void launch_p2p_mixed(int tile, int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, size_t n,
                       const int32_t* body_leaf, const double* x, const double* y, const double* z, const double* m,
-                      float4* loc, float soft2, double* ax, double* ay, double* az, double* pot) {
-    k_local_coords<<<grid_for(n, 256), 256, 0, s>>>(n, body_leaf, cv, x, y, z, m, loc);
-    {  // the small leaves' units, a warp each, persistent
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p_mixed_small, 32 * P2PW_WARPS, 0) !=
-                cudaSuccess ||
-            per_sm < 1)
-            per_sm = 1;
-        k_p2p_mixed_small<<<nsm * per_sm, 32 * P2PW_WARPS, 0, s>>>(L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
-    }
-    if (tile <= 128) launch_tile<128>(nsm, s, L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
-    else if (tile <= 256) launch_tile<256>(nsm, s, L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
-    else if (tile <= 512) launch_tile<512>(nsm, s, L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
-    else launch_tile<1024>(nsm, s, L, ncells, cv, U, loc, soft2, ax, ay, az, pot);
-    k_p2p_combine<<<grid_for((size_t)ncells * 32, 256), 256, 0, s>>>(ncells, cv, U, ax, ay, az, pot);
+                      float4* pairs, float soft2, double* ax, double* ay, double* az, double* pot) {
+    k_local_pairs<<<grid_for(n, 256), 256, 0, s>>>(n, body_leaf, cv, x, y, z, m, reinterpret_cast<float*>(pairs));
+    // `tile` bodies per block of four warps: 64 pairs per warp's tile at 512
+    if (tile <= 256) launch_tile<32>(nsm, s, L, cv, U, pairs, soft2, ax, ay, az, pot);
+    else if (tile <= 512) launch_tile<64>(nsm, s, L, cv, U, pairs, soft2, ax, ay, az, pot);
+    else launch_tile<128>(nsm, s, L, cv, U, pairs, soft2, ax, ay, az, pot);
+    launch_p2p_combine(s, ncells, L, cv, U, ax, ay, az, pot);
 }
 
 }  // namespace fmmx

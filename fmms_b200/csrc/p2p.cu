@@ -1,126 +1,275 @@
-// P2P: direct near-field interactions over the directed leaf list.
-//
-// One CTA per target leaf. The leaf's source leaves (its own included) are
-// streamed through shared memory in tiles of bodies; each target body is held
-// by R = BLOCK / targets threads that split the tile's bodies and are reduced
-// in a fixed order at the end, so results are deterministic and every thread
-// works even for small leaves. A target skips its own slot (the i != j of the
-// reference's self kernel, p2p.rs:13-46).
+// Near field: the work units of both forms, and the plain (FP64) P2P over the
+// directed leaf list.
 //
 // Interaction (p2p.rs:24-39, with optional Plummer softening s^2):
 //   d = x_j - x_i, r2 = |d|^2 + s^2, inv = 1/sqrt(r2),
-//   a_i += m_j inv^3 d, pot_i += m_j inv.
+//   a_i += m_j inv^3 d, pot_i += m_j inv,
+// a target skipping its own body (the i != j of the reference's self kernel,
+// p2p.rs:13-46).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
 namespace fmmx {
 
-#define P2P_BLOCK 128
-#define P2P_TILE 128
-#define P2P_SRC_CHUNK 256
+// Units, shares and leaves of units: see P2pUnits and p2p_shares.
+__global__ void k_p2p_plan(int ncells, DirList L, const uint32_t* __restrict__ count, uint32_t* __restrict__ units,
+                           uint32_t* __restrict__ scratch) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x) {
+        uint32_t nu = 0, sc = 0;
+        if (c < ncells) {
+            const uint32_t len = L.seg_end[c] - L.seg_begin[c], nt = count[c];
+            const uint32_t s = p2p_shares(nt, len);
+            nu = s * ((nt + P2P_NT - 1) / P2P_NT);
+            sc = s > 1 ? s * nt : 0;
+        }
+        units[c] = nu;
+        scratch[c] = sc;
+    }
+}
 
-__global__ void __launch_bounds__(P2P_BLOCK) k_p2p_f64(DirList L, int ncells, CellsView cv,
-                                                      const double* __restrict__ x, const double* __restrict__ y,
-                                                      const double* __restrict__ z, const double* __restrict__ m,
-                                                      double soft2, double* __restrict__ ax, double* __restrict__ ay,
-                                                      double* __restrict__ az, double* __restrict__ pot) {
-    __shared__ double tx[P2P_TILE], ty[P2P_TILE], tz[P2P_TILE], tm[P2P_TILE];
-    __shared__ uint32_t tslot[P2P_TILE];
-    __shared__ uint32_t pre[P2P_SRC_CHUNK + 1];
-    __shared__ uint32_t sfirst[P2P_SRC_CHUNK];
-    __shared__ double red[4][P2P_BLOCK];
-    const int tid = threadIdx.x;
-    for (int c = blockIdx.x; c < ncells; c += gridDim.x) {
-        const uint32_t beg = L.seg_begin[c], end = L.seg_end[c];
-        if (beg >= end) continue;
-        const uint32_t tf = cv.first[c], tn = cv.count[c];
-        for (uint32_t t0 = 0; t0 < tn; t0 += P2P_BLOCK) {
-            const int nt = (int)min((uint32_t)P2P_BLOCK, tn - t0);
-            const int R = P2P_BLOCK / nt;
-            const int it = tid % nt, rep = tid / nt;
-            const bool active = rep < R;
-            const uint32_t islot = tf + t0 + it;
-            double xi = 0, yi = 0, zi = 0;
-            if (active) {
-                xi = x[islot];
-                yi = y[islot];
-                zi = z[islot];
+// the leaf of every unit
+__global__ void k_p2p_unit_cells(int ncells, const uint32_t* __restrict__ uoff, int32_t* __restrict__ ucell) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x)
+        for (uint32_t u = uoff[c]; u < uoff[c + 1]; ++u) ucell[u] = c;
+}
+
+// The bodies of the leaves with several shares: the shares' partial sums, in
+// share order (one warp per leaf).
+__global__ void k_p2p_combine(int ncells, DirList L, CellsView cv, P2pUnits U, double* __restrict__ ax,
+                              double* __restrict__ ay, double* __restrict__ az, double* __restrict__ pot) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
+        if (U.soff[c + 1] == U.soff[c]) continue;
+        const uint32_t tn = cv.count[c], tf = cv.first[c];
+        const uint32_t nu = p2p_shares(tn, L.seg_end[c] - L.seg_begin[c]);
+        const double4* pp = U.part + U.soff[c];
+        for (uint32_t i = lane; i < tn; i += 32) {
+            double4 s = pp[i];
+            for (uint32_t k = 1; k < nu; ++k) {
+                const double4 v = pp[(size_t)k * tn + i];
+                s.x += v.x;
+                s.y += v.y;
+                s.z += v.z;
+                s.w += v.w;
             }
-            double sax = 0.0, say = 0.0, saz = 0.0, sp = 0.0;
-            for (uint32_t sc = beg; sc < end; sc += P2P_SRC_CHUNK) {
-                const int ns = (int)min((uint32_t)P2P_SRC_CHUNK, end - sc);
-                __syncthreads();
-                // exclusive prefix of the chunk's source leaf sizes
-                for (int q = tid; q < ns; q += P2P_BLOCK) {
-                    const int src = (int)L.src(L.key(sc + q));
-                    pre[q + 1] = cv.count[src];
-                    sfirst[q] = cv.first[src];
-                }
-                if (tid == 0) pre[0] = 0;
-                __syncthreads();
-                if (tid == 0)
-                    for (int q = 1; q <= ns; ++q) pre[q] += pre[q - 1];
-                __syncthreads();
-                const uint32_t total = pre[ns];
-                for (uint32_t b0 = 0; b0 < total; b0 += P2P_TILE) {
-                    const uint32_t nb = min((uint32_t)P2P_TILE, total - b0);
-                    if ((uint32_t)tid < nb) {
-                        const uint32_t g = b0 + tid;
-                        int lo = 0, hi = ns;  // last q with pre[q] <= g
-                        while (hi - lo > 1) {
-                            int mid = (lo + hi) >> 1;
-                            if (pre[mid] <= g) lo = mid;
-                            else hi = mid;
-                        }
-                        const uint32_t slot = sfirst[lo] + (g - pre[lo]);
-                        tx[tid] = x[slot];
-                        ty[tid] = y[slot];
-                        tz[tid] = z[slot];
-                        tm[tid] = m[slot];
-                        tslot[tid] = slot;
-                    }
-                    __syncthreads();
-                    if (active) {
-                        for (uint32_t j = rep; j < nb; j += R) {
-                            if (tslot[j] == islot) continue;
-                            const double dx = tx[j] - xi, dy = ty[j] - yi, dz = tz[j] - zi;
-                            const double r2 = dx * dx + dy * dy + dz * dz + soft2;
-                            const double inv = rsqrt(r2);
-                            const double mj = tm[j];
-                            const double inv3 = inv * inv * inv;
-                            const double f = mj * inv3;
-                            sax += f * dx;
-                            say += f * dy;
-                            saz += f * dz;
-                            sp += mj * inv;
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            red[0][tid] = sax;
-            red[1][tid] = say;
-            red[2][tid] = saz;
-            red[3][tid] = sp;
-            __syncthreads();
-            if (tid < nt) {
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-                for (int r = 0; r < R; ++r) {
-                    const int q = r * nt + tid;
-                    s0 += red[0][q];
-                    s1 += red[1][q];
-                    s2 += red[2][q];
-                    s3 += red[3][q];
-                }
-                const uint32_t slot = tf + t0 + tid;
-                ax[slot] = s0;
-                ay[slot] = s1;
-                az[slot] = s2;
-                pot[slot] = s3;
-            }
-            __syncthreads();
+            ax[tf + i] = s.x;
+            ay[tf + i] = s.y;
+            az[tf + i] = s.z;
+            pot[tf + i] = s.w;
         }
     }
+}
+
+void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
+                     uint32_t* scratch) {
+    k_p2p_plan<<<grid, 256, 0, s>>>(ncells, L, count, units, scratch);
+}
+
+void launch_p2p_unit_cells(cudaStream_t s, int ncells, const uint32_t* uoff, int32_t* ucell) {
+    k_p2p_unit_cells<<<grid_for(ncells, 128), 128, 0, s>>>(ncells, uoff, ucell);
+}
+
+void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,
+                        double* az, double* pot) {
+    k_p2p_combine<<<grid_for((size_t)ncells * 32, 256), 256, 0, s>>>(ncells, L, cv, U, ax, ay, az, pot);
+}
+
+// ------------------------------------------------------------- plain form
+// A warp per work unit, persistent, no block barriers: two targets per lane,
+// groups of G = ceil(nt / 2) lanes over the targets, R = 32 / G groups over the
+// source bodies of each tile, reduced in group order at the end. A table gives
+// each source body's leaf, and the next tile's loads are in flight while a tile
+// is computed. Bound by the FP64 pipe (about 20 FP64 instructions per
+// interaction, the reciprocal square root half of them).
+#define P2PD_CHUNK 128
+#define P2PD_MAP 2048
+#define P2PD_TILE 64
+#define P2PD_WARPS 4
+
+struct P2pF64Smem {
+    union {
+        double4 t[P2PD_TILE];
+        double red[8][32];
+    };
+    uint32_t shift[P2PD_CHUNK];  // first slot of the leaf - its first position in the chunk
+    uint8_t own[P2PD_MAP];
+};
+
+template <bool SELF>
+__device__ __forceinline__ void p2p_f64_term(double x, double y, double z, double m, bool self, double xi, double yi,
+                                             double zi, double soft2, double& ax, double& ay, double& az, double& pt) {
+    const double dx = x - xi, dy = y - yi, dz = z - zi;
+    double r2 = dx * dx + dy * dy + dz * dz + soft2;
+    double mj = m;
+    if (SELF && self) {
+        r2 = 1.0;
+        mj = 0.0;
+    }
+    const double inv = rsqrt(r2);
+    const double mi = mj * inv;
+    const double f = mi * (inv * inv);
+    ax += f * dx;
+    ay += f * dy;
+    az += f * dz;
+    pt += mi;
+}
+
+__global__ void __launch_bounds__(32 * P2PD_WARPS, 5) k_p2p_f64(DirList L, CellsView cv, P2pUnits U,
+                                                              const double* __restrict__ x,
+                                                              const double* __restrict__ y,
+                                                              const double* __restrict__ z,
+                                                              const double* __restrict__ m, double soft2,
+                                                              double* __restrict__ ax, double* __restrict__ ay,
+                                                              double* __restrict__ az, double* __restrict__ pot) {
+    constexpr int BPT = P2PD_TILE / 32;  // bodies staged per lane
+    constexpr int H = P2PD_CHUNK / 32;
+    __shared__ P2pF64Smem smem_w[P2PD_WARPS];
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    P2pF64Smem& S = smem_w[threadIdx.x >> 5];
+    for (;;) {
+        uint32_t u = 0;
+        if (lane == 0) u = atomicAdd(U.next, 1u);
+        u = __shfl_sync(FULL, u, 0);
+        if (u >= U.nunits) break;
+        const int c = U.ucell[u];
+        const uint32_t lb = L.seg_begin[c], len = L.seg_end[c] - lb;
+        const uint32_t tf = cv.first[c], tn = cv.count[c];
+        const uint32_t ns_all = p2p_shares(tn, len);
+        const uint32_t k = u - U.uoff[c], share = k % ns_all, t0 = (k / ns_all) * P2P_NT;
+        const uint32_t beg = lb + (uint32_t)((uint64_t)len * share / ns_all);
+        const uint32_t end = lb + (uint32_t)((uint64_t)len * (share + 1) / ns_all);
+        const int nt = (int)min((uint32_t)P2P_NT, tn - t0);
+        const int G = (nt + 1) >> 1;
+        const int R = 32 / G;
+        const int g = lane % G, rep = lane / G;
+        const bool active = rep < R;
+        const int i0 = g, i1 = min(g + G, nt - 1);  // (an odd last target is computed twice, written once)
+        const uint32_t s0 = tf + t0 + i0, s1 = tf + t0 + i1;
+        const double x0 = x[s0], y0 = y[s0], z0 = z[s0], x1 = x[s1], y1 = y[s1], z1 = z[s1];
+        double a0x = 0, a0y = 0, a0z = 0, p0 = 0, a1x = 0, a1y = 0, a1z = 0, p1 = 0;
+        for (uint32_t sc = beg; sc < end;) {
+            const int ns = (int)min((uint32_t)P2PD_CHUNK, end - sc);
+            __syncwarp();
+            int src[H];
+            uint32_t nb[H], fs[H];
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const int q = lane + 32 * h;
+                src[h] = q < ns ? (int)L.keys32[sc + q] : -1;
+            }
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                nb[h] = src[h] >= 0 ? cv.count[src[h]] : 0;
+                fs[h] = src[h] >= 0 ? cv.first[src[h]] : 0;
+            }
+            uint32_t base = 0;
+            int nl = 0, self_at = -1;  // leaves whose bodies fit in the table; the target leaf's first position
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const int q = lane + 32 * h;
+                uint32_t incl = nb[h];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                incl += base;
+                const uint32_t excl = incl - nb[h];
+                const bool fits = src[h] >= 0 && (incl <= P2PD_MAP || q == 0);
+                nl += __popc(__ballot_sync(FULL, fits));
+                if (fits) {
+                    S.shift[q] = fs[h] - excl;
+                    if (src[h] == c) self_at = (int)excl;
+                    if (incl <= P2PD_MAP)
+                        for (uint32_t e = excl; e < incl; ++e) S.own[e] = (uint8_t)q;
+                    nb[h] = incl;  // keeps the last leaf's end
+                }
+                base = __shfl_sync(FULL, incl, 31);
+            }
+            uint32_t total = 0;
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const uint32_t v = __shfl_sync(FULL, nb[h], (nl - 1) & 31);
+                if ((nl - 1) >> 5 == h) total = v;
+            }
+            const bool mapped = total <= P2PD_MAP;
+            const int sp = __reduce_max_sync(FULL, self_at);
+            __syncwarp();
+            sc += nl;
+            double4 v[BPT];
+            auto issue = [&](uint32_t b0) {  // load the bodies of the tile at b0
+#pragma unroll
+                for (int e = 0; e < BPT; ++e) {
+                    const uint32_t p = b0 + lane + 32 * e;
+                    if (p < total) {
+                        const uint32_t slot = p + S.shift[mapped ? S.own[p] : 0];
+                        v[e] = make_double4(x[slot], y[slot], z[slot], m[slot]);
+                    }
+                }
+            };
+            issue(0);
+            for (uint32_t b0 = 0; b0 < total; b0 += P2PD_TILE) {
+                const int nbt = (int)min((uint32_t)P2PD_TILE, total - b0);
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < BPT; ++e)
+                    if (lane + 32 * e < nbt) S.t[lane + 32 * e] = v[e];
+                __syncwarp();
+                issue(b0 + P2PD_TILE);
+                if (active) {
+                    if (sp < 0 || sp >= (int)b0 + nbt || sp + (int)tn <= (int)b0) {
+                        for (int j = rep; j < nbt; j += R) {
+                            const double4 q = S.t[j];
+                            p2p_f64_term<false>(q.x, q.y, q.z, q.w, false, x0, y0, z0, soft2, a0x, a0y, a0z, p0);
+                            p2p_f64_term<false>(q.x, q.y, q.z, q.w, false, x1, y1, z1, soft2, a1x, a1y, a1z, p1);
+                        }
+                    } else {
+                        const int o0 = sp - (int)b0 + (int)t0 + i0, o1 = sp - (int)b0 + (int)t0 + i1;
+                        for (int j = rep; j < nbt; j += R) {
+                            const double4 q = S.t[j];
+                            p2p_f64_term<true>(q.x, q.y, q.z, q.w, j == o0, x0, y0, z0, soft2, a0x, a0y, a0z, p0);
+                            p2p_f64_term<true>(q.x, q.y, q.z, q.w, j == o1, x1, y1, z1, soft2, a1x, a1y, a1z, p1);
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        S.red[0][lane] = a0x; S.red[1][lane] = a0y; S.red[2][lane] = a0z; S.red[3][lane] = p0;
+        S.red[4][lane] = a1x; S.red[5][lane] = a1y; S.red[6][lane] = a1z; S.red[7][lane] = p1;
+        __syncwarp();
+        for (int o = lane; o < 4 * nt; o += 32) {
+            const int t = o >> 2, comp = o & 3;
+            const int gi = t < G ? t : t - G;  // target t = gi + half * G
+            const int row = (t < G ? 0 : 4) + comp;
+            double s = 0.0;
+            for (int r = 0; r < R; ++r) s += S.red[row][r * G + gi];
+            if (ns_all == 1) {
+                double* out = comp == 0 ? ax : comp == 1 ? ay : comp == 2 ? az : pot;
+                out[tf + t0 + t] = s;
+            } else {
+                reinterpret_cast<double*>(U.part + U.soff[c] + (size_t)share * tn + t0 + t)[comp] = s;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const double* x,
+                    const double* y, const double* z, const double* m, double soft2, double* ax, double* ay,
+                    double* az, double* pot) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p_f64, 32 * P2PD_WARPS, 0) != cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
+    const unsigned need = (unsigned)(((uint64_t)U.nunits + P2PD_WARPS - 1) / P2PD_WARPS);
+    k_p2p_f64<<<std::max(1u, std::min(need, (unsigned)(nsm * per_sm))), 32 * P2PD_WARPS, 0, s>>>(
+        L, cv, U, x, y, z, m, soft2, ax, ay, az, pot);
+    launch_p2p_combine(s, ncells, L, cv, U, ax, ay, az, pot);
 }
 
 }  // namespace fmmx
