@@ -862,8 +862,8 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     }
     if (dehnen) {
         CK(cudaMemsetAsync(ctx->flags.p + TF_STACK, 0, sizeof(int), s), "memset");
-        k_fprepass<<<grid_for(n, 128), 128, 0, s>>>(cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, n, ctx->sys_off.p,
-                                                    ctx->nsys, ctx->level_cells.p, ctx->f.p, ctx->flags.p + TF_STACK);
+        launch_fprepass(s, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, n, ctx->sys_off.p, ctx->nsys,
+                        ctx->level_cells.p, ctx->f.p, ctx->flags.p + TF_STACK);
         CKL("f pre-pass");
     }
     if (mixed && !dehnen) {

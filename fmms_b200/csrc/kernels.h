@@ -93,8 +93,10 @@ __global__ void k_upward_exact(const int32_t* level_cells, int lstart, int lcnt,
                                const double* f, double* fmin, int skip_internal);
 __global__ void k_m2m_exact_block(const int32_t* level_cells, int lstart, int lcnt, CellsView cells, int p,
                                   zd* moments, double* pows, const double* f, double* fmin);
-__global__ void k_fprepass(CellsView cells, const double* x, const double* y, const double* z, const double* m,
-                           size_t n, const uint64_t* off, int nsys, const int32_t* roots, double* f, int* err);
+#define FPRE_WARPS 2
+void launch_fprepass(cudaStream_t s, CellsView cells, const double* x, const double* y, const double* z,
+                     const double* m, size_t n, const uint64_t* off, int nsys, const int32_t* roots, double* f,
+                     int* err);
 // one dual-walk iteration over frontier `cur` (k_walk_iter<DEHNEN>: Dehnen's error-estimate MAC, else
 // theta and soft_gap), 256-thread blocks; and its resident blocks per SM
 void launch_walk_iter(bool dehnen, unsigned grid, cudaStream_t s, CellsView cv, MacParams mp, const double* pows,
