@@ -90,7 +90,7 @@ struct CellsView {
     const double* cz;
     const double* mass;
     const double* rho;
-    const double4* geo;  // cx, cy, cz, rho of each cell in one 32-byte record (the walk's loads)
+    const double4* geo;  // cx, cy, cz, rho of each cell in one 32-byte record, the sign of rho set for a leaf
 };
 
 // SM count of the device, read when a context is created (grid sizes of the

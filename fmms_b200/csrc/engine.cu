@@ -132,6 +132,10 @@ struct Status {
 // overflow, cells per level and leaves, level-list cursors
 enum { TF_BAD = 0, TF_STACK = 1, TF_LEVELS = 2, TF_CURSOR = TF_LEVELS + FMMX_NLEVELS + 1,
        TF_SIZE = TF_CURSOR + FMMX_NLEVELS };
+// 64-bit words of the walk's state: chunks used, overflow flag, totals (WalkLists), and per level the work
+// counters of the level and of its heavy cells and the number of those
+enum { WS_USED = 0, WS_OVERFLOW = 1, WS_TOTALS = 2, WS_WORK = 6, WS_HWORK = WS_WORK + FMMX_NLEVELS,
+       WS_HEAVY = WS_HWORK + FMMX_NLEVELS, WS_SIZE = WS_HEAVY + FMMX_NLEVELS };
 
 }  // namespace
 
@@ -203,24 +207,24 @@ struct fmmx_ctx {
     DBuf<unsigned long long> rho_now;  // radii about the build's centres on a reused tree (FP64 bits)
     DBuf<float> ellf;
 
-    // walk
-    DBuf<uint2> front0, front1, m2l, p2p;
-    DBuf<int> wcounts;
-    DBuf<unsigned long long> wpops, inter;
-    uint32_t cap_front = 0, cap_m2l = 0, cap_p2p = 0;
-    uint64_t walk_cap0 = 0;  // FMMX_TEST_WALK_CAPACITY (tests of the overflow retry); 0: sized by the tree
+    // walk: the pool of list chunks, per-cell results, counters (WS_*)
+    DBuf<uint32_t> pool_entry, pool_next, down_n, down_head;
+    DBuf<uint2> pool_owner;
+    DBuf<uint8_t> list_redone;
+    DBuf<uint4> list_sizes, list_off;
+    DBuf<unsigned long long> walk_state;
+    uint32_t cap_pool = 0;   // chunks
+    DBuf<double2> mac_rows;  // per cell for Dehnen's MAC
+    DBuf<int32_t> heavy_list;
+    DBuf<uint32_t> heavy_ring;
+    uint64_t walk_cap0 = 0;  // FMMX_TEST_WALK_CAPACITY (entries; tests of the overflow retry); 0: sized by the tree
     int walk_retries = 0;
 
-    // directed lists
-    // per destination cell c: sources src[off[c] .. off[c+1]), ascending
-    DBuf<uint32_t> m2l_src_u, m2l_src, p2p_src_u, p2p_src;  // scattered, then sorted within segments
-    DBuf<uint32_t> m2l_off, p2p_off, list_cnt;               // nc + 1 each
-    DBuf<int> m2l_longs, p2p_longs;                         // long-segment lists, 2 nc + 128 each
-    DBuf<uint32_t> long_bounds;
-    DBuf<char> cub_tmp2;                // the M2L list's sort scratch (built beside the P2P)
-    DBuf<uint32_t> list_cnt2, long_bounds2;
-    // near-field work units of the mixed P2P (per leaf: units, scratch bodies)
-    DBuf<uint32_t> p2p_units, p2p_scr, p2p_uoff, p2p_soff;
+    // directed lists: per destination cell c the sources src[off[c] .. off[c+1])
+    DBuf<uint32_t> m2l_src, p2p_src;
+    DBuf<uint32_t> m2l_off, p2p_off;  // nc + 1 each
+    // near-field work units (per leaf: first unit, first partial sum)
+    DBuf<uint32_t> p2p_uoff, p2p_soff;
     DBuf<int32_t> p2p_ucell;
     uint32_t p2p_nunits = 0;
     DBuf<double4> p2p_part;
@@ -229,7 +233,6 @@ struct fmmx_ctx {
 
     DBuf<int> work;  // persistent-kernel work counter
     int nsm = 148;
-    int walk_blocks[2] = {0, 0};  // resident blocks of k_walk_iter<theta, Dehnen> on the whole device
     uint64_t launches = 0, launches_build = 0;
 
     fmmx_stats st;
@@ -273,7 +276,7 @@ fmmx_status finish(fmmx_ctx* ctx, fmmx_status st) {
     ctx->drop_graph();
     for (DBufBase* b : ctx->cache) b->release();
     ctx->built = ctx->evaluated = ctx->lists_valid = false;
-    ctx->cap_front = ctx->cap_m2l = ctx->cap_p2p = 0;
+    ctx->cap_pool = 0;
     return st;
 }
 
@@ -480,7 +483,7 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     const uint32_t n32 = (uint32_t)n, n_leaf = (uint32_t)ctx->cfg.n_leaf;
     const unsigned gt = (unsigned)((n + 1 + TREE_BLOCK * TREE_PER_THREAD - 1) / (TREE_BLOCK * TREE_PER_THREAD));
     CK(ctx->cell_id0.ensure(n + 1), "alloc cells");
-    tb = directed_list_temp(0, (int)n);
+    tb = scan_u32_temp((int)(n + 1));
     CK(ctx->cub_tmp.ensure(tb), "alloc scan");
     k_cell_count<<<gt, TREE_BLOCK, 0, s>>>(ctx->keys_sorted.p, n32, ctx->sys_off.p, nsys, n_leaf, ctx->idx.p,
                                            ctx->flags.p + TF_LEVELS);
@@ -535,8 +538,7 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
                                                                 view_mut(ctx), ctx->x.p, ctx->y.p, ctx->z.p,
                                                                 ctx->m.p, ctx->cfg.center_mode);
         }
-        k_pack_geo<<<grid_for(nc, 256), 256, 0, s>>>(nc, ctx->c_cx.p, ctx->c_cy.p, ctx->c_cz.p, ctx->c_rho.p,
-                                                     ctx->c_geo.p);
+        k_pack_geo<<<grid_for(nc, 256), 256, 0, s>>>(nc, view_mut(ctx), ctx->c_geo.p);
         LCOUNT(nlev);
     }
     CKL("geometry");
@@ -555,23 +557,28 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
 }
 
 // ---------------------------------------------------------------- evaluate
+// The walk and the interaction lists on stream s, with the lists' sizes read
+// back once in between; returns with the lists queued.
 fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     const int nc = ctx->nc;
-    // capacities follow the current tree (a context may see trees of very
-    // different sizes, e.g. the forests of a serving loop) and grow on overflow
-    auto at_least = [](uint32_t c, uint64_t w) { return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(c, w), 0x7fffffffull); };
-    if (ctx->walk_cap0 > 0) {  // test knob: start from the given capacity (and grow on overflow)
-        ctx->cap_front = at_least(ctx->cap_front, ctx->walk_cap0);
-        ctx->cap_m2l = at_least(ctx->cap_m2l, ctx->walk_cap0);
-        ctx->cap_p2p = at_least(ctx->cap_p2p, ctx->walk_cap0);
-    } else {
-        ctx->cap_front = at_least(ctx->cap_front, 64ull * nc + 1024);
-        ctx->cap_m2l = at_least(ctx->cap_m2l, 64ull * nc + 1024);
-        ctx->cap_p2p = at_least(ctx->cap_p2p, 32ull * nc + 1024);
-    }
+    // the pool's capacity follows the current tree (a context may see trees of
+    // very different sizes, e.g. the forests of a serving loop) and grows on overflow
+    const uint64_t most = 1ull << 28;
+    // chunks per cell at the first attempt (uniform systems take about 40); a context with a budget starts small
+    const uint64_t per = ctx->budget.limit || nc < 4096 ? 24 : 44;
+    const uint64_t want = ctx->walk_cap0 > 0 ? std::max<uint64_t>(ctx->walk_cap0 / 32, 1) : per * nc + 256;
+    ctx->cap_pool = (uint32_t)std::min(std::max<uint64_t>(ctx->cap_pool, want), most);
     ctx->walk_retries = 0;
-    CK(ctx->wcounts.ensure(WC_SIZE), "alloc");
-    CK(ctx->wpops.ensure(1), "alloc");
+    CK(ctx->walk_state.ensure(WS_SIZE), "alloc walk");
+    CK(ctx->down_n.ensure(nc), "alloc walk");
+    CK(ctx->down_head.ensure(nc), "alloc walk");
+    CK(ctx->list_redone.ensure(nc), "alloc walk");
+    CK(ctx->list_sizes.ensure(nc + 1), "alloc walk");
+    CK(ctx->list_off.ensure(nc + 1), "alloc walk");
+    for (DBuf<uint32_t>* b : {&ctx->m2l_off, &ctx->p2p_off, &ctx->p2p_uoff, &ctx->p2p_soff})
+        CK(b->ensure(nc + 1), "alloc lists");
+    const size_t tb = scan_u32x4_temp(nc + 1);
+    CK(ctx->cub_tmp.ensure(tb), "alloc scan");
     MacParams mp;
     mp.mode = ctx->cfg.mac_mode;
     mp.p = ctx->cfg.p;
@@ -579,161 +586,80 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     mp.theta = ctx->cfg.theta;
     mp.gap = ctx->cfg.soft_gap * ctx->cfg.softening;
     const CellsView cv = view(ctx);
+    const bool dehnen = mp.mode == FMMX_MAC_DEHNEN;
+    if (dehnen) {
+        CK(ctx->mac_rows.ensure((size_t)nc * (mp.p + 2)), "alloc walk");
+        k_mac_rows<<<grid_for(nc, 128), 128, 0, s>>>(nc, cv, mp.p, ctx->pows.p, ctx->fmin.p, ctx->mac_rows.p);
+        LCOUNT(1);
+    }
+    WalkHeavy heavy{nullptr, nullptr, nullptr, (uint32_t)ctx->nleaves, 0};
+    if (walk_needs_heavy(ctx->lvl_count, ctx->nlevels, ctx->nleaves)) {
+        heavy.blocks = walk_heavy_blocks(ctx->nleaves);
+        CK(ctx->heavy_list.ensure(nc), "alloc walk");
+        CK(ctx->heavy_ring.ensure((size_t)heavy.blocks * (size_t)ctx->nleaves), "alloc walk");
+        heavy.list = ctx->heavy_list.p;
+        heavy.ring = ctx->heavy_ring.p;
+    }
+    unsigned long long hs[WS_SIZE];
+    uint4 sizes;
+    WalkPool pool;
+    const WalkLists lists{ctx->down_n.p, ctx->down_head.p, ctx->list_redone.p, ctx->list_sizes.p,
+                          ctx->walk_state.p + WS_TOTALS};
     for (int attempt = 0;; ++attempt) {
-        CK(ctx->front0.ensure(ctx->cap_front), "alloc walk");
-        CK(ctx->front1.ensure(ctx->cap_front), "alloc walk");
-        CK(ctx->m2l.ensure(ctx->cap_m2l), "alloc walk");
-        CK(ctx->p2p.ensure(ctx->cap_p2p), "alloc walk");
-        WalkBufs w;
-        w.front[0] = ctx->front0.p;
-        w.front[1] = ctx->front1.p;
-        w.m2l = ctx->m2l.p;
-        w.p2p = ctx->p2p.p;
-        w.counts = ctx->wcounts.p;
-        w.pops_ptr = ctx->wpops.p;
-        w.cap_front = ctx->cap_front;
-        w.cap_m2l = ctx->cap_m2l;
-        w.cap_p2p = ctx->cap_p2p;
-        CK(cudaMemsetAsync(ctx->wcounts.p, 0, WC_SIZE * sizeof(int), s), "memset");
-        CK(cudaMemsetAsync(ctx->wpops.p, 0, sizeof(unsigned long long), s), "memset");
-        // seeds: the self pair of every root (one per system)
-        k_walk_init<<<grid_for(ctx->nsys, 128), 128, 0, s>>>(ctx->level_cells.p, ctx->nsys, ctx->front0.p);
-        LCOUNT(1);
-        const int seeds = ctx->nsys;  // pageable source: staged before the call returns
-        CK(cudaMemcpyAsync(ctx->wcounts.p + WC_FRONT0, &seeds, sizeof(int), cudaMemcpyHostToDevice, s), "copy");
-        int cur = 0;
-        int hc[WC_SIZE];
-        bool done = false;
-        const int max_iter = 8 * FMMX_NLEVELS + 16;
-        // One kernel per MAC, so the theta form carries none of the Dehnen
-        // estimate's registers (54 against 80: four resident blocks per SM
-        // instead of three), launched with exactly the resident blocks: the
-        // grid-stride loop then runs in one wave instead of a last, partly
-        // filled one.
-        const bool dehnen = mp.mode == FMMX_MAC_DEHNEN;
-        int& wb = ctx->walk_blocks[dehnen ? 1 : 0];
-        if (wb == 0) wb = walk_iter_blocks_per_sm(dehnen) * ctx->nsm;
-        for (int it = 0; it < max_iter && !done;) {
-            for (int b = 0; b < 6; ++b, ++it) {
-                launch_walk_iter(dehnen, (unsigned)wb, s, cv, mp, ctx->pows.p, ctx->fmin.p, w, cur);
-                LCOUNT(1);
-                CK(cudaMemsetAsync(ctx->wcounts.p + cur, 0, sizeof(int), s), "memset");
-                cur ^= 1;
-            }
-            CKL("walk");
-            CK(cudaMemcpyAsync(hc, ctx->wcounts.p, sizeof(hc), cudaMemcpyDeviceToHost, s), "copy");
-            CK(cudaStreamSynchronize(s), "walk");
-            if (hc[WC_OVERFLOW] || hc[cur] == 0) done = true;
+        CK(ctx->pool_entry.ensure(32 * (size_t)ctx->cap_pool), "alloc walk");
+        CK(ctx->pool_next.ensure(ctx->cap_pool), "alloc walk");
+        CK(ctx->pool_owner.ensure(ctx->cap_pool), "alloc walk");
+        CK(cudaMemsetAsync(ctx->pool_owner.p, 0xff, (size_t)ctx->cap_pool * sizeof(uint2), s), "memset");
+        pool = WalkPool{ctx->pool_entry.p, ctx->pool_next.p, ctx->pool_owner.p, ctx->cap_pool,
+                        reinterpret_cast<unsigned*>(ctx->walk_state.p + WS_USED),
+                        reinterpret_cast<int*>(ctx->walk_state.p + WS_OVERFLOW)};
+        CK(cudaMemsetAsync(ctx->walk_state.p, 0, WS_SIZE * sizeof(unsigned long long), s), "memset");
+        CK(cudaMemsetAsync(ctx->list_sizes.p + nc, 0, sizeof(uint4), s), "memset");
+        for (int L = 0; L < ctx->nlevels; ++L) {
+            unsigned long long* ws = ctx->walk_state.p + L;
+            heavy.count = reinterpret_cast<int*>(ws + WS_HEAVY);
+            LCOUNT(launch_walk_level(dehnen, s, ctx->level_cells.p + ctx->lvl_start[L], ctx->lvl_count[L], ctx->nleaves,
+                                     cv, ctx->c_parent.p, mp, ctx->mac_rows.p, pool, lists, heavy,
+                                     reinterpret_cast<int*>(ws + WS_WORK), reinterpret_cast<int*>(ws + WS_HWORK)));
         }
-        if (!done) return fail(ctx, FMMX_TIMEOUT, "dual walk did not terminate");
-        if (hc[WC_OVERFLOW]) {
-            if (attempt > 24) return fail(ctx, FMMX_OUT_OF_MEMORY, "walk capacity");
-            ctx->walk_retries++;
-            auto grow = [](uint32_t c, int used) {
-                uint64_t w2 = std::max<uint64_t>(4ull * c, (uint64_t)used + (uint64_t)used / 2 + 1024);
-                return (uint32_t)std::min<uint64_t>(w2, 0x7fffffffull);
-            };
-            if (hc[WC_OVERFLOW] & 1) ctx->cap_front = grow(ctx->cap_front, 0);
-            if (hc[WC_OVERFLOW] & 2) ctx->cap_p2p = grow(ctx->cap_p2p, hc[WC_P2P]);
-            if (hc[WC_OVERFLOW] & 4) ctx->cap_m2l = grow(ctx->cap_m2l, hc[WC_M2L]);
-            continue;
-        }
-        ctx->n_m2l = hc[WC_M2L];
-        ctx->n_p2p = hc[WC_P2P];
-        CK(cudaMemcpy(&ctx->pops, ctx->wpops.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost), "copy");
-        return FMMX_OK;
-    }
-}
-
-// The directed lists of one kind (M2L or P2P) from the walk's mutual pairs:
-// a counting sort on the destination, segment sorts, and -- after a host
-// read-back of the number of long segments -- CUB's segmented sort of those.
-// The two kinds run on different streams with their own scratch (tmp, cnt,
-// bounds). list_launch queues a list's kernels without waiting on the device;
-// list_finish reads back its long-segment count (waiting for that stream) and
-// sorts the long segments. Both lists are launched before either is finished,
-// so their builds -- bound by atomics and latency, not by the SMs' arithmetic
-// -- run side by side.
-fmmx_status list_launch(fmmx_ctx* ctx, bool near, cudaStream_t s, DBuf<char>& tmp, DBuf<uint32_t>& cnt) {
-    const int nc = ctx->nc;
-    const int npairs = near ? ctx->n_p2p : ctx->n_m2l;
-    const size_t ndir = near ? (npairs > 0 ? 2 * (size_t)npairs - (size_t)ctx->nleaves : 0)  // one entry per self pair
-                             : 2 * (size_t)npairs;
-    if (ndir > 0x7fffffffull) return fail(ctx, FMMX_OUT_OF_MEMORY, "interaction lists above 2^31 entries");
-    DBuf<uint32_t>& off = near ? ctx->p2p_off : ctx->m2l_off;
-    DBuf<uint32_t>& src_u = near ? ctx->p2p_src_u : ctx->m2l_src_u;
-    DBuf<uint32_t>& src = near ? ctx->p2p_src : ctx->m2l_src;
-    DBuf<int>& longs = near ? ctx->p2p_longs : ctx->m2l_longs;
-    CK(off.ensure(nc + 1), "alloc lists");
-    CK(cnt.ensure(nc + 1), "alloc lists");
-    // (P2P: room for 2 entries per pair -- the scatter writes inside the
-    // counted segments whatever the number of self pairs)
-    const size_t room = near ? 2 * (size_t)npairs : ndir;
-    CK(src_u.ensure(std::max<size_t>(room, 1)), "alloc lists");
-    CK(src.ensure(std::max<size_t>(room, 1)), "alloc lists");
-    CK(longs.ensure(2 * (size_t)nc + 128), "alloc lists");
-    if (near) {
-        CK(ctx->inter.ensure(1), "alloc");
-        CK(cudaMemsetAsync(ctx->inter.p, 0, sizeof(unsigned long long), s), "memset");
-    }
-    CK(tmp.ensure(directed_list_temp((int)ndir, nc)), "alloc sort");
-    LCOUNT(6);  // count, scan (2), scatter, segment sorts (2)
-    CK(build_directed_list(tmp.p, tmp.cap, near ? ctx->p2p.p : ctx->m2l.p, npairs, (int)ndir, nc,
-                           near ? ctx->c_count.p : nullptr, near ? ctx->inter.p : nullptr, cnt.p, off.p, src_u.p,
-                           src.p, longs.p, grid_for(npairs, 256), s),
-       near ? "p2p lists" : "m2l lists");
-    if (near) {
-        // near-field work units and the scratch for the partial sums of leaves with several shares
-        for (DBuf<uint32_t>* b : {&ctx->p2p_units, &ctx->p2p_scr, &ctx->p2p_uoff, &ctx->p2p_soff})
-            CK(b->ensure(nc + 1), "alloc lists");
-        CK(ctx->p2p_next.ensure(1), "alloc lists");
-        const DirList lp{nullptr, ctx->p2p_src.p, ctx->p2p_off.p, ctx->p2p_off.p + 1, 32};
-        launch_p2p_plan(grid_for(nc + 1, 256), s, nc, lp, ctx->c_count.p, ctx->p2p_units.p, ctx->p2p_scr.p);
-        CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_units.p, ctx->p2p_uoff.p, nc + 1, s), "p2p units");
-        CK(scan_u32(tmp.p, tmp.cap, ctx->p2p_scr.p, ctx->p2p_soff.p, nc + 1, s), "p2p units");
-        LCOUNT(5);
-    }
-    return FMMX_OK;
-}
-
-fmmx_status list_finish(fmmx_ctx* ctx, bool near, cudaStream_t s, DBuf<char>& tmp, DBuf<uint32_t>& bounds) {
-    const int nc = ctx->nc;
-    const int npairs = near ? ctx->n_p2p : ctx->n_m2l;
-    const size_t ndir = near ? (npairs > 0 ? 2 * (size_t)npairs - (size_t)ctx->nleaves : 0) : 2 * (size_t)npairs;
-    DBuf<uint32_t>& off = near ? ctx->p2p_off : ctx->m2l_off;
-    DBuf<uint32_t>& src_u = near ? ctx->p2p_src_u : ctx->m2l_src_u;
-    DBuf<uint32_t>& src = near ? ctx->p2p_src : ctx->m2l_src;
-    DBuf<int>& longs = near ? ctx->p2p_longs : ctx->m2l_longs;
-    // host read-back: the number of long segments (and the P2P scratch size)
-    int nlong = 0;
-    uint32_t nscr = 0, nunits = 0;
-    CK(cudaMemcpyAsync(&nlong, longs.p, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
-    if (near) {
-        CK(cudaMemcpyAsync(&nscr, ctx->p2p_soff.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "copy");
-        CK(cudaMemcpyAsync(&nunits, ctx->p2p_uoff.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "copy");
-    }
-    CK(cudaStreamSynchronize(s), "lists");
-    if (near) {
-        CK(ctx->p2p_part.ensure(std::max<size_t>(nscr, 1)), "alloc p2p scratch");
-        CK(ctx->p2p_ucell.ensure(std::max<size_t>(nunits, 1)), "alloc p2p scratch");
-        ctx->p2p_nunits = nunits;
-        launch_p2p_unit_cells(s, nc, ctx->p2p_uoff.p, ctx->p2p_ucell.p);
-        CKL("p2p units");
-        LCOUNT(1);
-    }
-    if (nlong > 0) {
-        const int end_bit = bits_for((uint64_t)nc);
-        CK(bounds.ensure(2 * (size_t)nlong), "alloc lists");
-        CK(tmp.ensure(long_segments_temp((int)ndir, nlong, end_bit)), "alloc sort");
+        CKL("walk");
+        CK(scan_u32x4(ctx->cub_tmp.p, ctx->cub_tmp.cap, ctx->list_sizes.p, ctx->list_off.p, nc + 1, s), "list offsets");
         LCOUNT(2);
-        CK(sort_long_segments(tmp.p, tmp.cap, off.p, longs.p, nlong, src_u.p, src.p, (int)ndir, end_bit, bounds.p,
-                              s),
-           near ? "p2p lists" : "m2l lists");
+        int stack_overflow = 0;
+        CK(cudaMemcpyAsync(hs, ctx->walk_state.p, sizeof(hs), cudaMemcpyDeviceToHost, s), "copy");
+        CK(cudaMemcpyAsync(&sizes, ctx->list_off.p + nc, sizeof(sizes), cudaMemcpyDeviceToHost, s), "copy");
+        if (dehnen)
+            CK(cudaMemcpyAsync(&stack_overflow, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
+        CK(cudaStreamSynchronize(s), "walk");
+        if (stack_overflow) return fail(ctx, FMMX_DEVICE_ERROR, "f pre-pass stack overflow");
+        if (!hs[WS_OVERFLOW]) break;
+        if (attempt > 24 || ctx->cap_pool >= most) return fail(ctx, FMMX_OUT_OF_MEMORY, "walk capacity");
+        ctx->walk_retries++;
+        const uint64_t used = (uint32_t)hs[WS_USED];
+        ctx->cap_pool = (uint32_t)std::min(std::max<uint64_t>(2ull * ctx->cap_pool, used + used / 4 + 64), most);
     }
+    const uint64_t dm = hs[WS_TOTALS + 2], dp = hs[WS_TOTALS + 3];
+    if (dm > 0x7fffffffull || dp > 0x7fffffffull)
+        return fail(ctx, FMMX_OUT_OF_MEMORY, "interaction lists above 2^31 entries");
+    ctx->pops = hs[WS_TOTALS];
+    ctx->p2p_inter = hs[WS_TOTALS + 1];
+    ctx->n_m2l = (int)(dm / 2);
+    ctx->n_p2p = (int)((dp + (uint64_t)ctx->nleaves) / 2);  // a leaf's self pair is one entry
+    ctx->p2p_nunits = sizes.z;
+    CK(ctx->m2l_src.ensure(std::max<size_t>(dm, 1)), "alloc lists");
+    CK(ctx->p2p_src.ensure(std::max<size_t>(dp, 1)), "alloc lists");
+    CK(ctx->p2p_ucell.ensure(std::max<size_t>(sizes.z, 1)), "alloc lists");
+    CK(ctx->p2p_part.ensure(std::max<size_t>(sizes.w, 1)), "alloc p2p scratch");
+    CK(ctx->p2p_next.ensure(1), "alloc lists");
+    if (ctx->events) CK(cudaEventRecord(ctx->ev[4], s), "event");
+    launch_lists_gather(s, nc, (uint32_t)hs[WS_USED], pool, lists, ctx->list_off.p, ctx->m2l_off.p, ctx->p2p_off.p, ctx->p2p_uoff.p,
+                        ctx->p2p_soff.p, ctx->m2l_src.p, ctx->p2p_src.p, ctx->p2p_ucell.p);
+    CKL("lists");
+    LCOUNT(1);
     return FMMX_OK;
 }
 
-// the near field's work units, as list_launch and list_finish left them
+// the near field's work units, as walk_impl left them
 P2pUnits near_units(fmmx_ctx* ctx) {
     return P2pUnits{ctx->p2p_uoff.p, ctx->p2p_ucell.p, ctx->p2p_soff.p, ctx->p2p_part.p, ctx->p2p_next.p,
                     ctx->p2p_nunits};
@@ -920,31 +846,15 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         ctx->lists_valid = false;
         fmmx_status st = walk_impl(ctx, s2);
         if (st != FMMX_OK) return st;
-        if (dehnen) {
-            int bad = 0;
-            CK(cudaMemcpy(&bad, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost), "copy");
-            if (bad) return fail(ctx, FMMX_DEVICE_ERROR, "f pre-pass stack overflow");
-        }
+        ctx->lists_valid = true;
+    } else if (tm) {
+        CK(cudaEventRecord(ev[4], s2), "event");
     }
-    if (tm) CK(cudaEventRecord(ev[4], s2), "event");
-    if (!reuse) {
-        CK(cudaEventRecord(ctx->fork[1], s2), "event");  // the walk's pairs are in place
-        fmmx_status st = list_launch(ctx, true, s2, ctx->cub_tmp, ctx->list_cnt);
-        if (st != FMMX_OK) return st;
-        CK(cudaStreamWaitEvent(s, ctx->fork[1], 0), "join");  // the M2L list reads the walk's pairs
-        if (tm) CK(cudaEventRecord(ev[14], s), "event");
-        st = list_launch(ctx, false, s, ctx->cub_tmp2, ctx->list_cnt2);
-        if (st != FMMX_OK) return st;
-        st = list_finish(ctx, true, s2, ctx->cub_tmp, ctx->long_bounds);
-        if (st != FMMX_OK) return st;
-    }
+    if (!reuse) CK(cudaEventRecord(ctx->fork[1], s2), "event");  // the lists are in place
     if (tm) CK(cudaEventRecord(ev[5], s2), "event");
 
-    // (each list's pointers are taken after its build, which may reallocate it)
+    // (the lists' pointers are taken after the walk, which may reallocate them)
     const DirList lp{nullptr, ctx->p2p_src.p, ctx->p2p_off.p, ctx->p2p_off.p + 1, 32};
-    // The near field starts on the second stream as soon as its list is
-    // built; the far field's list, launched beside it, is finished on the
-    // first stream after the near field is queued.
     if (mixed) {
         fmmx_status ms = near_mixed(ctx, lp, tm);
         if (ms != FMMX_OK) return ms;
@@ -958,12 +868,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         if (tm) CK(cudaEventRecord(ev[8], s2), "event");
         CK(cudaEventRecord(ctx->fork[2], s2), "event");
     }
-    if (!reuse) {
-        fmmx_status st = list_finish(ctx, false, s, ctx->cub_tmp2, ctx->long_bounds2);
-        if (st != FMMX_OK) return st;
-        if (tm) CK(cudaEventRecord(ev[15], s), "event");
-        ctx->lists_valid = true;
-    }
+    if (!reuse) CK(cudaStreamWaitEvent(s, ctx->fork[1], 0), "join");  // the M2L reads its list
     const DirList lm{nullptr, ctx->m2l_src.p, ctx->m2l_off.p, ctx->m2l_off.p + 1, 32};
     if (mixed) {
         fmmx_status ms = far_mixed(ctx, lm, d_acc, d_pot, tm);
@@ -1015,7 +920,6 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     if (tm) CK(cudaEventRecord(ev[9], s), "event");
     if (capture) return FMMX_OK;
     CK(cudaStreamSynchronize(s), "evaluate");
-    CK(cudaMemcpy(&ctx->p2p_inter, ctx->inter.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost), "copy");
     if (tm) {
         auto el = [&](int a, int b) {
             float ms = 0;
@@ -1025,7 +929,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         // stages on the two streams overlap: each is timed on its own stream
         ctx->st.ms_upward = el(2, 3);
         ctx->st.ms_walk = el(10, 4);
-        ctx->st.ms_lists = el(4, 5) + (reuse ? 0.0 : el(14, 15));
+        ctx->st.ms_lists = el(4, 5);
         ctx->st.ms_m2l = el(11, 6);
         ctx->st.ms_l2l = el(6, 7);
         ctx->st.ms_p2p = el(12, 8);
@@ -1144,6 +1048,7 @@ fmmx_status fmmx_create(const fmmx_config* cfg, fmmx_ctx** out) {
     g_nsm = ctx->nsm;
     make_tables(ctx->tab);
     upload_tables_exact(ctx->tab, ctx->stream);
+    upload_tables_walk(ctx->tab, ctx->stream);
     upload_tables_m2l(ctx->tab, ctx->stream);
     upload_tables_sweeps(ctx->tab, ctx->stream);
     upload_tables_mixed(ctx->tab, ctx->stream);
@@ -1497,9 +1402,25 @@ fmmx_status fmmx_export_lists(const fmmx_ctx* cctx, uint32_t* m2l, uint32_t* p2p
     if (!ctx->evaluated) return fail(ctx, FMMX_NOT_BUILT, "export before evaluate");
     cudaSetDevice(ctx->cfg.device);
     CK(cudaStreamSynchronize(ctx->stream), "sync");
-    if (m2l && ctx->n_m2l) CK(cudaMemcpy(m2l, ctx->m2l.p, (size_t)ctx->n_m2l * 8, cudaMemcpyDeviceToHost), "copy");
-    if (p2p && ctx->n_p2p) CK(cudaMemcpy(p2p, ctx->p2p.p, (size_t)ctx->n_p2p * 8, cudaMemcpyDeviceToHost), "copy");
-    return FMMX_OK;
+    // the mutual pairs (a, b), a before b in depth-first order, from the directed lists
+    auto pairs = [&](const DBuf<uint32_t>& off, const DBuf<uint32_t>& src, uint32_t* out) -> fmmx_status {
+        std::vector<uint32_t> o(ctx->nc + 1);
+        CK(cudaMemcpy(o.data(), off.p, o.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost), "copy");
+        std::vector<uint32_t> v(o.back());
+        if (!v.empty()) CK(cudaMemcpy(v.data(), src.p, v.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost), "copy");
+        for (uint32_t c = 0; c < (uint32_t)ctx->nc; ++c)
+            for (uint32_t i = o[c]; i < o[c + 1]; ++i)
+                if (v[i] >= c) {
+                    *out++ = c;
+                    *out++ = v[i];
+                }
+        return FMMX_OK;
+    };
+    if (m2l) {
+        const fmmx_status st = pairs(ctx->m2l_off, ctx->m2l_src, m2l);
+        if (st != FMMX_OK) return st;
+    }
+    return p2p ? pairs(ctx->p2p_off, ctx->p2p_src, p2p) : FMMX_OK;
 }
 
 fmmx_status fmmx_export_expansions(const fmmx_ctx* cctx, double* moments, double* locals, double* pows, double* f,

@@ -33,19 +33,30 @@ struct MacParams {
     double gap;  // minimum separation of the bodies of an M2L pair (soft_gap * softening); 0: none
 };
 
-enum { WC_FRONT0 = 0, WC_FRONT1 = 1, WC_M2L = 2, WC_P2P = 3, WC_OVERFLOW = 4, WC_SIZE = 8 };
+// Pool of list chunks of the walk: 32 entries each, each of one list.
+struct WalkPool {
+    uint32_t* entry;  // 32 cap
+    uint32_t* next;   // cap: the following chunk of a list passed down
+    uint2* owner;     // cap: whose entries the chunk of an M2L or P2P list holds (all bits set: nobody's)
+    uint32_t cap;     // chunks
+    unsigned* used;   // chunks reserved (beyond cap after an overflow)
+    int* overflow;    // set when a chunk was refused: the lists are incomplete
+};
 
-struct WalkBufs {
-    uint2* front[2];
-    uint2* m2l;
-    uint2* p2p;
-    int* counts;           // WC_* slots
-    unsigned long long* pops_ptr;
-    uint32_t cap_front, cap_m2l, cap_p2p;
+// Per-cell results of the walk: the list passed down to the children (entries
+// and first chunk), whether the cell was walked a second time (as a heavy one),
+// and the lists' sizes with the near field's work units and partial sums (m2l,
+// p2p, units, scratch).
+struct WalkLists {
+    uint32_t* down_n;
+    uint32_t* down_head;
+    uint8_t* redone;
+    uint4* sizes;                // ncells + 1
+    unsigned long long* totals;  // pairs examined, body interactions, directed M2L and P2P entries
 };
 
 // Segmented directed interaction list: for destination cell c, sources
-// src(key(i)) for i in [seg_begin[c], seg_end[c]), in ascending order.
+// src(key(i)) for i in [seg_begin[c], seg_end[c]), in the walk's order.
 struct DirList {
     const uint64_t* keys;    // entries (dst << shift) | src, or null
     const uint32_t* keys32;  // 32-bit entries (then keys is null); with shift = 32 the entries are the sources
@@ -72,7 +83,6 @@ __global__ void k_keys_seg(const double* pos, size_t n, const uint64_t* off, int
 __global__ void k_pack_by_system(const uint64_t* keys, const uint32_t* order, size_t n, const uint64_t* off, int nsys,
                                  uint32_t* sys, ulonglong2* val);
 __global__ void k_unpack_by_system(const ulonglong2* val, size_t n, uint64_t* keys, uint32_t* order);
-__global__ void k_walk_init(const int32_t* level_cells, int nroots, uint2* front);
 #define TREE_BLOCK 256
 #define TREE_PER_THREAD 4  // slots per thread of the two tree kernels
 __global__ void k_cell_count(const uint64_t* keys, uint32_t n, const uint64_t* off, int nsys, uint32_t n_leaf,
@@ -97,33 +107,40 @@ __global__ void k_m2m_exact_block(const int32_t* level_cells, int lstart, int lc
 void launch_fprepass(cudaStream_t s, CellsView cells, const double* x, const double* y, const double* z,
                      const double* m, size_t n, const uint64_t* off, int nsys, const int32_t* roots, double* f,
                      int* err);
-// one dual-walk iteration over frontier `cur` (k_walk_iter<DEHNEN>: Dehnen's error-estimate MAC, else
-// theta and soft_gap), 256-thread blocks; and its resident blocks per SM
-void launch_walk_iter(bool dehnen, unsigned grid, cudaStream_t s, CellsView cv, MacParams mp, const double* pows,
-                      const double* fmin, WalkBufs w, int cur);
-int walk_iter_blocks_per_sm(bool dehnen);
-__global__ void k_pack_geo(int nc, const double* cx, const double* cy, const double* cz, const double* rho,
-                           double4* geo);
+__global__ void k_pack_geo(int nc, CellsMut cells, double4* geo);
+
+// Cells whose walk is left to many warps: their ids, and a queue of ring_cap
+// sources for each of `blocks` blocks.
+struct WalkHeavy {
+    int32_t* list;
+    int* count;  // of the level, zero at its start
+    uint32_t* ring;
+    uint32_t ring_cap;
+    unsigned blocks;
+};
+
+// walk.cu
+void upload_tables_walk(const OrderTables& t, cudaStream_t s);
+// rows of p + 2 per cell for Dehnen's MAC
+__global__ void k_mac_rows(int nc, CellsView cv, int p, const double* pows, const double* fminv, double2* rows);
+// The cells of one level (Dehnen's error-estimate MAC, else theta and soft_gap); work, heavy_work: zero
+// counters. Returns the launches.
+int launch_walk_level(bool dehnen, cudaStream_t s, const int32_t* level_cells, int lcnt, int nleaves, CellsView cv,
+                      const int32_t* parent, MacParams mp, const double2* rows, WalkPool P, WalkLists Ls, WalkHeavy heavy,
+                      int* work, int* heavy_work);
+bool walk_needs_heavy(const int* lvl_count, int nlevels, int nleaves);
+unsigned walk_heavy_blocks(int nleaves);
+// contiguous lists from the chunks; off: the exclusive sums of W.sizes
+void launch_lists_gather(cudaStream_t s, int nc, uint32_t nchunks, WalkPool P, WalkLists W, const uint4* off, uint32_t* m2l_off,
+                         uint32_t* p2p_off, uint32_t* uoff, uint32_t* soff, uint32_t* m2l, uint32_t* p2p,
+                         int32_t* ucell);
 
 // lists.cu
-// Directed list of `np` walk pairs with `nitems` directed entries: per
-// destination c its sources src[off[c] .. off[c+1]) in ascending order
-// (off has ncells + 1 entries; cnt is ncells + 1 scratch counters). With
-// body_count, also adds the directed body-body interactions (P2P). Segments
-// longer than 4096 entries are left for sort_long_segments: `longs`
-// (2 ncells + 128 ints) receives their count at [0] and ids from [128].
-size_t directed_list_temp(int nitems, int ncells);
-cudaError_t build_directed_list(void* tmp, size_t tmp_bytes, const uint2* pairs, int np, int nitems, int ncells,
-                                const uint32_t* body_count, unsigned long long* interactions, uint32_t* cnt,
-                                uint32_t* off, uint32_t* src_unsorted, uint32_t* src, int* longs, unsigned grid,
-                                cudaStream_t s);
-size_t long_segments_temp(int nitems, int nlong, int end_bit);
-// the nlong long segments (count read back from longs[0]); bounds: 2 nlong scratch
-cudaError_t sort_long_segments(void* tmp, size_t tmp_bytes, const uint32_t* off, const int* longs, int nlong,
-                               const uint32_t* src_unsorted, uint32_t* src, int nitems, int end_bit, uint32_t* bounds,
-                               cudaStream_t s);
-// exclusive prefix sum of n values (temp storage as for directed_list_temp)
+// exclusive prefix sums of n values, and of four at once
+size_t scan_u32_temp(int n);
 cudaError_t scan_u32(void* tmp, size_t tmp_bytes, const uint32_t* in, uint32_t* out, int n, cudaStream_t s);
+size_t scan_u32x4_temp(int n);
+cudaError_t scan_u32x4(void* tmp, size_t tmp_bytes, const uint4* in, uint4* out, int n, cudaStream_t s);
 
 // m2l.cu
 void upload_tables_m2l(const OrderTables& t, cudaStream_t s);
@@ -174,9 +191,6 @@ __host__ __device__ __forceinline__ uint32_t p2p_shares(uint32_t nt, uint32_t le
     return s < most ? s : most;
 }
 
-void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
-                     uint32_t* scratch);
-void launch_p2p_unit_cells(cudaStream_t s, int ncells, const uint32_t* uoff, int32_t* ucell);
 void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,
                         double* az, double* pot);
 void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const double* x,

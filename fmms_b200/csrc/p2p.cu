@@ -13,28 +13,6 @@
 
 namespace fmmx {
 
-// Units, shares and leaves of units: see P2pUnits and p2p_shares.
-__global__ void k_p2p_plan(int ncells, DirList L, const uint32_t* __restrict__ count, uint32_t* __restrict__ units,
-                           uint32_t* __restrict__ scratch) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x) {
-        uint32_t nu = 0, sc = 0;
-        if (c < ncells) {
-            const uint32_t len = L.seg_end[c] - L.seg_begin[c], nt = count[c];
-            const uint32_t s = p2p_shares(nt, len);
-            nu = s * ((nt + P2P_NT - 1) / P2P_NT);
-            sc = s > 1 ? s * nt : 0;
-        }
-        units[c] = nu;
-        scratch[c] = sc;
-    }
-}
-
-// the leaf of every unit
-__global__ void k_p2p_unit_cells(int ncells, const uint32_t* __restrict__ uoff, int32_t* __restrict__ ucell) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x)
-        for (uint32_t u = uoff[c]; u < uoff[c + 1]; ++u) ucell[u] = c;
-}
-
 // The bodies of the leaves with several shares: the shares' partial sums, in
 // share order (one warp per leaf).
 __global__ void k_p2p_combine(int ncells, DirList L, CellsView cv, P2pUnits U, double* __restrict__ ax,
@@ -61,15 +39,6 @@ __global__ void k_p2p_combine(int ncells, DirList L, CellsView cv, P2pUnits U, d
             pot[tf + i] = s.w;
         }
     }
-}
-
-void launch_p2p_plan(unsigned grid, cudaStream_t s, int ncells, DirList L, const uint32_t* count, uint32_t* units,
-                     uint32_t* scratch) {
-    k_p2p_plan<<<grid, 256, 0, s>>>(ncells, L, count, units, scratch);
-}
-
-void launch_p2p_unit_cells(cudaStream_t s, int ncells, const uint32_t* uoff, int32_t* ucell) {
-    k_p2p_unit_cells<<<grid_for(ncells, 128), 128, 0, s>>>(ncells, uoff, ucell);
 }
 
 void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,

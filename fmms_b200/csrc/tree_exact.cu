@@ -1,6 +1,6 @@
 // Bit-exact stages of the engine: bounding box, Morton keys, octree topology,
-// cell geometry, P2M/M2M, multipole power, the f pre-pass and the dual tree
-// walk with its MAC.
+// cell geometry, P2M/M2M, multipole power and the f pre-pass (the walk with its
+// MAC is in walk.cu).
 //
 // Everything here feeds the multipole acceptance decisions, so it reproduces
 // the reference's FP64 operation order exactly and this file is compiled with
@@ -237,14 +237,6 @@ __global__ void k_unpack_by_system(const ulonglong2* __restrict__ val, size_t n,
         const ulonglong2 v = val[i];
         keys[i] = v.x;
         order[i] = (uint32_t)v.y;
-    }
-}
-
-// Walk seeds: the self pair of every root.
-__global__ void k_walk_init(const int32_t* __restrict__ level_cells, int nroots, uint2* __restrict__ front) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nroots; j += gridDim.x * blockDim.x) {
-        const int r = level_cells[j];
-        front[j] = make_uint2(r, r);
     }
 }
 
@@ -671,7 +663,7 @@ __global__ void __launch_bounds__(32 * GEO_WARPS) k_geometry_com(int nc, CellsMu
                 cells.cy[c] = cy;
                 cells.cz[c] = cz;
                 cells.rho[c] = rho;
-                geo[c] = make_double4(cx, cy, cz, rho);
+                geo[c] = make_double4(cx, cy, cz, -rho);  // the sign marks a leaf
             }
         }
         for (int par = cells.parent[c]; par >= 0; par = cells.parent[c]) {
@@ -1040,8 +1032,7 @@ __global__ void __launch_bounds__(32 * FPRE_WARPS) k_fprepass(CellsView cells, c
     const size_t stride = (size_t)gridDim.x * FPRE_WARPS * 32;
     // stack entry e of cell c for the given lanes
     auto put = [&](int e, int c, unsigned lanes) {
-        double4 g = cells.geo[c];
-        if (cells.leaf[c]) g.w = -g.w;
+        const double4 g = cells.geo[c];
         S.geo[e] = g;
         S.mass[e] = signbit(g.w) ? __hiloint2double((int)cells.count[c], (int)cells.first[c]) : cells.mass[c];
         S.cell[e] = c;
@@ -1124,241 +1115,11 @@ void launch_fprepass(cudaStream_t s, CellsView cells, const double* x, const dou
                                                                                  roots, f, err);
 }
 
-// cx, cy, cz, rho of every cell in one 32-byte record, for the walk
-__global__ void k_pack_geo(int nc, const double* __restrict__ cx, const double* __restrict__ cy,
-                           const double* __restrict__ cz, const double* __restrict__ rho, double4* __restrict__ geo) {
+// (centre, rho) of every cell in one 32-byte record for the walk and the near
+// field, the sign of rho set for a leaf
+__global__ void k_pack_geo(int nc, CellsMut cells, double4* __restrict__ geo) {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
-        geo[c] = make_double4(cx[c], cy[c], cz[c], rho[c]);
-}
-
-// ------------------------------------------------------------ MAC
-// error_estimate + accept, mac.rs:23-95 (operation order kept, including the
-// inner r*r of error_estimate).
-__device__ __forceinline__ bool accept_dehnen(const CellsView& cv, const MacParams& mp, const double* __restrict__ pows,
-                                              const double* __restrict__ fminv, int a, int b, const double4 ga,
-                                              const double4 gb) {
-    const double ax = ga.x, ay = ga.y, az = ga.z;
-    const double dx = gb.x - ax, dy = gb.y - ay, dz = gb.z - az;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double ra = ga.w, rb = gb.w;
-    const double sum_rho = ra + rb;
-    if (r2 <= sum_rho * sum_rho) return false;
-    const double r = sqrt(r2);
-    if (r == 0.0) return false;
-    const int p = mp.p;
-    const double rr2 = r * r;
-    double rp = 1.0;
-    for (int i = 0; i < p / 2; ++i) rp *= rr2;
-    if (p % 2 == 1) rp *= r;
-    double rpows[FMMX_MAXP + 1];
-    rpows[0] = 1.0;
-    for (int j = 1; j <= p; ++j) rpows[j] = rpows[j - 1] * rb;
-    const double* pw = pows + (size_t)a * (p + 1);
-    double s = 0.0;
-    for (int k = 0; k <= p; ++k) s += g_tab.binom[p][k] * pw[k] * rpows[p - k];
-    const double ma = cv.mass[a];
-    const double e = s / (ma * rp);
-    const double denom = ra + rb;
-    double est;
-    if (denom == 0.0) est = 0.0;
-    else est = 8.0 * fmax(ra, rb) / denom * e;
-    if (est == 0.0) return true;
-    return est * ma / r2 < mp.eps * fminv[b];
-}
-
-// Separation condition (extension, with softening): the bodies of the two
-// cells are at least mp.gap apart, r - rho_A - rho_B >= gap.
-__device__ __forceinline__ bool gap_ok(const MacParams& mp, const double4 ga, const double4 gb) {
-    if (!(mp.gap > 0.0)) return true;
-    const double dx = gb.x - ga.x, dy = gb.y - ga.y, dz = gb.z - ga.z;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    return sqrt(r2) - (ga.w + gb.w) >= mp.gap;
-}
-
-// The geometric MAC (extension): accept when (rho_A + rho_B) < theta r, both
-// ways round as the reference's walk applies its MAC (walk.rs:138-139), and
-// gap_ok. The
-// two directions and gap_ok evaluate the same r2 (the squares of b - a and
-// a - b are equal bit for bit) and the same rho sum (addition commutes), so
-// one square root decides all three.
-__device__ __forceinline__ bool accept_theta_pair(const MacParams& mp, const double4 ga, const double4 gb) {
-    const double dx = gb.x - ga.x, dy = gb.y - ga.y, dz = gb.z - ga.z;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double sum_rho = ga.w + gb.w;
-    const double r = sqrt(r2);
-    if (!(sum_rho < mp.theta * r)) return false;
-    return !(mp.gap > 0.0) || r - sum_rho >= mp.gap;
-}
-
-// ------------------------------------------------------------ dual walk
-// process_pair, walk.rs:94-190, applied to a whole frontier of cell pairs at
-// once. Every decision depends only on the pair, so the emitted M2L and P2P
-// pair sets equal those of the reference's depth-first stack walk. Appends are
-// warp-aggregated: one atomic per warp and list (a ballot for the M2L and P2P
-// lists, a prefix sum of the child-pair counts for the next frontier); the
-// order within a list is arbitrary, the directed lists are sorted afterwards.
-enum { WK_NONE = 0, WK_M2L = 1, WK_P2P = 2, WK_SPLIT_SELF = 3, WK_SPLIT = 4 };
-
-// children of a cell: 8 ids (-1 absent), 32-byte aligned, read as two int4
-__device__ __forceinline__ void load_children(const CellsView& cv, int c, int (&ch)[8]) {
-    const int4* p = reinterpret_cast<const int4*>(cv.child + 8 * (size_t)c);
-    const int4 u = p[0], v = p[1];
-    ch[0] = u.x; ch[1] = u.y; ch[2] = u.z; ch[3] = u.w;
-    ch[4] = v.x; ch[5] = v.y; ch[6] = v.z; ch[7] = v.w;
-}
-__device__ __forceinline__ int n_children(const CellsView& cv, int c) {
-    int ch[8];
-    load_children(cv, c, ch);
-    int n = 0;
-#pragma unroll
-    for (int o = 0; o < 8; ++o) n += ch[o] >= 0;
-    return n;
-}
-
-__device__ __forceinline__ int warp_append(int* counter, bool mine, int lane) {
-    const unsigned mask = __ballot_sync(0xffffffffu, mine);
-    if (!mask) return -1;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return mine ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
-}
-
-// Latency: a walk iteration is a chain of dependent L2 round trips (the
-// frontier entry, then the cells, then the appends), so every read a pair can
-// need -- both cells' leaf flags, geometry and children -- is issued at once
-// after the entry, and the three appends (M2L, P2P, next frontier) are one
-// atomic instruction from three lanes.
-template <bool DEHNEN>
-__global__ void k_walk_iter(CellsView cv, MacParams mp, const double* __restrict__ pows,
-                            const double* __restrict__ fminv, WalkBufs w, int cur) {
-    // After an overflow the frontier holds unwritten entries: stop, the host
-    // retries with larger buffers.
-    if (w.counts[WC_OVERFLOW]) return;
-    const int nin = min(w.counts[cur], (int)w.cap_front);
-    const int nxt = cur ^ 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(w.pops_ptr, (unsigned long long)nin);
-    const uint2* __restrict__ fin = w.front[cur];
-    uint2* fout = w.front[nxt];
-    const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * blockDim.x;
-    // whole warps step through the frontier together (the ballots need every lane)
-    for (int q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); q0 < nin; q0 += stride) {
-        const int q = q0 + lane;
-        int kind = WK_NONE, a = 0, b = 0, npush = 0;
-        bool split_a = false;
-        int cha[8], chb[8];
-        if (q < nin) {
-            const uint2 pr = fin[q];
-            a = (int)pr.x;
-            b = (int)pr.y;
-            const bool la = cv.leaf[a], lb = cv.leaf[b];
-            const double4 ga = cv.geo[a], gb = cv.geo[b];
-            load_children(cv, a, cha);
-            load_children(cv, b, chb);
-            if (a == b) {
-                if (la) {
-                    kind = WK_P2P;
-                } else {
-                    kind = WK_SPLIT_SELF;
-                    int nch = 0;
-#pragma unroll
-                    for (int o = 0; o < 8; ++o) nch += cha[o] >= 0;
-                    npush = nch * (nch + 1) / 2;
-                }
-            } else {
-                bool acc;
-                if (DEHNEN)
-                    acc = accept_dehnen(cv, mp, pows, fminv, a, b, ga, gb) &&
-                          accept_dehnen(cv, mp, pows, fminv, b, a, gb, ga) && gap_ok(mp, ga, gb);
-                else
-                    acc = accept_theta_pair(mp, ga, gb);
-                if (acc) {
-                    kind = WK_M2L;
-                } else if (la && lb) {
-                    kind = WK_P2P;
-                } else {
-                    // split b when a is a leaf or b is the larger cell, else split a
-                    kind = WK_SPLIT;
-                    split_a = lb || (!la && ga.w >= gb.w);
-                    int nch = 0;
-                    // chb takes the children of the cell that splits (element by
-                    // element, so both arrays stay in registers)
-#pragma unroll
-                    for (int o = 0; o < 8; ++o) {
-                        chb[o] = split_a ? cha[o] : chb[o];
-                        nch += chb[o] >= 0;
-                    }
-                    npush = nch;
-                }
-            }
-        }
-        const unsigned mm = __ballot_sync(0xffffffffu, kind == WK_M2L);
-        const unsigned mq = __ballot_sync(0xffffffffu, kind == WK_P2P);
-        // next frontier: inclusive prefix sum of the pushes across the warp
-        int incl = npush;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        // lanes 0, 1, 2 reserve the warp's M2L, P2P and frontier entries
-        int got = 0;
-        {
-            const int v = lane == 0 ? __popc(mm) : lane == 1 ? __popc(mq) : lane == 2 ? total : 0;
-            int* ctr = w.counts + (lane == 0 ? WC_M2L : lane == 1 ? WC_P2P : nxt);
-            if (v > 0) got = atomicAdd(ctr, v);
-        }
-        const int bm = __shfl_sync(0xffffffffu, got, 0);
-        const int bp = __shfl_sync(0xffffffffu, got, 1);
-        const int bf = __shfl_sync(0xffffffffu, got, 2);
-        const unsigned below = (1u << lane) - 1u;
-        if (kind == WK_M2L) {
-            const int sm = bm + __popc(mm & below);
-            if ((uint32_t)sm < w.cap_m2l) w.m2l[sm] = make_uint2(a, b);
-            else atomicOr(&w.counts[WC_OVERFLOW], 4);
-        } else if (kind == WK_P2P) {
-            const int sp = bp + __popc(mq & below);
-            if ((uint32_t)sp < w.cap_p2p) w.p2p[sp] = make_uint2(a, b);
-            else atomicOr(&w.counts[WC_OVERFLOW], 2);
-        }
-        if (total == 0) continue;
-        if ((uint32_t)(bf + total) > w.cap_front) {
-            if (lane == 0) atomicOr(&w.counts[WC_OVERFLOW], 1);
-            continue;
-        }
-        int pos = bf + incl - npush;
-        if (kind == WK_SPLIT_SELF) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (cha[i] < 0) continue;
-#pragma unroll
-                for (int j = i; j < 8; ++j)
-                    if (cha[j] >= 0) fout[pos++] = make_uint2(cha[i], cha[j]);
-            }
-        } else if (kind == WK_SPLIT) {
-#pragma unroll
-            for (int o = 0; o < 8; ++o) {
-                const int c = chb[o];
-                if (c < 0) continue;
-                fout[pos++] = split_a ? make_uint2(c, b) : make_uint2(a, c);
-            }
-        }
-    }
-}
-
-void launch_walk_iter(bool dehnen, unsigned grid, cudaStream_t s, CellsView cv, MacParams mp, const double* pows,
-                      const double* fmin, WalkBufs w, int cur) {
-    if (dehnen) k_walk_iter<true><<<grid, 256, 0, s>>>(cv, mp, pows, fmin, w, cur);
-    else k_walk_iter<false><<<grid, 256, 0, s>>>(cv, mp, pows, fmin, w, cur);
-}
-
-int walk_iter_blocks_per_sm(bool dehnen) {
-    int per_sm = 0;
-    const cudaError_t e = dehnen ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_iter<true>, 256, 0)
-                                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_iter<false>, 256, 0);
-    return e == cudaSuccess && per_sm > 0 ? per_sm : 1;
+        geo[c] = make_double4(cells.cx[c], cells.cy[c], cells.cz[c], cells.leaf[c] ? -cells.rho[c] : cells.rho[c]);
 }
 
 }  // namespace fmmx
