@@ -149,6 +149,7 @@ struct fmmx_ctx {
     OrderTables tab;
     std::vector<double> swap_host;
     DBuf<double> swap_dev;
+    DBuf<uint32_t> l2l_sched;  // product list of the mixed L2L
 
     // sizes of the current tree; a forest of nsys independent systems
     size_t n = 0;
@@ -186,7 +187,7 @@ struct fmmx_ctx {
     DBuf<char> cub_tmp;
 
     DBuf<uint32_t> cell_id0;  // n + 1: cells that start before each slot
-    DBuf<unsigned> geo_arrive;  // children of a cell whose geometry is done
+    DBuf<unsigned> geo_arrive, up_arrive;  // children of a cell whose geometry (moments) are done
     DBuf<unsigned long long> bbox_enc;
     DBuf<uint32_t> sort_sys, sort_sys_alt;  // a forest's second sort (by system)
     DBuf<ulonglong2> sort_val, sort_val_alt;
@@ -710,7 +711,7 @@ fmmx_status far_mixed(fmmx_ctx* ctx, const DirList& lm, double* d_acc, double* d
         const int cnt = ctx->lvl_count[L];
         const unsigned g = std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm);
         launch_l2l_mixed(L <= 3, g, s, ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, ctx->c_parent.p, ctx->ell.p,
-                         p, ctx->loc_f.p);
+                         p, ctx->l2l_sched.p, ctx->loc_f.p);
     }
     CKL("l2l (mixed)");
     if (tm) CK(cudaEventRecord(ev[7], s), "event");
@@ -743,7 +744,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     if (d_mass == nullptr) d_mass = ctx->build_mass;
     k_gather<<<grid_for(n, 256), 256, 0, s>>>(d_pos, d_mass, ctx->order.p, n, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p);
     CKL("gather");
-    LCOUNT(1 + ctx->nlevels + (ctx->cfg.mac_mode == FMMX_MAC_DEHNEN ? 1 : 0));  // gather, upward levels, f pre-pass
+    LCOUNT(4 + (ctx->cfg.mac_mode == FMMX_MAC_DEHNEN ? 1 : 0));  // gather, upward (mixed; plain counts its own), f pre-pass
     CK(ctx->moments.ensure((size_t)nc * dim), "alloc expansions");
     CK(ctx->locals.ensure((size_t)nc * dim), "alloc expansions");
     CK(ctx->pows.ensure((size_t)nc * (p + 1)), "alloc expansions");
@@ -764,6 +765,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         // sized on every mixed evaluation, so that a reuse step recorded into
         // a CUDA graph never allocates while capturing
         CK(ctx->rho_now.ensure(nc), "alloc expansions");
+        CK(ctx->up_arrive.ensure(nc), "alloc expansions");
         if (reuse) {  // the bodies moved since the build: radii about the same centres
             CK(cudaMemsetAsync(ctx->rho_now.p, 0, (size_t)nc * sizeof(unsigned long long), s), "memset");
             k_rho_bodies<<<grid_for(n, 256), 256, 0, s>>>(n, ctx->body_leaf.p, cv, ctx->x.p, ctx->y.p, ctx->z.p,
@@ -794,12 +796,10 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     }
     if (mixed && !dehnen) {
         // normalised FP32 upward pass; FP64 accumulation on the top three levels
-        for (int L = ctx->nlevels - 1; L >= 0; --L) {
-            const int cnt = ctx->lvl_count[L];
-            const unsigned g = std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm);
-            launch_upward_mixed(L <= 2, g, 4, s, ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, ctx->ell.p,
-                                ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, p, ctx->mom_f.p);
-        }
+        CK(cudaMemsetAsync(ctx->up_arrive.p, 0, (size_t)nc * sizeof(unsigned), s), "memset");
+        const int ntop = ctx->nlevels > 3 ? ctx->lvl_start[3] : nc;
+        launch_upward_mixed(s, ctx->level_cells.p, ntop, nc, cv, ctx->c_parent.p, ctx->ell.p, ctx->x.p, ctx->y.p,
+                            ctx->z.p, ctx->m.p, p, ctx->mom_f.p, ctx->up_arrive.p);
         CKL("upward (mixed)");
     } else {
         const int warps = 2;  // the P2M tables take 35 KB of shared memory per warp at p = 10
@@ -810,21 +810,19 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         if (smem_b > 48 * 1024)
             CK(cudaFuncSetAttribute(k_m2m_exact_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b),
                "attr");
-        // per level: the leaves' P2M (a warp per leaf), then the internal
-        // cells' M2M (a block per cell)
-        for (int L = ctx->nlevels - 1; L >= 0; --L) {
+        // the leaves' P2M (a warp per leaf), then level by level the internal
+        // cells' M2M (a block per cell, a wide one where a level has few)
+        k_upward_exact<<<std::min<unsigned>((nc + warps - 1) / warps, 16u * (unsigned)ctx->nsm), 32 * warps, smem, s>>>(
+            ctx->level_cells.p, 0, nc, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, p, ctx->moments.p, ctx->pows.p,
+            dehnen ? ctx->f.p : nullptr, ctx->fmin.p);
+        for (int L = ctx->nlevels - 2; L >= 0; --L) {
             const int cnt = ctx->lvl_count[L];
-            unsigned g = std::min<unsigned>((cnt + warps - 1) / warps, 16u * (unsigned)ctx->nsm);
-            k_upward_exact<<<g, 32 * warps, smem, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, ctx->x.p,
-                                                       ctx->y.p, ctx->z.p, ctx->m.p, p, ctx->moments.p, ctx->pows.p,
-                                                       dehnen ? ctx->f.p : nullptr, ctx->fmin.p, 1);
-            if (L < ctx->nlevels - 1) {
-                k_m2m_exact_block<<<std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm), 256, smem_b, s>>>(
-                    ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, p, ctx->moments.p, ctx->pows.p,
-                    dehnen ? ctx->f.p : nullptr, ctx->fmin.p);
-                LCOUNT(1);
-            }
+            k_m2m_exact_block<<<std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm),
+                                cnt <= 8 * ctx->nsm ? M2M_EXACT_WIDE : 256, smem_b, s>>>(
+                ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, p, ctx->moments.p, ctx->pows.p,
+                dehnen ? ctx->f.p : nullptr, ctx->fmin.p);
         }
+        LCOUNT(ctx->nlevels);
         CKL("upward");
         if (mixed) {  // the MAC saw exact FP64 moments; the translations use FP32
             k_moments_to_mixed<<<grid_for((size_t)nc * H, 256), 256, 0, s>>>(nc, p, ctx->moments.p, ctx->ell.p,
@@ -1011,7 +1009,7 @@ fmmx_status fmmx_create(const fmmx_config* cfg, fmmx_ctx** out) {
     fmmx_ctx* ctx = new fmmx_ctx();
     tl_registry = nullptr;
     for (DBufBase* b : reg)
-        if (b != &ctx->swap_dev) ctx->cache.push_back(b);
+        if (b != &ctx->swap_dev && b != &ctx->l2l_sched) ctx->cache.push_back(b);
     ctx->cfg = c;
     ctx->budget.limit = c.device_budget_bytes;
     BudgetScope bscope(&ctx->budget);
@@ -1053,6 +1051,16 @@ fmmx_status fmmx_create(const fmmx_config* cfg, fmmx_ctx** out) {
     upload_tables_sweeps(ctx->tab, ctx->stream);
     upload_tables_mixed(ctx->tab, ctx->stream);
     build_swap(c.p, ctx->swap_host);
+    std::vector<uint32_t> sched;
+    l2l_schedule(c.p, sched);
+    if (ctx->l2l_sched.ensure(sched.size()) != cudaSuccess ||
+        cudaMemcpyAsync(ctx->l2l_sched.p, sched.data(), sched.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                        ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        fmmx_destroy(ctx);
+        return FMMX_DEVICE_ERROR;
+    }
     if (ctx->swap_dev.ensure(ctx->swap_host.size()) != cudaSuccess ||
         cudaMemcpyAsync(ctx->swap_dev.p, ctx->swap_host.data(), ctx->swap_host.size() * sizeof(double),
                         cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||

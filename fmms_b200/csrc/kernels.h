@@ -2,6 +2,8 @@
 // kernel files and the host orchestration (engine.cu).
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace fmmx {
@@ -100,7 +102,8 @@ __host__ __device__ inline int p2m_round(int p) { return p <= 12 ? 32 : (p <= 16
 __host__ __device__ size_t upward_exact_smem_per_warp(int p);
 __global__ void k_upward_exact(const int32_t* level_cells, int lstart, int lcnt, CellsView cells, const double* x,
                                const double* y, const double* z, const double* m, int p, zd* moments, double* pows,
-                               const double* f, double* fmin, int skip_internal);
+                               const double* f, double* fmin);
+#define M2M_EXACT_WIDE 512  // threads where a level has few cells (N = 1e5, 14 levels: see the kernel)
 __global__ void k_m2m_exact_block(const int32_t* level_cells, int lstart, int lcnt, CellsView cells, int p,
                                   zd* moments, double* pows, const double* f, double* fmin);
 #define FPRE_WARPS 2
@@ -205,11 +208,13 @@ __global__ void k_rho_bodies(size_t n, const int32_t* body_leaf, CellsView cv, c
 __global__ void k_rho_level(const int32_t* level_cells, int lstart, int lcnt, CellsView cv,
                             unsigned long long* rho_bits);
 __global__ void k_moments_to_mixed(int nc, int p, const zd* full, const double* ell, zf* half);
-void launch_upward_mixed(bool fp64, unsigned grid, int warps, cudaStream_t s, const int32_t* level_cells,
-                         int lstart, int lcnt, CellsView cv, const double* ell, const double* x, const double* y,
-                         const double* z, const double* m, int p, zf* mom);
+// top: cells of the top three levels, ntop of them; arrive: nc zeros
+void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, CellsView cv, const int32_t* parent,
+                         const double* ell, const double* x, const double* y, const double* z, const double* m, int p,
+                         zf* mom, unsigned* arrive);
+void l2l_schedule(int p, std::vector<uint32_t>& out);  // the product list k_l2l_mixed works through
 void launch_l2l_mixed(bool fp64, unsigned grid, cudaStream_t s, const int32_t* level_cells, int lstart, int lcnt,
-                      CellsView cv, const int32_t* parent, const double* ell, int p, zf* loc);
+                      CellsView cv, const int32_t* parent, const double* ell, int p, const uint32_t* sched, zf* loc);
 __global__ void k_l2p_mixed(size_t n, const int32_t* body_leaf, const uint32_t* order, CellsView cv,
                             const double* ell, int p, const zf* loc, const double* x, const double* y,
                             const double* z, const double* nax, const double* nay, const double* naz,

@@ -14,6 +14,7 @@
 //   L2P: Ψ_0^0 = (1/l) sum conj(Υ_k^l(r^)) F^_k^l,  Ψ_1^m = (1/l^2) sum conj(Υ_k^l(r^)) F^_{k+1}^{m+l}
 // (the unnormalised forms are moments.rs:30-90 and translate.rs:175-309).
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -26,8 +27,32 @@ namespace fmmx {
 // from L1 in parallel.
 static __device__ OrderTables g_tab;
 
+// FP32 copies of the recursion's constants (a double read would need a
+// conversion per use).
+struct FloatTables {
+    float inv2m[FMMX_MAXP + 1];
+    float invc[FMMX_MAXP + 1][FMMX_MAXP + 1];
+};
+static __device__ FloatTables g_tabf;
+template <typename A>
+__device__ __forceinline__ A tab_inv2m(int m) {
+    if constexpr (sizeof(A) == 4) return g_tabf.inv2m[m];
+    else return g_tab.inv2m[m];
+}
+template <typename A>
+__device__ __forceinline__ A tab_invc(int n, int m) {
+    if constexpr (sizeof(A) == 4) return g_tabf.invc[n][m];
+    else return g_tab.invc[n][m];
+}
+
 void upload_tables_mixed(const OrderTables& t, cudaStream_t s) {
     cudaMemcpyToSymbolAsync(g_tab, &t, sizeof(t), 0, cudaMemcpyHostToDevice, s);
+    FloatTables f;
+    for (int m = 0; m <= FMMX_MAXP; ++m) f.inv2m[m] = (float)t.inv2m[m];
+    for (int n = 0; n <= FMMX_MAXP; ++n)
+        for (int m = 0; m <= FMMX_MAXP; ++m) f.invc[n][m] = (float)t.invc[n][m];
+    cudaMemcpyToSymbolAsync(g_tabf, &f, sizeof(f), 0, cudaMemcpyHostToDevice, s);
+    cudaStreamSynchronize(s);  // the staging copy dies here
 }
 
 __host__ __device__ constexpr int hx(int n, int m) { return n * (n + 1) / 2 + m; }
@@ -38,30 +63,6 @@ __device__ __forceinline__ void split_h(int e, int& n, int& m) {
     while ((q + 1) * (q + 2) / 2 <= e) ++q;
     n = q;
     m = e - q * (q + 1) / 2;
-}
-
-// v_{n,m} for any m from the half store (m >= 0)
-template <typename T>
-__device__ __forceinline__ cplx<T> half_get(const cplx<T>* v, int n, int m) {
-    if (m >= 0) return v[hx(n, m)];
-    const cplx<T> w = v[hx(n, -m)];
-    return ((-m) & 1) ? mk<T>(-w.re, w.im) : mk<T>(w.re, -w.im);
-}
-
-// Υ column m (harmonic.rs:141-173) of r into u (half layout), precision A.
-template <typename A>
-__device__ __forceinline__ void ups_column(A x, A y, A z, A r2, int p, int m, cplx<A>* u) {
-    cplx<A> d = mk<A>(A(1), A(0));
-    for (int j = 1; j <= m; ++j) d = zmul(zscale(mk<A>(x, y), (A)g_tab.inv2m[j]), d);
-    u[hx(m, m)] = d;
-    cplx<A> u1 = d, u2 = mk<A>(A(0), A(0));
-    for (int n = m + 1; n <= p; ++n) {
-        const A a = (A)(2 * n - 1) * z;
-        cplx<A> un = zscale(zsub(zscale(u1, a), zscale(u2, r2)), (A)g_tab.invc[n][m]);
-        u[hx(n, m)] = un;
-        u2 = u1;
-        u1 = un;
-    }
 }
 
 // Normalising length of every cell: rho, or the cell's box size h when rho = 0
@@ -129,162 +130,93 @@ __global__ void k_moments_to_mixed(int nc, int p, const zd* __restrict__ full, c
     }
 }
 
-// P2M / M2M for one level, one 128-thread CTA per cell. A = accumulation type
-// (double on the top three levels, float below). Output FP32 half layout.
-//  - leaf (P2M): thread t takes column m = t % (p+1) of the bodies
-//    g, g+G, g+2G, ... (g = t / (p+1), G <= 8 groups), accumulating the column
-//    in its own shared-memory entries; the group partials are then summed in a
-//    fixed order;
-//  - internal (M2M): first the Υ tables of the eight child offsets (one thread
-//    per child and column), then one thread per (child, entry) computes that
-//    child's contribution, and the children are summed in octant order.
-#define UPM_BLOCK 128
+// P2M of the leaves among cells [0, nc) (list == nullptr) or list[0 .. nc), a
+// warp per leaf and a lane per body: the lane runs through its body's Υ and
+// adds m Υ into its own column of shared memory; the columns are summed at the
+// end, lane e taking entry e from its own column on (distinct banks). A =
+// double for the leaves of the top three levels (`top`), float below. Bound by
+// shared memory and latency. (A 128-thread block per leaf, a thread per column
+// and body group, took 0.31 ms for 32,768 leaves of 32 bodies at p = 10.)
 template <typename A>
-__global__ void __launch_bounds__(UPM_BLOCK) k_upward_mixed(const int32_t* __restrict__ level_cells, int lstart,
-                                                            int lcnt, CellsView cv, const double* __restrict__ ell,
-                                                            const double* __restrict__ x,
-                                                            const double* __restrict__ y,
-                                                            const double* __restrict__ z,
-                                                            const double* __restrict__ m, int p,
-                                                            zf* __restrict__ mom) {
-    extern __shared__ unsigned char smem_raw[];
+__global__ void __launch_bounds__(128) k_p2m_mixed(const int32_t* __restrict__ list, int nc, bool top,
+                                                              CellsView cv, const double* __restrict__ ell,
+                                                              const double* __restrict__ x,
+                                                              const double* __restrict__ y,
+                                                              const double* __restrict__ z,
+                                                              const double* __restrict__ m, int p,
+                                                              zf* __restrict__ mom) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int H = (p + 1) * (p + 2) / 2;
-    const int P1 = p + 1;
-    cplx<A>* u = reinterpret_cast<cplx<A>*>(smem_raw);  // 8 x H: Υ of the child offsets
-    cplx<A>* part = u + 8 * H;                          // 8 x H: partial sums
-    zf* cm = reinterpret_cast<zf*>(part + 8 * H);       // 8 x H: the children's moments
-    A* bod = reinterpret_cast<A*>(cm + 8 * H);          // 4 x UPM_BLOCK: a chunk of the leaf's bodies
-    const int tid = threadIdx.x;
-    const int G = min(8, UPM_BLOCK / P1);
-    for (int j = blockIdx.x; j < lcnt; j += gridDim.x) {
-        const int c = level_cells[lstart + j];
+    const int lane = threadIdx.x & 31;
+    cplx<A>* sbuf = reinterpret_cast<cplx<A>*>(smem_raw) + (size_t)(threadIdx.x >> 5) * 32 * H;
+    cplx<A>* col = sbuf + lane;
+    const int wpb = blockDim.x >> 5, warps = gridDim.x * wpb;
+    for (int j = blockIdx.x * wpb + (threadIdx.x >> 5); j < nc; j += warps) {
+        const int c = list ? list[j] : j;
+        if (!cv.leaf[c] || (cv.level[c] <= 2) != top) continue;
         const double sx = cv.cx[c], sy = cv.cy[c], sz = cv.cz[c];
         const double il = 1.0 / ell[c];
-        int nparts;
-        if (cv.leaf[c]) {
-            nparts = G;
-            const int mc = tid % P1, g = tid / P1;
-            cplx<A>* acc = part + g * H;  // this thread's entries hx(n, mc), n >= mc
-            if (g < G)
-                for (int n = mc; n <= p; ++n) acc[hx(n, mc)] = mk<A>(A(0), A(0));
-            const uint32_t f = cv.first[c], cnt = cv.count[c];
-            for (uint32_t b0 = 0; b0 < cnt; b0 += UPM_BLOCK) {
-                // the chunk's bodies, relative and scaled, loaded by all threads at once
-                const uint32_t nb = min((uint32_t)UPM_BLOCK, cnt - b0);
-                __syncthreads();
-                if ((uint32_t)tid < nb) {
-                    const uint32_t q = f + b0 + tid;
-                    bod[tid] = (A)((x[q] - sx) * il);
-                    bod[UPM_BLOCK + tid] = (A)((y[q] - sy) * il);
-                    bod[2 * UPM_BLOCK + tid] = (A)((z[q] - sz) * il);
-                    bod[3 * UPM_BLOCK + tid] = (A)m[q];
+        const uint32_t f = cv.first[c], cnt = cv.count[c];
+        for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
+            const bool mine = b0 + lane < cnt;
+            const uint32_t q = f + b0 + (mine ? lane : 0);
+            const A rx = (A)((x[q] - sx) * il), ry = (A)((y[q] - sy) * il), rz = (A)((z[q] - sz) * il);
+            const A mb = mine ? (A)m[q] : A(0);
+            const A r2 = rx * rx + ry * ry + rz * rz;
+            cplx<A> d = mk<A>(mb, A(0));  // (the mass rides along: the recursions are linear)
+            auto add = [&](int e, cplx<A> v) {
+                if (b0 == 0) {
+                    col[32 * e] = v;
+                } else {
+                    const cplx<A> o = col[32 * e];
+                    col[32 * e] = mk<A>(o.re + v.re, o.im + v.im);
                 }
-                __syncthreads();
-                if (g >= G) continue;
-                for (uint32_t b = g; b < nb; b += G) {
-                    const A rx = bod[b], ry = bod[UPM_BLOCK + b], rz = bod[2 * UPM_BLOCK + b];
-                    const A mb = bod[3 * UPM_BLOCK + b];
-                    const A r2 = rx * rx + ry * ry + rz * rz;
-                    cplx<A> d = mk<A>(A(1), A(0));
-                    for (int q = 1; q <= mc; ++q) d = zmul(zscale(mk<A>(rx, ry), (A)g_tab.inv2m[q]), d);
-                    cplx<A> u1 = d, u2 = mk<A>(A(0), A(0));
-                    acc[hx(mc, mc)].re += d.re * mb;
-                    acc[hx(mc, mc)].im += d.im * mb;
-                    for (int n = mc + 1; n <= p; ++n) {
-                        const A a = (A)(2 * n - 1) * rz;
-                        const cplx<A> un = zscale(zsub(zscale(u1, a), zscale(u2, r2)), (A)g_tab.invc[n][mc]);
-                        u2 = u1;
-                        u1 = un;
-                        acc[hx(n, mc)].re += un.re * mb;
-                        acc[hx(n, mc)].im += un.im * mb;
-                    }
+            };
+            for (int mm = 0; mm <= p; ++mm) {
+                if (mm > 0) d = zmul(zscale(mk<A>(rx, ry), tab_inv2m<A>(mm)), d);
+                int e = hx(mm, mm);
+                add(e, d);
+                cplx<A> u1 = d, u2 = mk<A>(A(0), A(0));
+                for (int n = mm + 1; n <= p; ++n) {
+                    const A a = (A)(2 * n - 1) * rz;
+                    const cplx<A> un = zscale(zsub(zscale(u1, a), zscale(u2, r2)), tab_invc<A>(n, mm));
+                    u2 = u1;
+                    u1 = un;
+                    e += n;  // (n, mm)
+                    add(e, un);
                 }
-            }
-        } else {
-            nparts = 8;
-            for (int w = tid; w < 8 * P1; w += UPM_BLOCK) {
-                const int o = w / P1, mc = w % P1;
-                const int ch = cv.child[8 * c + o];
-                if (ch < 0) continue;
-                const A dx = (A)((cv.cx[ch] - sx) * il), dy = (A)((cv.cy[ch] - sy) * il),
-                        dz = (A)((cv.cz[ch] - sz) * il);
-                ups_column<A>(dx, dy, dz, dx * dx + dy * dy + dz * dz, p, mc, u + o * H);
-            }
-            for (int w = tid; w < 8 * H; w += UPM_BLOCK) {  // stage the children's moments
-                const int o = w / H, e = w % H;
-                const int ch = cv.child[8 * c + o];
-                if (ch >= 0) cm[w] = mom[(size_t)ch * half_stride(p) + e];
-            }
-            __syncthreads();
-            for (int w = tid; w < 8 * H; w += UPM_BLOCK) {
-                const int o = w / H, e = w % H;
-                const int ch = cv.child[8 * c + o];
-                A sr = 0, si = 0;
-                if (ch >= 0) {
-                    int n, mm;
-                    split_h(e, n, mm);
-                    const cplx<A>* uo = u + o * H;
-                    const A ratio = (A)(ell[ch] * il);
-                    const zf* mcv = cm + o * H;
-                    A rpow = 1;  // ratio^{n-k}, built from k = n down
-                    for (int k = n; k >= 0; --k) {
-                        const int nk = n - k;
-                        const int lo = max(-k, mm - nk), hi = min(k, mm + nk);
-                        A tr = 0, ti = 0;
-                        for (int l = lo; l <= hi; ++l) {
-                            const cplx<A> uu = half_get<A>(uo, k, l);
-                            const zf mv = half_get<float>(mcv, nk, mm - l);
-                            tr += uu.re * (A)mv.re - uu.im * (A)mv.im;
-                            ti += uu.re * (A)mv.im + uu.im * (A)mv.re;
-                        }
-                        sr += tr * rpow;
-                        si += ti * rpow;
-                        rpow *= ratio;
-                    }
-                }
-                part[o * H + e] = mk<A>(sr, si);
             }
         }
-        __syncthreads();
+        __syncwarp();
         zf* out = mom + (size_t)c * half_stride(p);
-        for (int e = tid; e < H; e += UPM_BLOCK) {
+        const int nl = (int)min(cnt, 32u);
+        for (int e = lane; e < H; e += 32) {
             A sr = 0, si = 0;
-            for (int q = 0; q < nparts; ++q) {
-                sr += part[q * H + e].re;
-                si += part[q * H + e].im;
+            const cplx<A>* row = sbuf + 32 * e;
+            if (nl == 32) {
+#pragma unroll 8
+                for (int l = 0; l < 32; ++l) {
+                    const cplx<A> v = row[(l + lane) & 31];
+                    sr += v.re;
+                    si += v.im;
+                }
+            } else {  // the first nl columns, from lane mod nl on
+                int l = lane % nl;
+                for (int k = 0; k < nl; ++k) {
+                    const cplx<A> v = row[l];
+                    sr += v.re;
+                    si += v.im;
+                    if (++l == nl) l = 0;
+                }
             }
             out[e] = mk<float>((float)sr, (float)si);
         }
-        __syncthreads();
+        __syncwarp();
     }
 }
 
-template <typename A>
-static size_t upward_smem(int H) {
-    return (size_t)16 * H * sizeof(cplx<A>) + (size_t)8 * H * sizeof(zf) + (size_t)4 * UPM_BLOCK * sizeof(A);
-}
-
-void launch_upward_mixed(bool fp64, unsigned grid, int warps, cudaStream_t s, const int32_t* level_cells,
-                         int lstart, int lcnt, CellsView cv, const double* ell, const double* x, const double* y,
-                         const double* z, const double* m, int p, zf* mom) {
-    (void)warps;
-    const int H = (p + 1) * (p + 2) / 2;
-    // above 48 KB (FP64 levels from p = 14) the kernel must opt in to more shared memory
-    if (fp64) {
-        const size_t sm = upward_smem<double>(H);
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_upward_mixed<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_upward_mixed<double><<<grid, UPM_BLOCK, sm, s>>>(level_cells, lstart, lcnt, cv, ell, x, y, z, m, p, mom);
-    } else {
-        const size_t sm = upward_smem<float>(H);
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_upward_mixed<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_upward_mixed<float><<<grid, UPM_BLOCK, sm, s>>>(level_cells, lstart, lcnt, cv, ell, x, y, z, m, p, mom);
-    }
-}
-
-// Υ column m as ups_column computes it, stored in the full layout (entry
-// (n, m) at n(n+1) + m for |m| <= n), with v_{n,-m} = (-1)^m conj(v_{n,m}).
+// Υ column m (harmonic.rs:141-173) of r in precision A, stored in the full layout
+// (entry (n, m) at n(n+1) + m for |m| <= n), with v_{n,-m} = (-1)^m conj(v_{n,m}).
 template <typename A>
 __device__ __forceinline__ void ups_column_full(A x, A y, A z, A r2, int p, int m, cplx<A>* u) {
     auto put = [&](int n, cplx<A> v) {
@@ -292,16 +224,176 @@ __device__ __forceinline__ void ups_column_full(A x, A y, A z, A r2, int p, int 
         if (m) u[n * (n + 1) - m] = (m & 1) ? mk<A>(-v.re, v.im) : mk<A>(v.re, -v.im);
     };
     cplx<A> d = mk<A>(A(1), A(0));
-    for (int j = 1; j <= m; ++j) d = zmul(zscale(mk<A>(x, y), (A)g_tab.inv2m[j]), d);
+    for (int j = 1; j <= m; ++j) d = zmul(zscale(mk<A>(x, y), tab_inv2m<A>(j)), d);
     put(m, d);
     cplx<A> u1 = d, u2 = mk<A>(A(0), A(0));
     for (int n = m + 1; n <= p; ++n) {
         const A a = (A)(2 * n - 1) * z;
-        const cplx<A> un = zscale(zsub(zscale(u1, a), zscale(u2, r2)), (A)g_tab.invc[n][m]);
+        const cplx<A> un = zscale(zsub(zscale(u1, a), zscale(u2, r2)), tab_invc<A>(n, m));
         put(n, un);
         u2 = u1;
         u1 = un;
     }
+}
+
+// M2M of every internal cell in one launch: a block per cell, up the tree from
+// the cells without internal children (the leaves' moments are there); the block
+// that finishes a cell's last internal child goes on with the cell, so no block
+// waits. First the Υ of the eight child offsets (a thread per child and column)
+// and the children's moments, both in the full layout (both signs of m), so that
+// a product is two loads and four FMAs; then a thread per (child, entry) sums that
+// child's contribution and the children are added in octant order. A = double on
+// the top three levels, float below. Bound by latency: the products of a cell
+// (13,700 at p = 10) take a few hundred instructions a thread. arrive: one zero
+// per cell. (With P2M in the same kernel and a launch per level: N = 1e3, 7
+// levels, 0.15 ms; N = 2^20 uniform 0.70 ms.)
+#define M2M_BLOCK 256
+#define M2M_SCAN 32  // cells a block looks over at a time for its starting points
+template <typename A>
+__device__ __forceinline__ void m2m_cell(int c, const int* __restrict__ ch, CellsView cv,
+                                         const double* __restrict__ ell, int p, zf* __restrict__ mom,
+                                         unsigned char* smem_raw) {
+    const int P1 = p + 1, H = P1 * (P1 + 1) / 2, F2 = P1 * P1;
+    cplx<A>* u = reinterpret_cast<cplx<A>*>(smem_raw);  // 8 x F2: Υ of the child offsets
+    cplx<A>* part = u + 8 * F2;                         // 8 x H: the children's contributions
+    zf* cm = reinterpret_cast<zf*>(part + 8 * H);       // 8 x F2: the children's moments
+    const int tid = threadIdx.x;
+    const double sx = cv.cx[c], sy = cv.cy[c], sz = cv.cz[c];
+    const double il = 1.0 / ell[c];
+    for (int w = tid; w < 8 * P1; w += M2M_BLOCK) {
+        const int o = w / P1, mc = w % P1;
+        if (ch[o] < 0) continue;
+        const A dx = (A)((cv.cx[ch[o]] - sx) * il), dy = (A)((cv.cy[ch[o]] - sy) * il),
+                dz = (A)((cv.cz[ch[o]] - sz) * il);
+        ups_column_full<A>(dx, dy, dz, dx * dx + dy * dy + dz * dz, p, mc, u + o * F2);
+    }
+    for (int w = tid; w < 8 * H; w += M2M_BLOCK) {  // (written by other SMs in this launch: read past the L1)
+        const int o = w / H, e = w % H;
+        if (ch[o] < 0) continue;
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(mom + (size_t)ch[o] * half_stride(p)) + e);
+        int n, mm;
+        split_h(e, n, mm);
+        zf* t = cm + o * F2 + n * (n + 1);
+        t[mm] = mk<float>(v.x, v.y);
+        if (mm) t[-mm] = (mm & 1) ? mk<float>(-v.x, v.y) : mk<float>(v.x, -v.y);
+    }
+    __syncthreads();
+    for (int w = tid; w < 8 * H; w += M2M_BLOCK) {
+        const int o = w / H, e = w % H;
+        A sr = 0, si = 0;
+        if (ch[o] >= 0) {
+            int n, mm;
+            split_h(e, n, mm);
+            const A ratio = (A)(ell[ch[o]] * il);
+            A rpow = 1;  // ratio^{n-k}, built from k = n down
+            for (int k = n; k >= 0; --k) {
+                const int nk = n - k;
+                const int lo = max(-k, mm - nk), hi = min(k, mm + nk);
+                const cplx<A>* uk = u + o * F2 + k * (k + 1);
+                const zf* mk_ = cm + o * F2 + nk * (nk + 1) + mm;
+                A tr = 0, ti = 0;
+                for (int l = lo; l <= hi; ++l) {
+                    const cplx<A> uu = uk[l];
+                    const zf mv = mk_[-l];
+                    tr += uu.re * (A)mv.re - uu.im * (A)mv.im;
+                    ti += uu.re * (A)mv.im + uu.im * (A)mv.re;
+                }
+                sr += tr * rpow;
+                si += ti * rpow;
+                rpow *= ratio;
+            }
+        }
+        part[o * H + e] = mk<A>(sr, si);
+    }
+    __syncthreads();
+    zf* out = mom + (size_t)c * half_stride(p);
+    for (int e = tid; e < H; e += M2M_BLOCK) {
+        A sr = 0, si = 0;
+        for (int o = 0; o < 8; ++o) {
+            sr += part[o * H + e].re;
+            si += part[o * H + e].im;
+        }
+        out[e] = mk<float>((float)sr, (float)si);
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(M2M_BLOCK) k_m2m_mixed(int nc, CellsView cv, const int32_t* __restrict__ parent,
+                                                        const double* __restrict__ ell, int p, zf* __restrict__ mom,
+                                                        unsigned* __restrict__ arrive) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int ch[8], start[M2M_SCAN], nstart, next;
+    const int tid = threadIdx.x;
+    for (int b = blockIdx.x * M2M_SCAN; b < nc; b += gridDim.x * M2M_SCAN) {
+        if (tid < M2M_SCAN) {  // internal cells without internal children, in order
+            const int c = b + tid;
+            bool first = c < nc && !cv.leaf[c];
+            if (first)
+                for (int o = 0; o < 8; ++o) {
+                    const int q = cv.child[8 * (size_t)c + o];
+                    if (q >= 0 && !cv.leaf[q]) first = false;
+                }
+            const unsigned mask = __ballot_sync(0xffffffffu, first);
+            if (first) start[__popc(mask & ((1u << tid) - 1u))] = c;
+            if (tid == 0) nstart = __popc(mask);
+        }
+        __syncthreads();
+        const int ns = nstart;
+        for (int k = 0; k < ns; ++k) {
+            for (int c = start[k]; c >= 0;) {
+                if (tid < 8) ch[tid] = cv.child[8 * (size_t)c + tid];
+                __syncthreads();
+                if (cv.level[c] <= 2) m2m_cell<double>(c, ch, cv, ell, p, mom, smem_raw);
+                else m2m_cell<float>(c, ch, cv, ell, p, mom, smem_raw);
+                // the parent, if this was its last internal child
+                if (tid < 32) {
+                    const int par = parent[c];
+                    int go = -1;
+                    if (par >= 0) {
+                        const int q = tid < 8 ? cv.child[8 * (size_t)par + tid] : -1;
+                        const unsigned inner = __ballot_sync(0xffffffffu, q >= 0 && !cv.leaf[q]);
+                        if (tid == 0) {
+                            __threadfence();  // the block's moments (ordered before by the barrier) before the arrival
+                            if (atomicAdd(&arrive[par], 1u) + 1 == (unsigned)__popc(inner)) {
+                                __threadfence();
+                                go = par;
+                            }
+                        }
+                    }
+                    if (tid == 0) next = go;
+                }
+                __syncthreads();
+                c = next;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+}
+
+// top: cells of the top three levels, ntop of them; nc cells in all
+void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, CellsView cv, const int32_t* parent,
+                         const double* ell, const double* x, const double* y, const double* z, const double* m, int p,
+                         zf* mom, unsigned* arrive) {
+    const int H = (p + 1) * (p + 2) / 2, F2 = (p + 1) * (p + 1);
+    // (the limits are the same whatever p, so that contexts of other orders on other threads cannot lower them)
+    const size_t most = 200 * 1024;
+    cudaFuncSetAttribute(k_p2m_mixed<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    cudaFuncSetAttribute(k_p2m_mixed<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    cudaFuncSetAttribute(k_m2m_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    auto warps = [&](size_t col) {  // per block: as many as its columns leave room for, 1 .. 4
+        int w = 4;
+        while (w > 1 && w * col > most) w >>= 1;
+        return w;
+    };
+    const size_t cf = (size_t)32 * H * sizeof(zf), cd = (size_t)32 * H * sizeof(zd);
+    const int wf = warps(cf), wd = warps(cd);
+    k_p2m_mixed<double><<<grid_for(ntop, wd), 32 * wd, wd * cd, s>>>(top, ntop, true, cv, ell, x, y, z, m, p, mom);
+    if (nc > ntop)
+        k_p2m_mixed<float><<<grid_for(nc, wf), 32 * wf, wf * cf, s>>>(nullptr, nc, false, cv, ell, x, y, z, m, p, mom);
+    const size_t sm = 8 * (size_t)(F2 + H) * sizeof(zd) + 8 * (size_t)F2 * sizeof(zf);
+    if (nc > 1)
+        k_m2m_mixed<<<grid_for(nc, M2M_SCAN), M2M_BLOCK, sm, s>>>(nc, cv, parent, ell, p, mom, arrive);
 }
 
 // L2L for the cells of one level (L >= 1), one warp per cell; A as above.
@@ -316,14 +408,33 @@ __device__ __forceinline__ void ups_column_full(A x, A y, A z, A r2, int p, int 
 // run is finished there; one that crosses runs leaves a partial sum in each
 // (slot 0: the output the run starts in, slot 1: the one it ends in), added
 // afterwards, in lane order, by the lane holding its first product -- a fixed
-// order, so the result bits do not depend on scheduling. The list is built
-// by every block at its start (item: Υ index, parent index, output, and a
-// last-product flag); Υ and the parent's locals sit in shared memory in the
-// full layout (both signs of m), so a product is two loads and four FMAs.
+// order, so the result bits do not depend on scheduling. The list (item: Υ
+// index, parent index, output, and a last-product flag) is made once per
+// context, l2l_schedule; every block copies it (building it in the kernel took
+// most of the 14 us of a launch over a few cells). Υ and the parent's locals sit
+// in shared memory in the full layout (both signs of m), so a product is two
+// loads and four FMAs.
 #define L2LB_WARPS 4
 
 __host__ __device__ constexpr int l2l_items(int p) {
     return (p + 1) * (p + 2) * (p + 2) * (p + 3) / 12;
+}
+
+// first item | n << 16 of every output (and the item count), then the items
+void l2l_schedule(int p, std::vector<uint32_t>& out) {
+    const int H = (p + 1) * (p + 2) / 2, T = l2l_items(p);
+    out.assign(H + 1 + T, 0);
+    int s = 0;
+    for (int n = 0; n <= p; ++n)
+        for (int m = 0; m <= n; ++m) {
+            const int e = hx(n, m);
+            out[e] = (uint32_t)s | ((uint32_t)n << 16);
+            for (int k = 0; k <= p - n; ++k)
+                for (int l = -k; l <= k; ++l, ++s)
+                    out[H + 1 + s] = (uint32_t)(k * (k + 1) + l) | ((uint32_t)((n + k) * (n + k + 1) + m + l) << 9) |
+                                     ((uint32_t)e << 18) | (k == p - n && l == k ? 0x80000000u : 0u);
+        }
+    out[H] = (uint32_t)T;
 }
 
 template <typename A>
@@ -338,6 +449,7 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
                                                               int lcnt, CellsView cv,
                                                               const int32_t* __restrict__ parent,
                                                               const double* __restrict__ ell, int p,
+                                                              const uint32_t* __restrict__ sched,
                                                               zf* __restrict__ loc) {
     extern __shared__ __align__(16) unsigned char lsm[];
     const int P1 = p + 1, H = P1 * (P1 + 1) / 2, F2 = P1 * P1, T = l2l_items(p);
@@ -351,20 +463,7 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
                                                   L2LB_WARPS * F2);  // first item | n << 16
     uint32_t* items = einfo + H + 1;
 
-    for (int e = threadIdx.x; e < H; e += blockDim.x) {
-        int n, m;
-        split_h(e, n, m);
-        int s = 0;
-        for (int q = 0; q < n; ++q) s += (q + 1) * (p - q + 1) * (p - q + 1);
-        const int w = p - n + 1;
-        s += m * w * w;
-        einfo[e] = (uint32_t)s | ((uint32_t)n << 16);
-        for (int k = 0; k <= p - n; ++k)
-            for (int l = -k; l <= k; ++l, ++s)
-                items[s] = (uint32_t)(k * (k + 1) + l) | ((uint32_t)((n + k) * (n + k + 1) + m + l) << 9) |
-                           ((uint32_t)e << 18) | (k == p - n && l == k ? 0x80000000u : 0u);
-    }
-    if (threadIdx.x == 0) einfo[H] = (uint32_t)T;
+    for (int e = threadIdx.x; e < H + 1 + T; e += blockDim.x) einfo[e] = sched[e];
     __syncthreads();
 
     const int W = ((T + 31) / 32) | 1;  // an odd stride keeps the lanes' item reads on distinct banks
@@ -434,22 +533,31 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
 }
 
 void launch_l2l_mixed(bool fp64, unsigned grid, cudaStream_t s, const int32_t* level_cells, int lstart, int lcnt,
-                      CellsView cv, const int32_t* parent, const double* ell, int p, zf* loc) {
+                      CellsView cv, const int32_t* parent, const double* ell, int p, const uint32_t* sched,
+                      zf* loc) {
     const unsigned blocks = std::max(1u, std::min(grid, (unsigned)((lcnt + L2LB_WARPS - 1) / L2LB_WARPS)));
     if (fp64) {
         const size_t sm = l2l_smem<double>(p);
         if (sm > 48 * 1024)
             cudaFuncSetAttribute(k_l2l_mixed<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_l2l_mixed<double><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, loc);
+        k_l2l_mixed<double><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
+                                                               loc);
     } else {
         const size_t sm = l2l_smem<float>(p);
         if (sm > 48 * 1024)
             cudaFuncSetAttribute(k_l2l_mixed<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_l2l_mixed<float><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, loc);
+        k_l2l_mixed<float><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
+                                                               loc);
     }
 }
 
-// L2P at every body plus the near field, scattered to particle-id order.
+// L2P at every body plus the near field, scattered to particle-id order: a
+// thread per body, Υ of its offset generated column by column (two-term
+// recursion in k) and contracted on the fly. The orders +l and -l of a real field
+// contribute equally to Ψ_0^0 and Ψ_1^0, and to Ψ_1^1 through L_{k+1,l+1} and
+// L_{k+1,l-1}, so only l >= 0 is run through; L_{k,l} is the last step's
+// L_{k+1,l}. Bound by issue (N = 2^20, p = 10: 0.25 ms with both signs written
+// out).
 __global__ void k_l2p_mixed(size_t n, const int32_t* __restrict__ body_leaf, const uint32_t* __restrict__ order,
                             CellsView cv, const double* __restrict__ ell, int p, const zf* __restrict__ loc,
                             const double* __restrict__ x, const double* __restrict__ y,
@@ -466,40 +574,32 @@ __global__ void k_l2p_mixed(size_t n, const int32_t* __restrict__ body_leaf, con
         float p00 = 0, p11r = 0, p11i = 0, p10 = 0;
         zf d = mk<float>(1.f, 0.f);
         for (int lm = 0; lm <= p; ++lm) {
-            if (lm > 0) d = zmul(zscale(mk<float>(rx, ry), (float)g_tab.inv2m[lm]), d);
-            zf u1 = d, u2 = mk<float>(0.f, 0.f);
-            const float sgn = (lm & 1) ? -1.f : 1.f;
+            if (lm > 0) d = zmul(zscale(mk<float>(rx, ry), g_tabf.inv2m[lm]), d);
+            zf u = d, u2 = mk<float>(0.f, 0.f);
+            zf f0 = L[hx(lm, lm)];
+            float s00 = 0, s10 = 0;
             for (int kk = lm; kk <= p; ++kk) {
-                zf uk;
-                if (kk == lm) {
-                    uk = d;
-                } else {
-                    const float a = (float)(2 * kk - 1) * rz;
-                    uk = zscale(zsub(zscale(u1, a), zscale(u2, r2)), (float)g_tab.invc[kk][lm]);
-                    u2 = u1;
-                    u1 = uk;
-                }
-                const zf f0 = L[hx(kk, lm)];
-                p00 += uk.re * f0.re + uk.im * f0.im;
-                if (kk < p) {
-                    const zf f11 = half_get<float>(L, kk + 1, lm + 1);
-                    const zf f10 = L[hx(kk + 1, lm)];
-                    p11r += uk.re * f11.re + uk.im * f11.im;
-                    p11i += uk.re * f11.im - uk.im * f11.re;
-                    p10 += uk.re * f10.re + uk.im * f10.im;
-                }
+                s00 += u.re * f0.re + u.im * f0.im;
+                if (kk == p) break;
+                const zf* row = L + hx(kk + 1, lm);
+                const zf f10 = row[0], f11 = row[1];
+                s10 += u.re * f10.re + u.im * f10.im;
+                p11r += u.re * f11.re + u.im * f11.im;
+                p11i += u.re * f11.im - u.im * f11.re;
                 if (lm > 0) {
-                    const zf g0 = half_get<float>(L, kk, -lm);
-                    p00 += sgn * (uk.re * g0.re - uk.im * g0.im);
-                    if (kk < p) {
-                        const zf g11 = half_get<float>(L, kk + 1, 1 - lm);
-                        const zf g10 = half_get<float>(L, kk + 1, -lm);
-                        p11r += sgn * (uk.re * g11.re - uk.im * g11.im);
-                        p11i += sgn * (uk.re * g11.im + uk.im * g11.re);
-                        p10 += sgn * (uk.re * g10.re - uk.im * g10.im);
-                    }
+                    const zf h = row[-1];
+                    p11r -= u.re * h.re + u.im * h.im;
+                    p11i += u.re * h.im - u.im * h.re;
                 }
+                const float a = (float)(2 * kk + 1) * rz;
+                const zf un = zscale(zsub(zscale(u, a), zscale(u2, r2)), g_tabf.invc[kk + 1][lm]);
+                u2 = u;
+                u = un;
+                f0 = f10;
             }
+            const float w = lm > 0 ? 2.f : 1.f;
+            p00 += w * s00;
+            p10 += w * s10;
         }
         const uint32_t id = order[k];
         acc[3 * (size_t)id + 0] = nax[k] - ((double)p11r * il) * il;

@@ -89,8 +89,10 @@ __global__ void __launch_bounds__(SW_BLOCK) k_l2l_f64(const int32_t* __restrict_
 }
 
 // One thread per body (slot order). The Υ table of s - x is generated column
-// by column (two-term recursion in n) and contracted on the fly, so no table
-// is stored.
+// by column (two-term recursion in k) and contracted on the fly, so no table
+// is stored. The locals of a real field mirror (L_{k,-l} = (-1)^l conj(L_{k,l})),
+// so the orders +l and -l contribute equally to Ψ_0^0 and Ψ_1^0, and to Ψ_1^1
+// through L_{k+1,l+1} and L_{k+1,l-1}: only l >= 0 is run through.
 __global__ void k_l2p_f64(size_t n, const int32_t* __restrict__ body_leaf, const uint32_t* __restrict__ order,
                           CellsView cv, int p, const zd* __restrict__ locals, const double* __restrict__ x,
                           const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ nax,
@@ -106,40 +108,31 @@ __global__ void k_l2p_f64(size_t n, const int32_t* __restrict__ body_leaf, const
         zd d = mk(1.0, 0.0);
         for (int l = 0; l <= p; ++l) {
             if (l > 0) d = zmul(zscale(mk(rx, ry), g_tab.inv2m[l]), d);
-            zd u1 = d, u2 = mk(0.0, 0.0);
-            const double sgn = (l & 1) ? -1.0 : 1.0;
+            zd u = d, u2 = mk(0.0, 0.0);
+            zd f0 = L[cidx(l, l)];
+            double s00 = 0.0, s10 = 0.0;
             for (int kk = l; kk <= p; ++kk) {
-                zd uk;
-                if (kk == l) {
-                    uk = d;
-                } else {
-                    const double a = (double)(2 * kk - 1) * rz;
-                    uk = zscale(zsub(zscale(u1, a), zscale(u2, r2)), g_tab.invc[kk][l]);
-                    u2 = u1;
-                    u1 = uk;
-                }
-                // conj(u) * F for +l; conj(u_{k,-l}) = (-1)^l u_{k,l} for -l
-                const zd f0 = L[cidx(kk, l)];
-                p00 += uk.re * f0.re + uk.im * f0.im;
-                if (kk < p) {
-                    const zd f11 = L[cidx(kk + 1, l + 1)];
-                    const zd f10 = L[cidx(kk + 1, l)];
-                    p11r += uk.re * f11.re + uk.im * f11.im;
-                    p11i += uk.re * f11.im - uk.im * f11.re;
-                    p10 += uk.re * f10.re + uk.im * f10.im;
-                }
+                s00 += u.re * f0.re + u.im * f0.im;  // conj(u) * F
+                if (kk == p) break;
+                const zd* row = L + cidx(kk + 1, l);
+                const zd f10 = row[0], f11 = row[1];
+                s10 += u.re * f10.re + u.im * f10.im;
+                p11r += u.re * f11.re + u.im * f11.im;
+                p11i += u.re * f11.im - u.im * f11.re;
                 if (l > 0) {
-                    const zd g0 = L[cidx(kk, -l)];
-                    p00 += sgn * (uk.re * g0.re - uk.im * g0.im);
-                    if (kk < p) {
-                        const zd g11 = L[cidx(kk + 1, 1 - l)];
-                        const zd g10 = L[cidx(kk + 1, -l)];
-                        p11r += sgn * (uk.re * g11.re - uk.im * g11.im);
-                        p11i += sgn * (uk.re * g11.im + uk.im * g11.re);
-                        p10 += sgn * (uk.re * g10.re - uk.im * g10.im);
-                    }
+                    const zd h = row[-1];
+                    p11r -= u.re * h.re + u.im * h.im;
+                    p11i += u.re * h.im - u.im * h.re;
                 }
+                const double a = (double)(2 * kk + 1) * rz;
+                const zd un = zscale(zsub(zscale(u, a), zscale(u2, r2)), g_tab.invc[kk + 1][l]);
+                u2 = u;
+                u = un;
+                f0 = f10;
             }
+            const double w = l > 0 ? 2.0 : 1.0;
+            p00 += w * s00;
+            p10 += w * s10;
         }
         const uint32_t id = order[k];
         acc[3 * (size_t)id + 0] = nax[k] + (0.0 - p11r);

@@ -750,22 +750,18 @@ __device__ __forceinline__ void upsilon_column(double dx, double dy, double dz, 
 }
 
 // Shared memory of k_upward_exact per warp: the cell's accumulator (dim
-// complex), then either the Υ table of an M2M child offset (dim complex) or,
-// for a leaf's P2M, the m >= 0 Υ tables of a round of B bodies, entry-major
-// in separate real and imaginary arrays of stride B + 1 (conflict-free both
-// when a lane writes its body's table and when lanes read one body's
-// entries).
+// complex), then the m >= 0 Υ tables of a round of B bodies, entry-major in
+// separate real and imaginary arrays of stride B + 1 (conflict-free both when a
+// lane writes its body's table and when lanes read one body's entries).
 __host__ __device__ size_t upward_exact_smem_per_warp(int p) {
     const int B = p2m_round(p), H = (p + 1) * (p + 2) / 2;
-    const size_t u = (size_t)dimp(p) * sizeof(zd), tab = 2 * (size_t)H * (B + 1) * sizeof(double);
-    return (size_t)dimp(p) * sizeof(zd) + (u > tab ? u : tab);
+    return (size_t)dimp(p) * sizeof(zd) + 2 * (size_t)H * (B + 1) * sizeof(double);
 }
 
-// One warp per cell of a level, deepest level first (compute_moments,
-// moments.rs:96-108): P2M for leaves (p2m_cell :30-53), M2M for internal
-// cells (m2m_cell :56-90), then the multipole power (:150-168) and, when f is
-// given, fmin (mac.rs:151-173). With skip_internal (the engine's choice), the
-// internal cells of the level are left to k_m2m_exact_block.
+// The leaves among the given cells, a warp each (all levels in one launch; the
+// internal cells follow level by level in k_m2m_exact_block): P2M (p2m_cell,
+// moments.rs:30-53), then the multipole power (:150-168) and, when f is given,
+// fmin (mac.rs:151-173).
 //
 // P2M: the lanes build the Υ tables of B bodies at once (a lane per body, the
 // recursion of upsilon_table_into, harmonic.rs:141-173); then each lane owns
@@ -776,7 +772,7 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
                                const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ m, int p,
                                zd* __restrict__ moments, double* __restrict__ pows, const double* __restrict__ f,
-                               double* __restrict__ fmin_out, int skip_internal) {
+                               double* __restrict__ fmin_out) {
     extern __shared__ unsigned char smem_raw[];
     const int dim = dimp(p);
     const int H = (p + 1) * (p + 2) / 2;
@@ -785,18 +781,17 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
     const int wib = threadIdx.x >> 5;
     unsigned char* wbase = smem_raw + (size_t)wib * upward_exact_smem_per_warp(p);
     zd* acc = reinterpret_cast<zd*>(wbase);
-    zd* u = acc + dim;                                   // M2M: Υ of the child offset
-    double* tre = reinterpret_cast<double*>(acc + dim);  // P2M: Υ tables, real parts
+    double* tre = reinterpret_cast<double*>(acc + dim);  // Υ tables, real parts
     double* tim = tre + (size_t)H * S;                   //      imaginary parts
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int j = warp; j < lcnt; j += nwarps) {
         const int c = level_cells[lstart + j];
-        if (skip_internal && !cells.leaf[c]) continue;
+        if (!cells.leaf[c]) continue;
         const double zx = cells.cx[c], zy = cells.cy[c], zz = cells.cz[c];
         for (int e = lane; e < dim; e += 32) acc[e] = mk(0.0, 0.0);
         __syncwarp();
-        if (cells.leaf[c]) {
+        {
             const uint32_t fst = cells.first[c], end = fst + cells.count[c];
             double ar[8], ai[8];  // this lane's coefficients e = lane + 32 t (m >= 0 half, H <= 231)
 #pragma unroll
@@ -864,28 +859,6 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
                 }
             }
             __syncwarp();
-        } else {
-            for (int o = 0; o < 8; ++o) {
-                const int ch = cells.child[8 * c + o];
-                if (ch < 0) continue;
-                const double dx = cells.cx[ch] - zx, dy = cells.cy[ch] - zy, dz = cells.cz[ch] - zz;
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                for (int mm = lane; mm <= p; mm += 32) upsilon_column(dx, dy, dz, r2, p, mm, u);
-                __syncwarp();
-                const zd* mc = moments + (size_t)ch * dim;
-                for (int e = lane; e < dim; e += 32) {
-                    int n, mm;
-                    split_nm(e, n, mm);
-                    zd s = mk(0.0, 0.0);
-                    for (int k = 0; k <= n; ++k) {
-                        const int nk = n - k;
-                        const int lo = max(-k, mm - nk), hi = min(k, mm + nk);
-                        for (int l = lo; l <= hi; ++l) s = zadd(s, zmul(u[cidx(k, l)], mc[cidx(nk, mm - l)]));
-                    }
-                    acc[e] = zadd(acc[e], s);
-                }
-                __syncwarp();
-            }
         }
         zd* out = moments + (size_t)c * dim;
         for (int e = lane; e < dim; e += 32) out[e] = acc[e];
@@ -901,15 +874,8 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
         }
         if (f != nullptr && lane == 0) {
             double mn = INFINITY;
-            if (cells.leaf[c]) {
-                const uint32_t fst = cells.first[c], end = fst + cells.count[c];
-                for (uint32_t k = fst; k < end; ++k) mn = fmin(mn, f[k]);
-            } else {
-                for (int o = 0; o < 8; ++o) {
-                    int ch = cells.child[8 * c + o];
-                    if (ch >= 0) mn = fmin(mn, fmin_out[ch]);
-                }
-            }
+            const uint32_t fst = cells.first[c], end = fst + cells.count[c];
+            for (uint32_t k = fst; k < end; ++k) mn = fmin(mn, f[k]);
             fmin_out[c] = mn;
         }
         __syncwarp();
@@ -922,7 +888,7 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
 // every coefficient adds its children's sums in octant order, as m2m_cell
 // (moments.rs:56-90) does one child after the other. Power and fmin as in
 // k_upward_exact. Shared memory: 16 dim complex.
-__global__ void __launch_bounds__(256) k_m2m_exact_block(const int32_t* __restrict__ level_cells, int lstart,
+__global__ void __launch_bounds__(M2M_EXACT_WIDE) k_m2m_exact_block(const int32_t* __restrict__ level_cells, int lstart,
                                                          int lcnt, CellsView cells, int p, zd* __restrict__ moments,
                                                          double* __restrict__ pows, const double* __restrict__ f,
                                                          double* __restrict__ fmin_out) {
