@@ -2,7 +2,8 @@
 // reference (direct.rs:6-31 one-sided, and the sampled error of
 // crates/bench/src/main.rs:34-78). Sources are split across blockIdx.y; each
 // split writes its partial sums and k_direct_reduce adds them in split order,
-// so the result is deterministic.
+// so the result is deterministic. Bound by the FP64 pipe (a square root and a
+// division per pair, instead of the one reciprocal root, took half the time).
 #include <mutex>
 
 #include "common.cuh"
@@ -11,6 +12,18 @@
 namespace fmmx {
 
 #define DIR_BLOCK 128
+
+// Splits of the sources for nt targets: 32, and more where there are too few
+// target blocks to fill the GPU (a warp's worth of sources each at least);
+// nsplit * nt stays within 32 x 4096 or, for more targets, 32 nt.
+int direct_splits(size_t n, size_t nt) {
+    const size_t blocks = (nt + DIR_BLOCK - 1) / DIR_BLOCK;
+    const size_t want = 8 * 148 / blocks, room = (size_t)32 * 4096 / (nt < 4096 ? nt : 4096);
+    size_t s = want < room ? want : room;
+    const size_t by_n = (n + DIR_BLOCK - 1) / DIR_BLOCK;
+    if (s > by_n) s = by_n;
+    return (int)(s < 32 ? 32 : s > 1024 ? 1024 : s);
+}
 
 __global__ void __launch_bounds__(DIR_BLOCK) k_direct_targets(const double* __restrict__ pos,
                                                               const double* __restrict__ mass, size_t n,
@@ -24,7 +37,7 @@ __global__ void __launch_bounds__(DIR_BLOCK) k_direct_targets(const double* __re
     const double yi = active ? pos[3 * (size_t)ti + 1] : 0.0;
     const double zi = active ? pos[3 * (size_t)ti + 2] : 0.0;
     const size_t per = (n + gridDim.y - 1) / gridDim.y;
-    const size_t j0 = blockIdx.y * per, j1 = min(n, j0 + per);
+    const size_t j0 = min(n, blockIdx.y * per), j1 = min(n, j0 + per);
     double ax = 0, ay = 0, az = 0, ph = 0, f = 0;
     for (size_t b0 = j0; b0 < j1; b0 += DIR_BLOCK) {
         const size_t j = b0 + threadIdx.x;
@@ -37,11 +50,12 @@ __global__ void __launch_bounds__(DIR_BLOCK) k_direct_targets(const double* __re
         __syncthreads();
         const int nb = (int)min((size_t)DIR_BLOCK, j1 - b0);
         if (active) {
+#pragma unroll 4
             for (int k = 0; k < nb; ++k) {
                 if (b0 + k == ti) continue;
                 const double dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;
                 const double r2 = dx * dx + dy * dy + dz * dz + soft2;
-                const double inv = 1.0 / sqrt(r2);
+                const double inv = rsqrt(r2);
                 const double inv2 = inv * inv;
                 const double inv3 = inv2 * inv;
                 ax += sm[k] * inv3 * dx;
@@ -126,7 +140,7 @@ __global__ void __launch_bounds__(DIR_BLOCK) k_direct_targets_checked(const doub
     const double yi = valid ? pos[3 * (size_t)ti + 1] : 0.0;
     const double zi = valid ? pos[3 * (size_t)ti + 2] : 0.0;
     const size_t per = (n + gridDim.y - 1) / gridDim.y;
-    const size_t j0 = blockIdx.y * per, j1 = min(n, j0 + per);
+    const size_t j0 = min(n, blockIdx.y * per), j1 = min(n, j0 + per);
     double ax = 0, ay = 0, az = 0, ph = 0, f = 0;
     for (size_t b0 = j0; b0 < j1; b0 += DIR_BLOCK) {
         const size_t j = b0 + threadIdx.x;
@@ -139,11 +153,12 @@ __global__ void __launch_bounds__(DIR_BLOCK) k_direct_targets_checked(const doub
         __syncthreads();
         const int nb = (int)min((size_t)DIR_BLOCK, j1 - b0);
         if (valid) {
+#pragma unroll 4
             for (int k = 0; k < nb; ++k) {
                 if (b0 + k == ti) continue;
                 const double dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;
                 const double r2 = dx * dx + dy * dy + dz * dz + soft2;
-                const double inv = 1.0 / sqrt(r2);
+                const double inv = rsqrt(r2);
                 const double inv2 = inv * inv;
                 const double inv3 = inv2 * inv;
                 ax += sm[k] * inv3 * dx;
@@ -208,12 +223,13 @@ extern "C" fmmx_status fmmx_direct_targets_noalloc(int device, void* stream, siz
     if (st == FMMX_OK && cudaPeekAtLastError() != cudaSuccess) st = FMMX_DEVICE_ERROR;
     if (st == FMMX_OK) {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        dim3 g((unsigned)((nt + DIR_BLOCK - 1) / DIR_BLOCK), FMMX_NOALLOC_NSPLIT);
+        const int nsplit = fmmx::direct_splits(n, nt);  // nsplit * nt within the static array
+        dim3 g((unsigned)((nt + DIR_BLOCK - 1) / DIR_BLOCK), (unsigned)nsplit);
         fmmx::k_direct_targets_checked<<<g, DIR_BLOCK, 0, s>>>(d_pos, d_mass, n, d_targets, nt,
                                                                softening * softening, scratch);
         if (cudaGetLastError() != cudaSuccess) st = FMMX_DEVICE_ERROR;
         if (st == FMMX_OK) {
-            fmmx::k_direct_reduce<<<fmmx::grid_for(nt, 128), 128, 0, s>>>(scratch, FMMX_NOALLOC_NSPLIT, nt, d_acc,
+            fmmx::k_direct_reduce<<<fmmx::grid_for(nt, 128), 128, 0, s>>>(scratch, nsplit, nt, d_acc,
                                                                           d_pot, d_fscale);
             if (cudaGetLastError() != cudaSuccess) st = FMMX_DEVICE_ERROR;
         }

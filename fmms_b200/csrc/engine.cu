@@ -1461,22 +1461,31 @@ fmmx_status fmmx_direct_targets(int device, size_t n, const double* pos, const d
     for (size_t q = 0; q < nt; ++q)
         if (targets[q] >= n) return FMMX_INVALID_ARG;
     cudaSetDevice(device);
-    const int nsplit = 32;
-    double *dpos = nullptr, *dmass = nullptr, *part = nullptr, *dacc = nullptr, *dpot = nullptr, *df = nullptr;
-    uint32_t* dt = nullptr;
+    const int nsplit = direct_splits(n, nt);
+    // one allocation for everything (seven cost more than the kernel for 10^5 bodies), in 256-byte steps
+    size_t bytes = 0;
+    auto room = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    };
+    const size_t opos = room(3 * n * 8), omass = room(n * 8), ot = room(nt * 4), opart = room(nsplit * nt * 5 * 8),
+                 oacc = room(nt * 3 * 8), opot = room(nt * 8), of = room(nt * 8);
+    char* d = nullptr;
     fmmx_status st = FMMX_OK;
     cudaStream_t s = nullptr;
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&dpos, 3 * n * 8) != cudaSuccess || cudaMalloc(&dmass, n * 8) != cudaSuccess ||
-        cudaMalloc(&dt, nt * 4) != cudaSuccess || cudaMalloc(&part, nsplit * nt * 5 * 8) != cudaSuccess ||
-        cudaMalloc(&dacc, nt * 3 * 8) != cudaSuccess || cudaMalloc(&dpot, nt * 8) != cudaSuccess ||
-        cudaMalloc(&df, nt * 8) != cudaSuccess) {
+        cudaMalloc((void**)&d, bytes) != cudaSuccess) {
+        cudaGetLastError();
         st = FMMX_OUT_OF_MEMORY;
     } else {
+        double *dpos = (double*)(d + opos), *dmass = (double*)(d + omass), *part = (double*)(d + opart),
+               *dacc = (double*)(d + oacc), *dpot = (double*)(d + opot), *df = (double*)(d + of);
+        uint32_t* dt = (uint32_t*)(d + ot);
         cudaMemcpyAsync(dpos, pos, 3 * n * 8, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(dmass, mass, n * 8, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(dt, targets, nt * 4, cudaMemcpyHostToDevice, s);
-        dim3 g((unsigned)((nt + 127) / 128), nsplit);
+        dim3 g((unsigned)((nt + 127) / 128), (unsigned)nsplit);
         k_direct_targets<<<g, 128, 0, s>>>(dpos, dmass, n, dt, nt, softening * softening, part);
         k_direct_reduce<<<grid_for(nt, 128), 128, 0, s>>>(part, nsplit, nt, dacc, dpot, df);
         cudaMemcpyAsync(acc, dacc, nt * 3 * 8, cudaMemcpyDeviceToHost, s);
@@ -1484,8 +1493,7 @@ fmmx_status fmmx_direct_targets(int device, size_t n, const double* pos, const d
         if (fscale) cudaMemcpyAsync(fscale, df, nt * 8, cudaMemcpyDeviceToHost, s);
         if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) st = FMMX_DEVICE_ERROR;
     }
-    for (void* q : {(void*)dpos, (void*)dmass, (void*)dt, (void*)part, (void*)dacc, (void*)dpot, (void*)df})
-        if (q) cudaFree(q);
+    if (d) cudaFree(d);
     if (s) cudaStreamDestroy(s);
     return st;
 }

@@ -232,6 +232,7 @@ __global__ void k_kick_rows(size_t n3, double* v, const double* a, const double*
 __global__ void k_drift_rows(size_t n3, double* x, const double* v, const double* dt);
 
 // direct.cu
+int direct_splits(size_t n, size_t nt);  // splits of the sources
 __global__ void k_direct_targets(const double* pos, const double* mass, size_t n, const uint32_t* tgt, size_t nt,
                                  double soft2, double* part);
 __global__ void k_direct_reduce(const double* part, int nsplit, size_t nt, double* acc, double* pot, double* fsc);
