@@ -699,8 +699,11 @@ __device__ __forceinline__ void mask_self(float4& a, float4& b, int h, float x, 
 // staging a pair is a lookup, two 16-byte loads, six additions and two 16-byte
 // stores, and the next tile's loads are in flight while a tile is computed. The
 // target's own body is masked only in the tiles that overlap the target leaf.
-// Bound by issue: per interaction 7.5 packed FP32x2 and MUFU instructions plus
-// staging shared by the unit's targets.
+// Bound by the FMA pipe and latency: per interaction 7.5 packed FP32x2 and MUFU
+// instructions plus staging shared by the unit's targets; FMA pipe 62 % busy at 15
+// bodies per leaf. Four blocks per SM of 128 registers and no unrolling of the
+// pair loop (uniform 2^20, leaf 64: 2.03 ms; five blocks of 96 registers 2.08,
+// six of 80 2.08; unrolled by two 2.12, 2.14, 2.12).
 #define P2PW_CHUNK 128
 #define P2PW_MAP 1024
 #define P2PW_WARPS 4
@@ -721,7 +724,7 @@ struct P2pWarpSmem {
 };
 
 template <int TP>
-__global__ void __launch_bounds__(32 * P2PW_WARPS, 5) k_p2p_mixed(DirList L, CellsView cv, P2pUnits U,
+__global__ void __launch_bounds__(32 * P2PW_WARPS, 4) k_p2p_mixed(DirList L, CellsView cv, P2pUnits U,
                                                                 const float4* __restrict__ pairs, float soft2_1,
                                                                 double* __restrict__ ax, double* __restrict__ ay,
                                                                 double* __restrict__ az, double* __restrict__ pot) {
@@ -868,7 +871,7 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS, 5) k_p2p_mixed(DirList L, Cel
                 if (active) {
                     const int last = sp + (int)((tn + 1) >> 1);  // the target leaf's own pairs: sp .. last - 1
                     if (sp < 0 || sp >= (int)b0 + npair || last <= (int)b0) {
-#pragma unroll 2
+#pragma unroll 1
                         for (int j = rep; j < npair; j += R) {
                             const float4 a = S.t.ta[j], b = S.t.tz[j];
                             p2p_pair(a, b, nx0, ny0, nz0, soft2, q0x, q0y, q0z, q0p);
