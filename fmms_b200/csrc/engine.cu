@@ -744,7 +744,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     if (d_mass == nullptr) d_mass = ctx->build_mass;
     k_gather<<<grid_for(n, 256), 256, 0, s>>>(d_pos, d_mass, ctx->order.p, n, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p);
     CKL("gather");
-    LCOUNT(4 + (ctx->cfg.mac_mode == FMMX_MAC_DEHNEN ? 1 : 0));  // gather, upward (mixed; plain counts its own), f pre-pass
+    LCOUNT(4 + (ctx->cfg.mac_mode == FMMX_MAC_DEHNEN ? 2 : 0));  // gather, upward (mixed; plain counts its own), f pre-pass
     CK(ctx->moments.ensure((size_t)nc * dim), "alloc expansions");
     CK(ctx->locals.ensure((size_t)nc * dim), "alloc expansions");
     CK(ctx->pows.ensure((size_t)nc * (p + 1)), "alloc expansions");
@@ -781,17 +781,18 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         k_cell_scale<<<grid_for(nc, 256), 256, 0, s>>>(nc, rho, ctx->c_h.p, ctx->ell.p, ctx->ellf.p);
         LCOUNT(1);
     }
-    // the second stream starts once the bodies are gathered (and, for the
-    // Dehnen MAC, whose walk reads the multipole power and fmin, after the
-    // upward pass)
-    if (!dehnen) {
-        CK(cudaEventRecord(ctx->fork[0], s), "event");
-        CK(cudaStreamWaitEvent(s2, ctx->fork[0], 0), "fork");
-    }
+    // the second stream starts once the bodies are gathered: the walk, or for
+    // the Dehnen MAC the f pre-pass and fmin (its walk reads the multipole power
+    // too and waits for the upward pass)
+    CK(cudaEventRecord(ctx->fork[0], s), "event");
+    CK(cudaStreamWaitEvent(s2, ctx->fork[0], 0), "fork");
     if (dehnen) {
-        CK(cudaMemsetAsync(ctx->flags.p + TF_STACK, 0, sizeof(int), s), "memset");
-        launch_fprepass(s, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, n, ctx->sys_off.p, ctx->nsys,
+        CK(ctx->up_arrive.ensure(nc), "alloc expansions");
+        CK(cudaMemsetAsync(ctx->flags.p + TF_STACK, 0, sizeof(int), s2), "memset");
+        CK(cudaMemsetAsync(ctx->up_arrive.p, 0, (size_t)nc * sizeof(unsigned), s2), "memset");
+        launch_fprepass(s2, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, n, ctx->sys_off.p, ctx->nsys,
                         ctx->level_cells.p, ctx->f.p, ctx->flags.p + TF_STACK);
+        k_fmin<<<grid_for(nc, 4), 128, 0, s2>>>(nc, cv, ctx->c_parent.p, ctx->f.p, ctx->fmin.p, ctx->up_arrive.p);
         CKL("f pre-pass");
     }
     if (mixed && !dehnen) {
@@ -813,14 +814,12 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         // the leaves' P2M (a warp per leaf), then level by level the internal
         // cells' M2M (a block per cell, a wide one where a level has few)
         k_upward_exact<<<std::min<unsigned>((nc + warps - 1) / warps, 16u * (unsigned)ctx->nsm), 32 * warps, smem, s>>>(
-            ctx->level_cells.p, 0, nc, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, p, ctx->moments.p, ctx->pows.p,
-            dehnen ? ctx->f.p : nullptr, ctx->fmin.p);
+            ctx->level_cells.p, 0, nc, cv, ctx->x.p, ctx->y.p, ctx->z.p, ctx->m.p, p, ctx->moments.p, ctx->pows.p);
         for (int L = ctx->nlevels - 2; L >= 0; --L) {
             const int cnt = ctx->lvl_count[L];
             k_m2m_exact_block<<<std::min<unsigned>(cnt, 16u * (unsigned)ctx->nsm),
                                 cnt <= 8 * ctx->nsm ? M2M_EXACT_WIDE : 256, smem_b, s>>>(
-                ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, p, ctx->moments.p, ctx->pows.p,
-                dehnen ? ctx->f.p : nullptr, ctx->fmin.p);
+                ctx->level_cells.p, ctx->lvl_start[L], cnt, cv, p, ctx->moments.p, ctx->pows.p);
         }
         LCOUNT(ctx->nlevels);
         CKL("upward");

@@ -101,11 +101,12 @@ __global__ void k_geometry_level(const int32_t* level_cells, int lstart, int lcn
 __host__ __device__ inline int p2m_round(int p) { return p <= 12 ? 32 : (p <= 16 ? 16 : 8); }
 __host__ __device__ size_t upward_exact_smem_per_warp(int p);
 __global__ void k_upward_exact(const int32_t* level_cells, int lstart, int lcnt, CellsView cells, const double* x,
-                               const double* y, const double* z, const double* m, int p, zd* moments, double* pows,
-                               const double* f, double* fmin);
-#define M2M_EXACT_WIDE 512  // threads where a level has few cells (N = 1e5, 14 levels: see the kernel)
+                               const double* y, const double* z, const double* m, int p, zd* moments, double* pows);
+#define M2M_EXACT_WIDE 512  // threads where a level has few cells
 __global__ void k_m2m_exact_block(const int32_t* level_cells, int lstart, int lcnt, CellsView cells, int p,
-                                  zd* moments, double* pows, const double* f, double* fmin);
+                                  zd* moments, double* pows);
+__global__ void k_fmin(int nc, CellsView cv, const int32_t* parent, const double* f, double* fmin_out,
+                       unsigned* arrive);
 #define FPRE_WARPS 2
 void launch_fprepass(cudaStream_t s, CellsView cells, const double* x, const double* y, const double* z,
                      const double* m, size_t n, const uint64_t* off, int nsys, const int32_t* roots, double* f,

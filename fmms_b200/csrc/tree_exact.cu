@@ -760,8 +760,7 @@ __host__ __device__ size_t upward_exact_smem_per_warp(int p) {
 
 // The leaves among the given cells, a warp each (all levels in one launch; the
 // internal cells follow level by level in k_m2m_exact_block): P2M (p2m_cell,
-// moments.rs:30-53), then the multipole power (:150-168) and, when f is given,
-// fmin (mac.rs:151-173).
+// moments.rs:30-53), then the multipole power (:150-168).
 //
 // P2M: the lanes build the Υ tables of B bodies at once (a lane per body, the
 // recursion of upsilon_table_into, harmonic.rs:141-173); then each lane owns
@@ -771,8 +770,7 @@ __host__ __device__ size_t upward_exact_smem_per_warp(int p) {
 __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lstart, int lcnt, CellsView cells,
                                const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ m, int p,
-                               zd* __restrict__ moments, double* __restrict__ pows, const double* __restrict__ f,
-                               double* __restrict__ fmin_out) {
+                               zd* __restrict__ moments, double* __restrict__ pows) {
     extern __shared__ unsigned char smem_raw[];
     const int dim = dimp(p);
     const int H = (p + 1) * (p + 2) / 2;
@@ -872,12 +870,6 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
             }
             pows[(size_t)c * (p + 1) + n] = sqrt(s);
         }
-        if (f != nullptr && lane == 0) {
-            double mn = INFINITY;
-            const uint32_t fst = cells.first[c], end = fst + cells.count[c];
-            for (uint32_t k = fst; k < end; ++k) mn = fmin(mn, f[k]);
-            fmin_out[c] = mn;
-        }
         __syncwarp();
     }
 }
@@ -890,8 +882,7 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
 // k_upward_exact. Shared memory: 16 dim complex.
 __global__ void __launch_bounds__(M2M_EXACT_WIDE) k_m2m_exact_block(const int32_t* __restrict__ level_cells, int lstart,
                                                          int lcnt, CellsView cells, int p, zd* __restrict__ moments,
-                                                         double* __restrict__ pows, const double* __restrict__ f,
-                                                         double* __restrict__ fmin_out) {
+                                                         double* __restrict__ pows) {
     extern __shared__ unsigned char smem_raw[];
     const int dim = dimp(p);
     zd* ut = reinterpret_cast<zd*>(smem_raw);  // 8 Υ tables
@@ -949,12 +940,6 @@ __global__ void __launch_bounds__(M2M_EXACT_WIDE) k_m2m_exact_block(const int32_
                 s += w * (v.re * v.re + v.im * v.im);
             }
             pows[(size_t)c * (p + 1) + n] = sqrt(s);
-        }
-        if (f != nullptr && tid == 0) {
-            double mn = INFINITY;
-            for (int o = 0; o < 8; ++o)
-                if (ch[o] >= 0) mn = fmin(mn, fmin_out[ch[o]]);
-            fmin_out[c] = mn;
         }
         __syncthreads();
     }
@@ -1079,6 +1064,41 @@ void launch_fprepass(cudaStream_t s, CellsView cells, const double* x, const dou
     cudaFuncSetAttribute(k_fprepass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_fprepass<<<grid_for((n + 31) / 32, FPRE_WARPS), 32 * FPRE_WARPS, smem, s>>>(cells, x, y, z, m, n, off, nsys,
                                                                                  roots, f, err);
+}
+
+// fmin of every cell (mac.rs:151-173), the smallest f of its bodies: a warp per
+// leaf, then up the tree as in k_geometry_com. arrive: one zero per cell.
+__global__ void __launch_bounds__(128) k_fmin(int nc, CellsView cv, const int32_t* __restrict__ parent,
+                                              const double* __restrict__ f, double* __restrict__ fmin_out,
+                                              unsigned* __restrict__ arrive) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * 4;
+    for (int c0 = blockIdx.x * 4 + (threadIdx.x >> 5); c0 < nc; c0 += warps) {
+        if (!cv.leaf[c0]) continue;
+        int c = c0;
+        const uint32_t fst = cv.first[c], cnt = cv.count[c];
+        double mn = INFINITY;
+        for (uint32_t i = lane; i < cnt; i += 32) mn = fmin(mn, f[fst + i]);
+        for (;;) {
+            for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(FULL, mn, o));
+            if (lane == 0) fmin_out[c] = mn;
+            const int par = parent[c];
+            if (par < 0) break;
+            const int ch = lane < 8 ? cv.child[8 * (size_t)par + lane] : -1;
+            const unsigned have = __ballot_sync(FULL, ch >= 0);
+            unsigned prev = 0;
+            if (lane == 0) {
+                __threadfence();
+                prev = atomicAdd(&arrive[par], 1u);
+            }
+            prev = __shfl_sync(FULL, prev, 0);
+            if (prev + 1 != (unsigned)__popc(have)) break;  // a sibling's warp goes on
+            __threadfence();
+            mn = ch >= 0 ? __ldcg(fmin_out + ch) : INFINITY;
+            c = par;
+        }
+    }
 }
 
 // (centre, rho) of every cell in one 32-byte record for the walk and the near
