@@ -205,7 +205,7 @@ struct fmmx_ctx {
     // mixed form: normalised FP32 half-layout expansions and the per-cell length
     DBuf<zf> mom_f, loc_f;
     DBuf<double> ell;
-    DBuf<unsigned long long> rho_now;  // radii about the build's centres on a reused tree (FP64 bits)
+    DBuf<double> rho_now;  // radii about the build's centres on a reused tree
     DBuf<float> ellf;
 
     // walk: the pool of list chunks, per-cell results, counters (WS_*)
@@ -767,16 +767,11 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         CK(ctx->rho_now.ensure(nc), "alloc expansions");
         CK(ctx->up_arrive.ensure(nc), "alloc expansions");
         if (reuse) {  // the bodies moved since the build: radii about the same centres
-            CK(cudaMemsetAsync(ctx->rho_now.p, 0, (size_t)nc * sizeof(unsigned long long), s), "memset");
-            k_rho_bodies<<<grid_for(n, 256), 256, 0, s>>>(n, ctx->body_leaf.p, cv, ctx->x.p, ctx->y.p, ctx->z.p,
-                                                          ctx->rho_now.p);
-            for (int L = ctx->nlevels - 1; L >= 0; --L) {
-                const int cnt = ctx->lvl_count[L];
-                k_rho_level<<<grid_for(cnt, 256), 256, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt, cv,
-                                                               ctx->rho_now.p);
-            }
-            LCOUNT(1 + ctx->nlevels);
-            rho = reinterpret_cast<const double*>(ctx->rho_now.p);
+            CK(cudaMemsetAsync(ctx->up_arrive.p, 0, (size_t)nc * sizeof(unsigned), s), "memset");
+            k_rho_now<<<grid_for(nc, 4), 128, 0, s>>>(nc, cv, ctx->c_parent.p, ctx->x.p, ctx->y.p, ctx->z.p,
+                                                      ctx->rho_now.p, ctx->up_arrive.p);
+            LCOUNT(1);
+            rho = ctx->rho_now.p;
         }
         k_cell_scale<<<grid_for(nc, 256), 256, 0, s>>>(nc, rho, ctx->c_h.p, ctx->ell.p, ctx->ellf.p);
         LCOUNT(1);

@@ -204,10 +204,8 @@ void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv
 // mixed.cu
 void upload_tables_mixed(const OrderTables& t, cudaStream_t s);
 __global__ void k_cell_scale(int nc, const double* rho, const double* h, double* ell, float* ellf);
-__global__ void k_rho_bodies(size_t n, const int32_t* body_leaf, CellsView cv, const double* x, const double* y,
-                             const double* z, unsigned long long* rho_bits);
-__global__ void k_rho_level(const int32_t* level_cells, int lstart, int lcnt, CellsView cv,
-                            unsigned long long* rho_bits);
+__global__ void k_rho_now(int nc, CellsView cv, const int32_t* parent, const double* x, const double* y,
+                          const double* z, double* rho, unsigned* arrive);
 __global__ void k_moments_to_mixed(int nc, int p, const zd* full, const double* ell, zf* half);
 // top: cells of the top three levels, ntop of them; arrive: nc zeros
 void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, CellsView cv, const int32_t* parent,

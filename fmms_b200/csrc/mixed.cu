@@ -55,6 +55,17 @@ void upload_tables_mixed(const OrderTables& t, cudaStream_t s) {
     cudaStreamSynchronize(s);  // the staging copy dies here
 }
 
+// Touches the tables' lines at once. The recursions read a table row per step;
+// cold, each would wait for the L2 in turn (3 us of a kernel on a small tree).
+template <typename A>
+__device__ __forceinline__ void warm_tables(int p) {
+    for (int i = threadIdx.x; i < 3 * (p + 1); i += blockDim.x) {
+        const int n = i / 3, m = min(8 * (i % 3), FMMX_MAXP);
+        if constexpr (sizeof(A) == 4) asm volatile("" ::"f"(g_tabf.invc[n][m]), "f"(g_tabf.inv2m[m]));
+        else asm volatile("" ::"d"(g_tab.invc[n][m]), "d"(g_tab.inv2m[m]));
+    }
+}
+
 __host__ __device__ constexpr int hx(int n, int m) { return n * (n + 1) / 2 + m; }
 
 __device__ __forceinline__ void split_h(int e, int& n, int& m) {
@@ -84,34 +95,52 @@ __global__ void k_cell_scale(int nc, const double* __restrict__ rho, const doubl
 // reused tree: the bodies have drifted since the build, and a cell whose built
 // radius is tiny (a tight pair) would otherwise normalise its moments by a
 // length far below the bodies' distances from its centre, overflowing FP32
-// (M_n / l^n). Never below the built radius. Leaves from their bodies (an
-// atomic max on the bit pattern, which orders like the value for
-// non-negative doubles), internal cells from their children, deepest level
-// first (the construction of tree.rs:152-227 with the centres held fixed).
-__global__ void k_rho_bodies(size_t n, const int32_t* __restrict__ body_leaf, CellsView cv,
-                             const double* __restrict__ x, const double* __restrict__ y,
-                             const double* __restrict__ z, unsigned long long* __restrict__ rho_bits) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-        const int c = body_leaf[k];
-        const double dx = x[k] - cv.cx[c], dy = y[k] - cv.cy[c], dz = z[k] - cv.cz[c];
-        const double d = sqrt(dx * dx + dy * dy + dz * dz);
-        atomicMax(rho_bits + c, (unsigned long long)__double_as_longlong(d));
-    }
-}
-__global__ void k_rho_level(const int32_t* __restrict__ level_cells, int lstart, int lcnt, CellsView cv,
-                            unsigned long long* __restrict__ rho_bits) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < lcnt; j += gridDim.x * blockDim.x) {
-        const int c = level_cells[lstart + j];
-        double r = fmax(cv.rho[c], __longlong_as_double((long long)rho_bits[c]));
-        if (!cv.leaf[c]) {
-            for (int o = 0; o < 8; ++o) {
-                const int ch = cv.child[8 * c + o];
-                if (ch < 0) continue;
-                const double dx = cv.cx[ch] - cv.cx[c], dy = cv.cy[ch] - cv.cy[c], dz = cv.cz[ch] - cv.cz[c];
-                r = fmax(r, __longlong_as_double((long long)rho_bits[ch]) + sqrt(dx * dx + dy * dy + dz * dz));
+// (M_n / l^n). Never below the built radius. A warp per leaf over its bodies, then
+// up the tree: the warp that finishes a cell's last child goes on with the cell
+// (the construction of tree.rs:152-227 with the centres held fixed). arrive: one
+// zero per cell.
+__global__ void __launch_bounds__(128) k_rho_now(int nc, CellsView cv, const int32_t* __restrict__ parent,
+                                                 const double* __restrict__ x, const double* __restrict__ y,
+                                                 const double* __restrict__ z, double* __restrict__ rho,
+                                                 unsigned* __restrict__ arrive) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * 4;
+    for (int c0 = blockIdx.x * 4 + (threadIdx.x >> 5); c0 < nc; c0 += warps) {
+        if (!cv.leaf[c0]) continue;
+        int c = c0;
+        double r = 0.0;
+        {
+            const double cx = cv.cx[c], cy = cv.cy[c], cz = cv.cz[c];
+            const uint32_t f = cv.first[c], cnt = cv.count[c];
+            for (uint32_t i = lane; i < cnt; i += 32) {
+                const double dx = x[f + i] - cx, dy = y[f + i] - cy, dz = z[f + i] - cz;
+                r = fmax(r, sqrt(dx * dx + dy * dy + dz * dz));
             }
         }
-        rho_bits[c] = (unsigned long long)__double_as_longlong(r);
+        for (;;) {
+            for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(FULL, r, o));
+            r = fmax(cv.rho[c], r);
+            if (lane == 0) rho[c] = r;
+            const int par = parent[c];
+            if (par < 0) break;
+            const int ch = lane < 8 ? cv.child[8 * (size_t)par + lane] : -1;
+            const unsigned have = __ballot_sync(FULL, ch >= 0);
+            unsigned prev = 0;
+            if (lane == 0) {
+                __threadfence();
+                prev = atomicAdd(&arrive[par], 1u);
+            }
+            prev = __shfl_sync(FULL, prev, 0);
+            if (prev + 1 != (unsigned)__popc(have)) break;  // a sibling's warp goes on
+            __threadfence();
+            r = 0.0;
+            if (ch >= 0) {
+                const double dx = cv.cx[ch] - cv.cx[par], dy = cv.cy[ch] - cv.cy[par], dz = cv.cz[ch] - cv.cz[par];
+                r = __ldcg(rho + ch) + sqrt(dx * dx + dy * dy + dz * dz);
+            }
+            c = par;
+        }
     }
 }
 
@@ -151,6 +180,7 @@ __global__ void __launch_bounds__(128) k_p2m_mixed(const int32_t* __restrict__ l
     cplx<A>* sbuf = reinterpret_cast<cplx<A>*>(smem_raw) + (size_t)(threadIdx.x >> 5) * 32 * H;
     cplx<A>* col = sbuf + lane;
     const int wpb = blockDim.x >> 5, warps = gridDim.x * wpb;
+    warm_tables<A>(p);
     for (int j = blockIdx.x * wpb + (threadIdx.x >> 5); j < nc; j += warps) {
         const int c = list ? list[j] : j;
         if (!cv.leaf[c] || (cv.level[c] <= 2) != top) continue;
@@ -247,7 +277,7 @@ __device__ __forceinline__ void ups_column_full(A x, A y, A z, A r2, int p, int 
 // (13,700 at p = 10) take a few hundred instructions a thread. arrive: one zero
 // per cell. (With P2M in the same kernel and a launch per level: N = 1e3, 7
 // levels, 0.15 ms; N = 2^20 uniform 0.70 ms.)
-#define M2M_BLOCK 256
+#define M2M_BLOCK 512
 #define M2M_SCAN 32  // cells a block looks over at a time for its starting points
 template <typename A>
 __device__ __forceinline__ void m2m_cell(int c, const int* __restrict__ ch, CellsView cv,
@@ -278,8 +308,8 @@ __device__ __forceinline__ void m2m_cell(int c, const int* __restrict__ ch, Cell
         if (mm) t[-mm] = (mm & 1) ? mk<float>(-v.x, v.y) : mk<float>(v.x, -v.y);
     }
     __syncthreads();
-    for (int w = tid; w < 8 * H; w += M2M_BLOCK) {
-        const int o = w / H, e = w % H;
+    for (int w = tid; w < 8 * H; w += M2M_BLOCK) {  // the entries of most products first
+        const int o = w & 7, e = H - 1 - (w >> 3);
         A sr = 0, si = 0;
         if (ch[o] >= 0) {
             int n, mm;
@@ -324,6 +354,8 @@ __global__ void __launch_bounds__(M2M_BLOCK) k_m2m_mixed(int nc, CellsView cv, c
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int ch[8], start[M2M_SCAN], nstart, next;
     const int tid = threadIdx.x;
+    warm_tables<float>(p);
+    warm_tables<double>(p);
     for (int b = blockIdx.x * M2M_SCAN; b < nc; b += gridDim.x * M2M_SCAN) {
         if (tid < M2M_SCAN) {  // internal cells without internal children, in order
             const int c = b + tid;
@@ -463,6 +495,7 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
                                                   L2LB_WARPS * F2);  // first item | n << 16
     uint32_t* items = einfo + H + 1;
 
+    warm_tables<A>(p);
     for (int e = threadIdx.x; e < H + 1 + T; e += blockDim.x) einfo[e] = sched[e];
     __syncthreads();
 
@@ -564,6 +597,7 @@ __global__ void k_l2p_mixed(size_t n, const int32_t* __restrict__ body_leaf, con
                             const double* __restrict__ z, const double* __restrict__ nax,
                             const double* __restrict__ nay, const double* __restrict__ naz,
                             const double* __restrict__ npot, double* __restrict__ acc, double* __restrict__ pot) {
+    warm_tables<float>(p);
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         const int c = body_leaf[k];
         const double l = ell[c], il = 1.0 / l;
