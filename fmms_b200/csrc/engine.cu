@@ -70,6 +70,11 @@ struct DBuf : DBufBase {
         cap = 0;
         bud = nullptr;
     }
+    void swap(DBuf& o) {
+        std::swap(p, o.p);
+        std::swap(cap, o.cap);
+        std::swap(bud, o.bud);
+    }
     // Grows by at least half of the current capacity, so a context that sees
     // slowly growing inputs (a serving loop's forests) reallocates -- and
     // cudaFree synchronises the device -- only a logarithmic number of times;
@@ -190,7 +195,6 @@ struct fmmx_ctx {
     DBuf<unsigned> geo_arrive, up_arrive;  // children of a cell whose geometry (moments) are done
     DBuf<unsigned long long> bbox_enc;
     DBuf<uint32_t> sort_sys, sort_sys_alt;  // a forest's second sort (by system)
-    DBuf<ulonglong2> sort_val, sort_val_alt;
 
     // cells (depth-first pre-order)
     DBuf<uint32_t> c_first, c_count;
@@ -406,7 +410,7 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     CK(ctx->keys.ensure(n), "alloc keys");
     CK(ctx->keys_sorted.ensure(n), "alloc keys");
     CK(ctx->idx.ensure(n + 1), "alloc idx");
-    CK(ctx->order.ensure(n), "alloc order");
+    CK(ctx->order.ensure(n + 1), "alloc order");  // (it may change places with idx)
     for (DBuf<double>* b : {&ctx->x, &ctx->y, &ctx->z, &ctx->m, &ctx->nax, &ctx->nay, &ctx->naz, &ctx->npot})
         CK(b->ensure(n), "alloc bodies");
     CK(ctx->box.ensure(8 * (size_t)nsys), "alloc box");
@@ -460,20 +464,24 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
                               nbits, s),
            "key sort");
         if (nsys > 1) {
+            // positions before and after the sort in buffers that are free until the cells are made
             CK(ctx->sort_sys.ensure(n), "alloc sort");
             CK(ctx->sort_sys_alt.ensure(n), "alloc sort");
-            CK(ctx->sort_val.ensure(n), "alloc sort");
-            CK(ctx->sort_val_alt.ensure(n), "alloc sort");
+            CK(ctx->cell_id0.ensure(n + 1), "alloc cells");
+            CK(ctx->body_leaf.ensure(n), "alloc cells");
+            uint32_t* at = reinterpret_cast<uint32_t*>(ctx->body_leaf.p);
             const int sbits = bits_for((uint64_t)(nsys - 1));
             tb = sort_by_system_temp((int)n, sbits);
             CK(ctx->cub_tmp.ensure(tb), "alloc sort");
-            k_pack_by_system<<<grid_for(n, 256), 256, 0, s>>>(ctx->keys_sorted.p, ctx->order.p, n, ctx->sys_off.p, nsys,
-                                                              ctx->sort_sys.p, ctx->sort_val.p);
-            CK(sort_by_system(ctx->cub_tmp.p, tb, ctx->sort_sys.p, ctx->sort_sys_alt.p, ctx->sort_val.p,
-                              ctx->sort_val_alt.p, (int)n, sbits, s),
+            k_entry_system<<<grid_for(n, 256), 256, 0, s>>>(ctx->order.p, n, ctx->sys_off.p, nsys, ctx->sort_sys.p,
+                                                            ctx->cell_id0.p);
+            CK(sort_by_system(ctx->cub_tmp.p, tb, ctx->sort_sys.p, ctx->sort_sys_alt.p, ctx->cell_id0.p, at, (int)n,
+                              sbits, s),
                "key sort");
-            k_unpack_by_system<<<grid_for(n, 256), 256, 0, s>>>(ctx->sort_val_alt.p, n, ctx->keys_sorted.p,
-                                                                ctx->order.p);
+            k_permute_entries<<<grid_for(n, 256), 256, 0, s>>>(at, n, ctx->keys_sorted.p, ctx->order.p, ctx->keys.p,
+                                                               ctx->idx.p);
+            ctx->keys.swap(ctx->keys_sorted);
+            ctx->idx.swap(ctx->order);
             LCOUNT(3);
         }
     }
@@ -567,7 +575,8 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     const uint64_t most = 1ull << 28;
     // chunks per cell at the first attempt (uniform systems take about 40); a context with a budget starts small
     const uint64_t per = ctx->budget.limit || nc < 4096 ? 24 : 44;
-    const uint64_t want = ctx->walk_cap0 > 0 ? std::max<uint64_t>(ctx->walk_cap0 / 32, 1) : per * nc + 256;
+    const uint64_t spare = 16ull * std::min<uint64_t>((uint64_t)nc, 512);  // what the blocks of a small level reserve
+    const uint64_t want = ctx->walk_cap0 > 0 ? std::max<uint64_t>(ctx->walk_cap0 / 32, 1) : per * nc + spare + 256;
     ctx->cap_pool = (uint32_t)std::min(std::max<uint64_t>(ctx->cap_pool, want), most);
     ctx->walk_retries = 0;
     CK(ctx->walk_state.ensure(WS_SIZE), "alloc walk");

@@ -82,9 +82,10 @@ __global__ void k_bbox_seg_final(const unsigned long long* enc, int nsys, double
 #define BBOX_CHUNK 2048  // bodies per block of k_bbox_seg
 __global__ void k_keys_seg(const double* pos, size_t n, const uint64_t* off, int nsys, const double* box,
                            uint64_t* keys, uint32_t* idx);
-__global__ void k_pack_by_system(const uint64_t* keys, const uint32_t* order, size_t n, const uint64_t* off, int nsys,
-                                 uint32_t* sys, ulonglong2* val);
-__global__ void k_unpack_by_system(const ulonglong2* val, size_t n, uint64_t* keys, uint32_t* order);
+__global__ void k_entry_system(const uint32_t* order, size_t n, const uint64_t* off, int nsys, uint32_t* sys,
+                               uint32_t* at);
+__global__ void k_permute_entries(const uint32_t* at, size_t n, const uint64_t* keys_in, const uint32_t* order_in,
+                                  uint64_t* keys, uint32_t* order);
 #define TREE_BLOCK 256
 #define TREE_PER_THREAD 4  // slots per thread of the two tree kernels
 __global__ void k_cell_count(const uint64_t* keys, uint32_t n, const uint64_t* off, int nsys, uint32_t n_leaf,

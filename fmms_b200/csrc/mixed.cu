@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
     uint32_t* items = einfo + H + 1;
 
     warm_tables<A>(p);
+#pragma unroll 8
     for (int e = threadIdx.x; e < H + 1 + T; e += blockDim.x) einfo[e] = sched[e];
     __syncthreads();
 
@@ -518,9 +519,11 @@ __global__ void __launch_bounds__(L2LB_WARPS * 32) k_l2l_mixed(const int32_t* __
         }
         __syncwarp();
         A sr = 0, si = 0;
-        uint32_t it = 0;
+        uint32_t it = 0, ahead = r0 < r1 ? items[r0] : 0u;
+#pragma unroll 4
         for (int i = r0; i < r1; ++i) {
-            it = items[i];
+            it = ahead;
+            if (i + 1 < r1) ahead = items[i + 1];
             const cplx<A> a = U[it & 511u];
             const zf b = F[(it >> 9) & 511u];
             sr += a.re * (A)b.re + a.im * (A)b.im;  // conj(a) * b

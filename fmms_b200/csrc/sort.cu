@@ -21,16 +21,16 @@ cudaError_t sort_pairs_u64_u32(void* tmp, size_t tmp_bytes, const uint64_t* kin,
     return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, end_bit, s);
 }
 
-// Stable sort of 16-byte values by a 32-bit key (a forest's entries by system).
+// Stable sort of positions by a 32-bit key (a forest's entries by system).
 size_t sort_by_system_temp(int n, int end_bit) {
     size_t bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
-                                    (const ulonglong2*)nullptr, (ulonglong2*)nullptr, n, 0, end_bit);
+                                    (const uint32_t*)nullptr, (uint32_t*)nullptr, n, 0, end_bit);
     return bytes;
 }
 
-cudaError_t sort_by_system(void* tmp, size_t tmp_bytes, const uint32_t* kin, uint32_t* kout, const ulonglong2* vin,
-                           ulonglong2* vout, int n, int end_bit, cudaStream_t s) {
+cudaError_t sort_by_system(void* tmp, size_t tmp_bytes, const uint32_t* kin, uint32_t* kout, const uint32_t* vin,
+                           uint32_t* vout, int n, int end_bit, cudaStream_t s) {
     return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, end_bit, s);
 }
 

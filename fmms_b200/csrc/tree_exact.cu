@@ -220,23 +220,23 @@ __global__ void k_gather(const double* __restrict__ pos, const double* __restric
     }
 }
 
-// System of each entry of `order` (sorted by key over the whole forest), for
-// the second, stable sort by system; value: the key and the input index.
-__global__ void k_pack_by_system(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ order, size_t n,
-                                 const uint64_t* __restrict__ off, int nsys, uint32_t* __restrict__ sys,
-                                 ulonglong2* __restrict__ val) {
+// System of each entry of `order` (sorted by key over the whole forest) and its
+// position, for the second, stable sort by system; then keys and order in that
+// sort's order.
+__global__ void k_entry_system(const uint32_t* __restrict__ order, size_t n, const uint64_t* __restrict__ off, int nsys,
+                               uint32_t* __restrict__ sys, uint32_t* __restrict__ at) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t id = order[i];
-        sys[i] = (uint32_t)system_of(off, nsys, id);
-        val[i] = make_ulonglong2(keys[i], id);
+        sys[i] = (uint32_t)system_of(off, nsys, order[i]);
+        at[i] = (uint32_t)i;
     }
 }
-__global__ void k_unpack_by_system(const ulonglong2* __restrict__ val, size_t n, uint64_t* __restrict__ keys,
-                                   uint32_t* __restrict__ order) {
+__global__ void k_permute_entries(const uint32_t* __restrict__ at, size_t n, const uint64_t* __restrict__ keys_in,
+                                  const uint32_t* __restrict__ order_in, uint64_t* __restrict__ keys,
+                                  uint32_t* __restrict__ order) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const ulonglong2 v = val[i];
-        keys[i] = v.x;
-        order[i] = (uint32_t)v.y;
+        const uint32_t q = at[i];
+        keys[i] = keys_in[q];
+        order[i] = order_in[q];
     }
 }
 

@@ -270,16 +270,18 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
     uint32_t res_next = 0, res_end = 0;  // reserved chunks
     unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0;  // thread sums (n*: thread 0)
     int par_w = 0;  // parity of the step's wsum slots
-    for (;;) {
-        int j = 0;
-        if (W == 1) {
-            if (lane == 0) j = atomicAdd(work, 1);
-            j = __shfl_sync(FULL, j, 0);
-        } else {
-            __syncthreads();
-            if (tid == 0) bcast[1] = (uint32_t)atomicAdd(work, 1);
-            __syncthreads();
-            j = (int)bcast[1];
+    for (int round = 0;; ++round) {
+        int j = blockIdx.x;  // the block's first cell; from then on the next one that no block has
+        if (round > 0) {
+            if (W == 1) {
+                if (lane == 0) j = (int)gridDim.x + atomicAdd(work, 1);
+                j = __shfl_sync(FULL, j, 0);
+            } else {
+                __syncthreads();
+                if (tid == 0) bcast[1] = gridDim.x + (uint32_t)atomicAdd(work, 1);
+                __syncthreads();
+                j = (int)bcast[1];
+            }
         }
         if (j >= ncell) break;
         const int c = cells[j];
@@ -569,12 +571,12 @@ static void launch_form(unsigned most, cudaStream_t s, const int32_t* level_cell
     auto kern = k_walk_level<DEHNEN, W, RING>;
     constexpr size_t smem = (size_t)RING * sizeof(uint32_t);
     unsigned grid = most;
-    uint32_t batch = W == 32 ? 16u : 6u;  // chunks reserved per atomic: a small level wants little waste
+    uint32_t batch = W == 1 ? 6u : 16u;  // chunks reserved per atomic: a small level wants little waste
     if (RING) {
+        if (smem > 48 * 1024)  // (per device, so at every launch)
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         static std::atomic<int> per_sm{0};
         if (per_sm.load() == 0) {
-            if (smem > 48 * 1024)
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             int b = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 32 * W, smem) != cudaSuccess || b < 1) b = 1;
             per_sm.store(b);
