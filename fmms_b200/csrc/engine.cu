@@ -1,14 +1,13 @@
 // Host orchestration of the engine behind the C ABI (include/fmmx.h).
 //
 // fmmx_build   = Fmm::new / refresh (fmm.rs:26-56): bounding box, Morton keys,
-//                key sort, level-by-level node creation, depth-first
-//                renumbering, body gather, cell geometry.
+//                key sort, body gather, cells, cell geometry.
 // fmmx_evaluate = Fmm::run (fmm.rs:60-142): gather, f pre-pass, P2M/M2M and
-//                multipole power, dual walk, directed lists, M2L, L2L, P2P,
+//                multipole power, dual walk with the lists, M2L, L2L, P2P,
 //                L2P + scatter.
 //
-// All work runs on one stream; the host waits on it only where a size must be
-// known (node count after the build, list lengths after the walk).
+// Work runs on two streams; the host waits only where a size must be known
+// (the cells of a tree, the lists after the walk) and at the end of a build or evaluation.
 #include <cuda_runtime.h>
 
 #include <algorithm>

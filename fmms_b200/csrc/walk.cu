@@ -17,8 +17,8 @@
 // alone: no list has to be sorted or scattered. (The walk used to append mutual
 // pairs with atomics, a frontier at a time, and a counting sort and segment sorts
 // made the lists. Walk and lists alone on the device: N = 2^22, 64 clusters,
-// 14.4 + 47 -> 22.5 + 2.5 ms; uniform 2^20 0.41 + 0.99 -> 0.48 + 0.07; 10^3
-// bodies 0.145 + 0.22 -> 0.14 + 0.01.)
+// 14.4 + 47 -> 21.1 + 2.5 ms; uniform 2^20 0.41 + 0.99 -> 0.44 + 0.07; 10^3
+// bodies 0.145 + 0.22 -> 0.13 + 0.01.)
 //
 // The sources of a cell are taken in blocks of WK_BLOCK inherited entries; of a
 // block first in, first out: its entries, then the children of those that split
