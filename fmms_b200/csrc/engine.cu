@@ -661,7 +661,9 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     CK(ctx->p2p_part.ensure(std::max<size_t>(sizes.w, 1)), "alloc p2p scratch");
     CK(ctx->p2p_next.ensure(1), "alloc lists");
     if (ctx->events) CK(cudaEventRecord(ctx->ev[4], s), "event");
-    launch_lists_gather(s, nc, (uint32_t)hs[WS_USED], pool, lists, ctx->list_off.p, ctx->m2l_off.p, ctx->p2p_off.p, ctx->p2p_uoff.p,
+    // chunks reserved but not used may lie beyond the pool: no entry is there
+    const uint32_t nchunks = std::min((uint32_t)hs[WS_USED], pool.cap);
+    launch_lists_gather(s, nc, nchunks, pool, lists, ctx->list_off.p, ctx->m2l_off.p, ctx->p2p_off.p, ctx->p2p_uoff.p,
                         ctx->p2p_soff.p, ctx->m2l_src.p, ctx->p2p_src.p, ctx->p2p_ucell.p);
     CKL("lists");
     LCOUNT(1);

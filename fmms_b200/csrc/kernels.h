@@ -41,7 +41,8 @@ struct WalkPool {
     uint32_t* next;   // cap: the following chunk of a list passed down
     uint2* owner;     // cap: whose entries the chunk of an M2L or P2P list holds (all bits set: nobody's)
     uint32_t cap;     // chunks
-    unsigned* used;   // chunks reserved (beyond cap after an overflow)
+    unsigned* used;   // chunks reserved; above cap after an overflow, but also where only the unused tails of the
+                      // last reservations (up to 16 chunks per block) lie beyond the pool
     int* overflow;    // set when a chunk was refused: the lists are incomplete
 };
 
@@ -135,7 +136,7 @@ int launch_walk_level(bool dehnen, cudaStream_t s, const int32_t* level_cells, i
                       int* work, int* heavy_work);
 bool walk_needs_heavy(const int* lvl_count, int nlevels, int nleaves);
 unsigned walk_heavy_blocks(int nleaves);
-// contiguous lists from the chunks; off: the exclusive sums of W.sizes
+// contiguous lists from the first nchunks chunks (at most P.cap); off: the exclusive sums of W.sizes
 void launch_lists_gather(cudaStream_t s, int nc, uint32_t nchunks, WalkPool P, WalkLists W, const uint4* off, uint32_t* m2l_off,
                          uint32_t* p2p_off, uint32_t* uoff, uint32_t* soff, uint32_t* m2l, uint32_t* p2p,
                          int32_t* ucell);

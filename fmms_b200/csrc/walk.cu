@@ -527,7 +527,7 @@ __global__ void k_lists_gather(int nc, uint32_t nchunks, WalkPool P, WalkLists L
         // lane: one chunk's place and entries
         const uint32_t id = 32 * b + lane;
         uint32_t dst = 0, n = 0, kind = 0;
-        if (id < nchunks) {
+        if (id < nchunks && id < P.cap) {  // (the unused tail of a reservation may lie beyond the pool)
             const uint2 w = P.owner[id];
             if (w.x != ~0u) {
                 const uint32_t idx = w.y & 0x1fffffffu;

@@ -78,6 +78,42 @@ def test_walk_overflow_retry_gives_the_same_bits(monkeypatch):
         assert g.stats()["n_m2l"] == ref.stats()["n_m2l"] and g.stats()["n_p2p"] == ref.stats()["n_p2p"]
 
 
+@pytest.mark.parametrize("n,n_leaf,dense", [(1500, 8, False), (30_000, 4, True)])
+def test_walk_capacity_between_used_and_reserved(monkeypatch, n, n_leaf, dense):
+    """A block reserves several chunks at a time (6 or 16), so a pool may hold
+    every chunk that is used while the tails of the last reservations lie beyond
+    it: no overflow, and the lists are copied from inside the pool alone. Every
+    capacity around the smallest one without a retry gives the same bits."""
+    mass, pos, _ = fx().gen_plummer_ic(n, 1.0, 1.0, 20.0, 8)
+    if dense:  # many cells per level: a warp each, thousands of reservations
+        pos = np.concatenate([pos, pos[: n // 4] * 1e-3])
+        mass = np.concatenate([mass, mass[: n // 4]])
+    kw = dict(mac="theta", theta=0.5, softening=1e-3)
+    ref = fx().Fmm(mass, pos, 2, 0.0, n_leaf, **kw)
+    r0 = ref.run()
+    lists0 = ref.export_lists()
+
+    def with_chunks(chunks):
+        monkeypatch.setenv("FMMX_TEST_WALK_CAPACITY", str(32 * chunks))
+        g = fx().Fmm(mass, pos, 2, 0.0, n_leaf, **kw)
+        monkeypatch.delenv("FMMX_TEST_WALK_CAPACITY")
+        return g, g.run()
+
+    lo, hi = 1, 1 << 20  # retries at lo, none at hi
+    assert with_chunks(lo)[0].stats()["walk_retries"] > 0
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        if with_chunks(mid)[0].stats()["walk_retries"]:
+            lo = mid
+        else:
+            hi = mid
+    for chunks in list(range(max(hi - 6, 1), hi + 20)) + [hi + 100, 2 * hi]:
+        g, r = with_chunks(chunks)
+        assert np.array_equal(r.accel, r0.accel) and np.array_equal(r.pot, r0.pot), chunks
+        for a, b in zip(g.export_lists(), lists0):
+            assert np.array_equal(a, b), chunks
+
+
 def test_corrupted_ensemble_offsets():
     m1, p1 = fx().gen_plummer(3000, seed=1)
     m2, p2 = fx().gen_plummer(2000, seed=2)
