@@ -138,7 +138,7 @@ enum { TF_BAD = 0, TF_STACK = 1, TF_LEVELS = 2, TF_CURSOR = TF_LEVELS + FMMX_NLE
        TF_SIZE = TF_CURSOR + FMMX_NLEVELS };
 // 64-bit words of the walk's state: chunks used, overflow flag, totals (WalkLists), and per level the work
 // counters of the level and of its heavy cells and the number of those
-enum { WS_USED = 0, WS_OVERFLOW = 1, WS_TOTALS = 2, WS_WORK = 6, WS_HWORK = WS_WORK + FMMX_NLEVELS,
+enum { WS_USED = 0, WS_OVERFLOW = 1, WS_TOTALS = 2, WS_WORK = WS_TOTALS + 6, WS_HWORK = WS_WORK + FMMX_NLEVELS,
        WS_HEAVY = WS_HWORK + FMMX_NLEVELS, WS_SIZE = WS_HEAVY + FMMX_NLEVELS };
 
 }  // namespace
@@ -222,6 +222,7 @@ struct fmmx_ctx {
     DBuf<int32_t> heavy_list;
     DBuf<uint32_t> heavy_ring;
     uint64_t walk_cap0 = 0;  // FMMX_TEST_WALK_CAPACITY (entries; tests of the overflow retry); 0: sized by the tree
+    uint64_t p2p_parts_max = 0xffffffffull;  // partial sums (FMMX_TEST_P2P_PARTIALS: a smaller bound, for tests)
     int walk_retries = 0;
 
     // directed lists: per destination cell c the sources src[off[c] .. off[c+1])
@@ -230,7 +231,7 @@ struct fmmx_ctx {
     // near-field work units (per leaf: first unit, first partial sum)
     DBuf<uint32_t> p2p_uoff, p2p_soff;
     DBuf<int32_t> p2p_ucell;
-    uint32_t p2p_nunits = 0;
+    uint32_t p2p_nunits = 0, p2p_grain = P2P_GRAIN;
     DBuf<double4> p2p_part;
     DBuf<float4> body_pairs;  // mixed near field: bodies relative to their leaf's centre, FP32, with the mass, in pairs
     DBuf<unsigned> p2p_next;
@@ -610,7 +611,6 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
         heavy.ring = ctx->heavy_ring.p;
     }
     unsigned long long hs[WS_SIZE];
-    uint4 sizes;
     WalkPool pool;
     const WalkLists lists{ctx->down_n.p, ctx->down_head.p, ctx->list_redone.p, ctx->list_sizes.p,
                           ctx->walk_state.p + WS_TOTALS};
@@ -636,7 +636,6 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
         LCOUNT(2);
         int stack_overflow = 0;
         CK(cudaMemcpyAsync(hs, ctx->walk_state.p, sizeof(hs), cudaMemcpyDeviceToHost, s), "copy");
-        CK(cudaMemcpyAsync(&sizes, ctx->list_off.p + nc, sizeof(sizes), cudaMemcpyDeviceToHost, s), "copy");
         if (dehnen)
             CK(cudaMemcpyAsync(&stack_overflow, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
         CK(cudaStreamSynchronize(s), "walk");
@@ -654,12 +653,35 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     ctx->p2p_inter = hs[WS_TOTALS + 1];
     ctx->n_m2l = (int)(dm / 2);
     ctx->n_p2p = (int)((dp + (uint64_t)ctx->nleaves) / 2);  // a leaf's self pair is one entry
-    ctx->p2p_nunits = sizes.z;
     CK(ctx->m2l_src.ensure(std::max<size_t>(dm, 1)), "alloc lists");
     CK(ctx->p2p_src.ensure(std::max<size_t>(dp, 1)), "alloc lists");
-    CK(ctx->p2p_ucell.ensure(std::max<size_t>(sizes.z, 1)), "alloc lists");
-    CK(ctx->p2p_part.ensure(std::max<size_t>(sizes.w, 1)), "alloc p2p scratch");
     CK(ctx->p2p_next.ensure(1), "alloc lists");
+    // the near field's units and partial sums, coarser where they are too many for the 32-bit sums or the memory
+    uint64_t units = hs[WS_TOTALS + 4], parts = hs[WS_TOTALS + 5];
+    for (uint32_t grain = P2P_GRAIN;;) {
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (units <= 0x7fffffffull && parts <= ctx->p2p_parts_max) {
+            e = ctx->p2p_ucell.ensure(std::max<size_t>(units, 1));
+            if (e == cudaSuccess) e = ctx->p2p_part.ensure(std::max<size_t>(parts, 1));
+        }
+        ctx->p2p_grain = grain;
+        ctx->p2p_nunits = (uint32_t)units;
+        if (e == cudaSuccess) break;
+        if (grain == P2P_WHOLE || e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "alloc p2p scratch");
+        ctx->budget.over = false;
+        grain = grain < (1u << 20) ? 8 * grain : P2P_WHOLE;
+        unsigned long long* t = lists.totals + 4;
+        CK(cudaMemsetAsync(t, 0, 2 * sizeof(*t), s), "memset");
+        launch_near_sizes(s, nc, ctx->c_count.p, grain, lists);
+        CKL("list offsets");
+        CK(scan_u32x4(ctx->cub_tmp.p, ctx->cub_tmp.cap, ctx->list_sizes.p, ctx->list_off.p, nc + 1, s), "list offsets");
+        LCOUNT(2);
+        unsigned long long ht[2];
+        CK(cudaMemcpyAsync(ht, t, sizeof(ht), cudaMemcpyDeviceToHost, s), "copy");
+        CK(cudaStreamSynchronize(s), "list offsets");
+        units = ht[0];
+        parts = ht[1];
+    }
     if (ctx->events) CK(cudaEventRecord(ctx->ev[4], s), "event");
     // chunks reserved but not used may lie beyond the pool: no entry is there
     const uint32_t nchunks = std::min((uint32_t)hs[WS_USED], pool.cap);
@@ -673,7 +695,7 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
 // the near field's work units, as walk_impl left them
 P2pUnits near_units(fmmx_ctx* ctx) {
     return P2pUnits{ctx->p2p_uoff.p, ctx->p2p_ucell.p, ctx->p2p_soff.p, ctx->p2p_part.p, ctx->p2p_next.p,
-                    ctx->p2p_nunits};
+                    ctx->p2p_nunits, ctx->p2p_grain};
 }
 
 // Mixed form, near field: FP32 + double-single P2P on the second stream.
@@ -1018,6 +1040,8 @@ fmmx_status fmmx_create(const fmmx_config* cfg, fmmx_ctx** out) {
     ctx->budget.limit = c.device_budget_bytes;
     BudgetScope bscope(&ctx->budget);
     if (const char* wc = std::getenv("FMMX_TEST_WALK_CAPACITY")) ctx->walk_cap0 = std::strtoull(wc, nullptr, 10);
+    if (const char* pm = std::getenv("FMMX_TEST_P2P_PARTIALS"))
+        ctx->p2p_parts_max = std::min<uint64_t>(std::strtoull(pm, nullptr, 10), ctx->p2p_parts_max);
     std::memset(&ctx->st, 0, sizeof(ctx->st));
     if (c.stream) {
         ctx->stream = (cudaStream_t)c.stream;

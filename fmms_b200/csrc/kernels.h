@@ -55,7 +55,8 @@ struct WalkLists {
     uint32_t* down_head;
     uint8_t* redone;
     uint4* sizes;                // ncells + 1
-    unsigned long long* totals;  // pairs examined, body interactions, directed M2L and P2P entries
+    // pairs examined, body interactions, directed M2L and P2P entries, near-field work units and partial sums
+    unsigned long long* totals;
 };
 
 // Segmented directed interaction list: for destination cell c, sources
@@ -175,28 +176,48 @@ struct P2pUnits {
     const uint32_t* soff;  // ncells + 1
     double4* part;
     unsigned* next;  // work counter, zero at launch
-    uint32_t nunits;
+    uint32_t nunits;  // below 2^31: the counter passes it by one per warp
+    uint32_t grain;   // see p2p_shares
 };
 
 // Work units of the near field, a warp each: up to P2P_NT targets of a leaf
-// against an equal share of its source leaves, p2p_shares(targets, sources) of
-// them. The share depends on the leaf alone -- about the same work per unit,
-// 2048 target-source-leaf products -- so a leaf in a dense core with thousands
+// against an equal share of its source leaves, p2p_shares(targets, sources, grain)
+// of them. The share depends on the leaf alone -- about the same work per unit,
+// `grain` target-source-leaf products -- so a leaf in a dense core with thousands
 // of neighbours, or one of few leaves of a small system, spreads over many warps
 // (the load-balancing aim of the reference's split_fat, crates/visual/src/
 // gpufmm.rs:1350-1414). A leaf with one share writes its bodies' sums directly;
 // the shares of the others write partial sums, which k_p2p_combine adds per
 // body in share order (a fixed order: the results do not depend on which warp
-// ran which unit).
-__host__ __device__ __forceinline__ uint32_t p2p_shares(uint32_t nt, uint32_t len) {
+// ran which unit). The grain is P2P_GRAIN unless the partial sums (32 bytes for
+// every body and share of a split leaf; leaves of 250 bodies with 10^3 sources each:
+// 600 bytes a body) are more than 2^32 - 1 or than the memory holds; the walk
+// then takes a coarser one, in the end P2P_WHOLE: one share a leaf, no partial sums.
+#define P2P_GRAIN 2048u
+#define P2P_WHOLE 0xffffffffu
+__host__ __device__ __forceinline__ uint32_t p2p_shares(uint32_t nt, uint32_t len, uint32_t grain) {
+    if (grain == P2P_WHOLE) return len ? 1u : 0u;
     const uint32_t t = nt < P2P_NT ? nt : P2P_NT;
-    uint32_t per = 2048u / (t > 0 ? t : 1u);
-    per = per > 512u ? 512u : per;
+    uint32_t per = grain / (t > 0 ? t : 1u);
+    per = per > grain / 4 ? grain / 4 : per;
     uint32_t s = (len + per - 1) / per;
     const uint32_t most = (1u << 22) / (nt > 0 ? nt : 1u) + 1u;  // bounds the partial sums of a very large leaf
     return s < most ? s : most;
 }
 
+// a cell's list sizes with its near-field units and partial sums
+__host__ __device__ __forceinline__ uint4 near_sizes(uint32_t m2l, uint32_t p2p, uint32_t count, uint32_t grain) {
+    const uint32_t sh = p2p ? p2p_shares(count, p2p, grain) : 0u;
+    uint4 v;
+    v.x = m2l;
+    v.y = p2p;
+    v.z = sh * ((count + P2P_NT - 1) / P2P_NT);
+    v.w = sh > 1 ? sh * count : 0u;
+    return v;
+}
+// units and partial sums of the leaves for another grain: sizes[c].z, .w and their sums totals[4], [5]
+// (both zero before)
+void launch_near_sizes(cudaStream_t s, int ncells, const uint32_t* count, uint32_t grain, WalkLists Ls);
 void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,
                         double* az, double* pot);
 void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const double* x,

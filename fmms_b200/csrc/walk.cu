@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
     const int ncell = RING ? lcnt : min((int)*heavy.count, lcnt);
     const int32_t* cells = RING ? level_cells : heavy.list;
     uint32_t res_next = 0, res_end = 0;  // reserved chunks
-    unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0;  // thread sums (n*: thread 0)
+    unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0, nunits = 0, nparts = 0;  // thread sums (n*: thread 0)
     int par_w = 0;  // parity of the step's wsum slots
     for (int round = 0;; ++round) {
         int j = blockIdx.x;  // the block's first cell; from then on the next one that no block has
@@ -485,8 +485,10 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
             Ls.down_n[c] = ld.n;
             Ls.down_head[c] = ld.head;
             Ls.redone[c] = RING ? 0 : 1;
-            const uint32_t sh = lp.n ? p2p_shares(tn, lp.n) : 0u;
-            Ls.sizes[c] = make_uint4(lm.n, lp.n, sh * ((tn + P2P_NT - 1) / P2P_NT), sh > 1 ? sh * tn : 0u);
+            const uint4 sz = near_sizes(lm.n, lp.n, tn, P2P_GRAIN);
+            nunits += sz.z;
+            nparts += sz.w;
+            Ls.sizes[c] = sz;
         }
     }
 #pragma unroll
@@ -499,6 +501,8 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
         if (inter) atomicAdd(Ls.totals + 1, inter);
         if (nm2l) atomicAdd(Ls.totals + 2, nm2l);
         if (np2p) atomicAdd(Ls.totals + 3, np2p);
+        if (nunits) atomicAdd(Ls.totals + 4, nunits);
+        if (nparts) atomicAdd(Ls.totals + 5, nparts);
     }
 }
 

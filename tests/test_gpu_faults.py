@@ -114,6 +114,44 @@ def test_walk_capacity_between_used_and_reserved(monkeypatch, n, n_leaf, dense):
             assert np.array_equal(a, b), chunks
 
 
+@pytest.mark.parametrize("precision", ["plain", "mixed"])
+def test_near_field_partial_sums_bounded(monkeypatch, precision):
+    """Leaves of 250 bodies with long lists have many partial sums. Where they
+    are more than the 32-bit sums address (here: than a small bound,
+    FMMX_TEST_P2P_PARTIALS) the shares are coarser, in the end one per leaf with
+    no partial sums. Only the grouping of a body's sum changes: 100,000 terms in
+    FP64 (plain, about 1e-16 each), or in FP32 groups of some 64 pairs (mixed)."""
+    mass, pos = fx().gen_plummer(20_000, seed=8)
+    kw = dict(mac="theta", theta=0.2, softening=1e-3, precision=precision)
+    r0 = fx().Fmm(mass, pos, 2, 0.0, 256, **kw).run()
+    rel = 1e-13 if precision == "plain" else 1e-6
+    for bound in (5000, 0):
+        monkeypatch.setenv("FMMX_TEST_P2P_PARTIALS", str(bound))
+        g = fx().Fmm(mass, pos, 2, 0.0, 256, **kw)
+        monkeypatch.delenv("FMMX_TEST_P2P_PARTIALS")
+        r1 = g.run()
+        r2 = g.run()  # the lists of the second evaluation, in the buffers of the first
+        assert np.array_equal(r1.accel, r2.accel)
+        for a, b in ((r1.accel, r0.accel), (r1.pot, r0.pot)):
+            assert np.linalg.norm(a - b) <= rel * np.linalg.norm(b)
+            assert not np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision,mib", [("plain", 77), ("mixed", 86)])
+def test_budget_of_large_leaves(precision, mib):
+    """100,000 bodies in leaves of up to 256 with lists of 10^3 leaves: 64 MB of
+    partial sums that the budget does not hold; the shares are coarser instead."""
+    mass, pos = fx().gen_plummer(100_000, seed=7)
+    kw = dict(mac="theta", theta=0.2, precision=precision)
+    r0 = fx().Fmm(mass, pos, 2, 0.0, 256, **kw).run()
+    g = fx().Fmm(None, None, 2, 0.0, 256, device_budget_bytes=mib * 1_000_000, **kw)
+    g.refresh(mass, pos)
+    r1 = g.run()
+    assert g.stats()["device_bytes"] <= mib * 1_000_000
+    rel = 1e-13 if precision == "plain" else 1e-6
+    assert np.linalg.norm(r1.accel - r0.accel) <= rel * np.linalg.norm(r0.accel)
+
+
 def test_corrupted_ensemble_offsets():
     m1, p1 = fx().gen_plummer(3000, seed=1)
     m2, p2 = fx().gen_plummer(2000, seed=2)
