@@ -570,8 +570,8 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
 // back once in between; returns with the lists queued.
 fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     const int nc = ctx->nc;
-    // the pool's capacity follows the current tree (a context may see trees of
-    // very different sizes, e.g. the forests of a serving loop) and grows on overflow
+    // the pool: at least what the current tree is expected to take, more after
+    // an overflow, never less than it has had; no walk's work grows with it
     const uint64_t most = 1ull << 28;
     // chunks per cell at the first attempt (uniform systems take about 40); a context with a budget starts small
     const uint64_t per = ctx->budget.limit || nc < 4096 ? 24 : 44;
@@ -618,7 +618,6 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
         CK(ctx->pool_entry.ensure(32 * (size_t)ctx->cap_pool), "alloc walk");
         CK(ctx->pool_next.ensure(ctx->cap_pool), "alloc walk");
         CK(ctx->pool_owner.ensure(ctx->cap_pool), "alloc walk");
-        CK(cudaMemsetAsync(ctx->pool_owner.p, 0xff, (size_t)ctx->cap_pool * sizeof(uint2), s), "memset");
         pool = WalkPool{ctx->pool_entry.p, ctx->pool_next.p, ctx->pool_owner.p, ctx->cap_pool,
                         reinterpret_cast<unsigned*>(ctx->walk_state.p + WS_USED),
                         reinterpret_cast<int*>(ctx->walk_state.p + WS_OVERFLOW)};

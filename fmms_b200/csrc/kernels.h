@@ -39,7 +39,8 @@ struct MacParams {
 struct WalkPool {
     uint32_t* entry;  // 32 cap
     uint32_t* next;   // cap: the following chunk of a list passed down
-    uint2* owner;     // cap: whose entries the chunk of an M2L or P2P list holds (all bits set: nobody's)
+    uint2* owner;     // cap: whose entries the chunk of an M2L or P2P list holds (x: all bits set, nobody's); set by the
+                      // walk for every chunk reserved, so nothing is cleared before it
     uint32_t cap;     // chunks
     unsigned* used;   // chunks reserved; above cap after an overflow, but also where only the unused tails of the
                       // last reservations (up to 16 chunks per block) lie beyond the pool

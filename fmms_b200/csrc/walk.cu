@@ -213,7 +213,8 @@ __device__ __forceinline__ void list_add(const WalkPool& P, ListTail& t, uint32_
             if (kind == 2u && t.last < P.cap) P.next[t.last] = base;
             for (uint32_t k = 0; k < q && base + k < P.cap; ++k) {
                 if (kind == 2u) P.next[base + k] = base + k + 1;
-                else P.owner[base + k] = make_uint2(cell, kind << 30 | redone << 29 | (((t.n + 31) >> 5) + k));
+                P.owner[base + k] = kind == 2u ? make_uint2(~0u, 0u)
+                                               : make_uint2(cell, kind << 30 | redone << 29 | (((t.n + 31) >> 5) + k));
             }
         }
         if (t.head == ~0u) t.head = base;
@@ -269,6 +270,11 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
     const int32_t* cells = RING ? level_cells : heavy.list;
     uint32_t res_next = 0, res_end = 0;  // reserved chunks
     unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0, nunits = 0, nparts = 0;  // thread sums (n*: thread 0)
+    // the unused rest of the reservation (fewer than `batch` chunks): nobody's
+    auto give_back = [&]() {
+        const uint32_t id = res_next + (uint32_t)tid;
+        if (id < res_end && id < P.cap) P.owner[id] = make_uint2(~0u, 0u);
+    };
     int par_w = 0;  // parity of the step's wsum slots
     for (int round = 0;; ++round) {
         int j = blockIdx.x;  // the block's first cell; from then on the next one that no block has
@@ -295,8 +301,10 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
         unsigned long long cinter = 0;
         bool given_up = false;
         // q chunks in a row: from the group's reservation (every thread tracks it), refilled `batch` at a time
+        // (what is left of the old one then belongs to nobody)
         auto reserve = [&](uint32_t q) -> uint32_t {
             if (q > res_end - res_next) {
+                give_back();
                 const uint32_t take = q > batch ? q : batch;
                 uint32_t b = 0;
                 if (tid == 0) b = atomicAdd(P.used, take);
@@ -491,6 +499,7 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
             Ls.sizes[c] = sz;
         }
     }
+    give_back();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         pops += __shfl_xor_sync(FULL, pops, o);

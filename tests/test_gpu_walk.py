@@ -62,3 +62,29 @@ def test_results_do_not_depend_on_the_form():
             h = fx.Fmm(parts[s][0], parts[s][1], 4, 0.0, 4, **kw).run()
             a, b = int(off[s]), int(off[s + 1])
             assert np.array_equal(r.accel[a:b], h.accel) and np.array_equal(r.pot[a:b], h.pot)
+
+
+def test_walk_time_does_not_grow_with_what_the_context_held():
+    """A context that has evaluated a million bodies in small leaves (a pool of
+    gigabytes) walks a small system in the time a new one does: nothing of the
+    pool's size is cleared or read."""
+    import fmms_b200 as fx
+
+    mass, pos = fx.gen_plummer(1000, seed=2)
+    kw = dict(mac="theta", theta=0.9, softening=1e-3)
+
+    def walk_ms(g):
+        g.refresh(mass, pos)
+        t = []
+        for _ in range(60):
+            r = g.run()
+            t.append(g.stats()["ms_walk"])
+        return min(t), r.accel
+
+    big_m, big_p = fx.gen_plummer(1 << 20, seed=3)
+    used = fx.Fmm(big_m, big_p, 1, 0.0, 4, **kw)
+    used.run()
+    t1, a1 = walk_ms(used)
+    t0, a0 = walk_ms(fx.Fmm(None, None, 1, 0.0, 4, **kw))
+    assert np.array_equal(a0, a1)
+    assert t1 < 1.12 * t0, (t0, t1)
