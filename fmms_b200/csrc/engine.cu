@@ -218,6 +218,7 @@ struct fmmx_ctx {
     DBuf<uint4> list_sizes, list_off;
     DBuf<unsigned long long> walk_state;
     uint32_t cap_pool = 0;   // chunks
+    bool pool_short = false; // the memory did not hold the expected capacity
     DBuf<double2> mac_rows;  // per cell for Dehnen's MAC
     DBuf<int32_t> heavy_list;
     DBuf<uint32_t> heavy_ring;
@@ -282,6 +283,7 @@ fmmx_status finish(fmmx_ctx* ctx, fmmx_status st) {
     for (DBufBase* b : ctx->cache) b->release();
     ctx->built = ctx->evaluated = ctx->lists_valid = false;
     ctx->cap_pool = 0;
+    ctx->pool_short = false;
     return st;
 }
 
@@ -566,6 +568,25 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
 }
 
 // ---------------------------------------------------------------- evaluate
+// Room for `want` list chunks or, where the memory or the budget does not hold
+// them, for as many as it holds, more than `least` (which were too few).
+cudaError_t pool_room(fmmx_ctx* ctx, uint64_t least, uint64_t want) {
+    for (;;) {
+        cudaError_t e = ctx->pool_entry.ensure(32 * (size_t)want);
+        if (e == cudaSuccess) e = ctx->pool_next.ensure(want);
+        if (e == cudaSuccess) e = ctx->pool_owner.ensure(want);
+        if (e == cudaSuccess) ctx->cap_pool = (uint32_t)want;
+        const uint64_t next = least + (want - least) / 2;
+        if (e != cudaErrorMemoryAllocation || next <= least + least / 32) return e;
+        ctx->budget.over = false;
+        ctx->pool_entry.release();
+        ctx->pool_next.release();
+        ctx->pool_owner.release();
+        ctx->pool_short = true;
+        want = next;
+    }
+}
+
 // The walk and the interaction lists on stream s, with the lists' sizes read
 // back once in between; returns with the lists queued.
 fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
@@ -577,7 +598,8 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     const uint64_t per = ctx->budget.limit || nc < 4096 ? 24 : 44;
     const uint64_t spare = 16ull * std::min<uint64_t>((uint64_t)nc, 512);  // what the blocks of a small level reserve
     const uint64_t want = ctx->walk_cap0 > 0 ? std::max<uint64_t>(ctx->walk_cap0 / 32, 1) : per * nc + spare + 256;
-    ctx->cap_pool = (uint32_t)std::min(std::max<uint64_t>(ctx->cap_pool, want), most);
+    uint64_t cap = std::min(std::max<uint64_t>(ctx->cap_pool, want), most), least = 0;
+    if (ctx->pool_short && ctx->cap_pool > 0) cap = ctx->cap_pool;  // (what an earlier walk ended with)
     ctx->walk_retries = 0;
     CK(ctx->walk_state.ensure(WS_SIZE), "alloc walk");
     CK(ctx->down_n.ensure(nc), "alloc walk");
@@ -606,18 +628,23 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     if (walk_needs_heavy(ctx->lvl_count, ctx->nlevels, ctx->nleaves)) {
         heavy.blocks = walk_heavy_blocks(ctx->nleaves);
         CK(ctx->heavy_list.ensure(nc), "alloc walk");
-        CK(ctx->heavy_ring.ensure((size_t)heavy.blocks * (size_t)ctx->nleaves), "alloc walk");
+        for (;;) {  // fewer queues where the memory does not hold them
+            const cudaError_t e = ctx->heavy_ring.ensure((size_t)heavy.blocks * (size_t)ctx->nleaves);
+            if (e == cudaSuccess) break;
+            if (e != cudaErrorMemoryAllocation || heavy.blocks == 1) return cuda_fail(ctx, e, "alloc walk");
+            ctx->budget.over = false;
+            heavy.blocks = (heavy.blocks + 1) / 2;
+        }
         heavy.list = ctx->heavy_list.p;
         heavy.ring = ctx->heavy_ring.p;
     }
     unsigned long long hs[WS_SIZE];
+    uint64_t dm = 0, dp = 0;  // directed entries
     WalkPool pool;
     const WalkLists lists{ctx->down_n.p, ctx->down_head.p, ctx->list_redone.p, ctx->list_sizes.p,
                           ctx->walk_state.p + WS_TOTALS};
     for (int attempt = 0;; ++attempt) {
-        CK(ctx->pool_entry.ensure(32 * (size_t)ctx->cap_pool), "alloc walk");
-        CK(ctx->pool_next.ensure(ctx->cap_pool), "alloc walk");
-        CK(ctx->pool_owner.ensure(ctx->cap_pool), "alloc walk");
+        CK(pool_room(ctx, least, cap), "alloc walk");
         pool = WalkPool{ctx->pool_entry.p, ctx->pool_next.p, ctx->pool_owner.p, ctx->cap_pool,
                         reinterpret_cast<unsigned*>(ctx->walk_state.p + WS_USED),
                         reinterpret_cast<int*>(ctx->walk_state.p + WS_OVERFLOW)};
@@ -639,21 +666,34 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
             CK(cudaMemcpyAsync(&stack_overflow, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
         CK(cudaStreamSynchronize(s), "walk");
         if (stack_overflow) return fail(ctx, FMMX_DEVICE_ERROR, "f pre-pass stack overflow");
-        if (!hs[WS_OVERFLOW]) break;
-        if (attempt > 24 || ctx->cap_pool >= most) return fail(ctx, FMMX_OUT_OF_MEMORY, "walk capacity");
-        ctx->walk_retries++;
         const uint64_t used = (uint32_t)hs[WS_USED];
-        ctx->cap_pool = (uint32_t)std::min(std::max<uint64_t>(2ull * ctx->cap_pool, used + used / 4 + 64), most);
+        if (hs[WS_OVERFLOW]) {
+            if (attempt > 48 || ctx->cap_pool >= most) return fail(ctx, FMMX_OUT_OF_MEMORY, "walk capacity");
+            least = ctx->cap_pool;
+            cap = std::min(std::max<uint64_t>(2 * least, used + used / 4 + 64), most);
+        } else {
+            dm = hs[WS_TOTALS + 2];
+            dp = hs[WS_TOTALS + 3];
+            if (dm > 0x7fffffffull || dp > 0x7fffffffull)
+                return fail(ctx, FMMX_OUT_OF_MEMORY, "interaction lists above 2^31 entries");
+            cudaError_t e = ctx->m2l_src.ensure(std::max<size_t>(dm, 1));
+            if (e == cudaSuccess) e = ctx->p2p_src.ensure(std::max<size_t>(dp, 1));
+            if (e == cudaSuccess) break;
+            // the lists did not fit beside the pool: once more with what this walk used of it
+            cap = used + used / 16 + 64;
+            if (e != cudaErrorMemoryAllocation || attempt > 48 || cap >= ctx->cap_pool) return cuda_fail(ctx, e, "alloc lists");
+            ctx->budget.over = false;
+            ctx->pool_entry.release();
+            ctx->pool_next.release();
+            ctx->pool_owner.release();
+            ctx->pool_short = true;
+        }
+        ctx->walk_retries++;
     }
-    const uint64_t dm = hs[WS_TOTALS + 2], dp = hs[WS_TOTALS + 3];
-    if (dm > 0x7fffffffull || dp > 0x7fffffffull)
-        return fail(ctx, FMMX_OUT_OF_MEMORY, "interaction lists above 2^31 entries");
     ctx->pops = hs[WS_TOTALS];
     ctx->p2p_inter = hs[WS_TOTALS + 1];
     ctx->n_m2l = (int)(dm / 2);
     ctx->n_p2p = (int)((dp + (uint64_t)ctx->nleaves) / 2);  // a leaf's self pair is one entry
-    CK(ctx->m2l_src.ensure(std::max<size_t>(dm, 1)), "alloc lists");
-    CK(ctx->p2p_src.ensure(std::max<size_t>(dp, 1)), "alloc lists");
     CK(ctx->p2p_next.ensure(1), "alloc lists");
     // the near field's units and partial sums, coarser where they are too many for the 32-bit sums or the memory
     uint64_t units = hs[WS_TOTALS + 4], parts = hs[WS_TOTALS + 5];

@@ -152,6 +152,28 @@ def test_budget_of_large_leaves(precision, mib):
     assert np.linalg.norm(r1.accel - r0.accel) <= rel * np.linalg.norm(r0.accel)
 
 
+@pytest.mark.parametrize("n,p,n_leaf,mb", [(1000, 8, 16, 1.65), (3000, 2, 4, 8.5), (20_000, 4, 8, 56.0)])
+def test_budget_without_the_walk_expected_capacity(n, p, n_leaf, mb):
+    """A budget that holds the lists but not the pool a walk starts with: the
+    walk takes what there is, and the results are those without a budget. (The
+    first budget is what the engine took with pair buffers in place of the pool.)"""
+    mass, pos = fx().gen_plummer(n, seed=7)
+    kw = dict(mac="theta", theta=0.5, softening=1e-3)
+    r0 = fx().Fmm(mass, pos, p, 0.0, n_leaf, **kw).run()
+    budget = int(mb * 1e6)
+    g = fx().Fmm(None, None, p, 0.0, n_leaf, device_budget_bytes=budget, **kw)
+    for _ in range(3):
+        g.refresh(mass, pos)
+        r = g.run()
+        assert np.array_equal(r.accel, r0.accel) and np.array_equal(r.pot, r0.pot)
+        assert g.stats()["device_bytes"] <= budget
+    small = fx().gen_plummer(500, seed=9)  # a smaller system, then the first one again
+    g.refresh(*small)
+    g.run()
+    g.refresh(mass, pos)
+    assert np.array_equal(g.run().accel, r0.accel)
+
+
 def test_corrupted_ensemble_offsets():
     m1, p1 = fx().gen_plummer(3000, seed=1)
     m2, p2 = fx().gen_plummer(2000, seed=2)
