@@ -232,7 +232,7 @@ struct fmmx_ctx {
     // near-field work units (per leaf: first unit, first partial sum)
     DBuf<uint32_t> p2p_uoff, p2p_soff;
     DBuf<int32_t> p2p_ucell;
-    uint32_t p2p_nunits = 0, p2p_grain = P2P_GRAIN;
+    uint32_t p2p_nunits = 0;
     DBuf<double4> p2p_part;
     DBuf<float4> body_pairs;  // mixed near field: bodies relative to their leaf's centre, FP32, with the mass, in pairs
     DBuf<unsigned> p2p_next;
@@ -640,6 +640,7 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     }
     unsigned long long hs[WS_SIZE];
     uint64_t dm = 0, dp = 0;  // directed entries
+    uint4 sizes;
     WalkPool pool;
     const WalkLists lists{ctx->down_n.p, ctx->down_head.p, ctx->list_redone.p, ctx->list_sizes.p,
                           ctx->walk_state.p + WS_TOTALS};
@@ -662,6 +663,7 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
         LCOUNT(2);
         int stack_overflow = 0;
         CK(cudaMemcpyAsync(hs, ctx->walk_state.p, sizeof(hs), cudaMemcpyDeviceToHost, s), "copy");
+        CK(cudaMemcpyAsync(&sizes, ctx->list_off.p + nc, sizeof(sizes), cudaMemcpyDeviceToHost, s), "copy");
         if (dehnen)
             CK(cudaMemcpyAsync(&stack_overflow, ctx->flags.p + TF_STACK, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
         CK(cudaStreamSynchronize(s), "walk");
@@ -695,20 +697,24 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     ctx->n_m2l = (int)(dm / 2);
     ctx->n_p2p = (int)((dp + (uint64_t)ctx->nleaves) / 2);  // a leaf's self pair is one entry
     CK(ctx->p2p_next.ensure(1), "alloc lists");
-    // the near field's units and partial sums, coarser where they are too many for the 32-bit sums or the memory
-    uint64_t units = hs[WS_TOTALS + 4], parts = hs[WS_TOTALS + 5];
-    for (uint32_t grain = P2P_GRAIN;;) {
+    // the near field's units and partial sums, coarser where they are too many for the 32-bit sums or the
+    // memory. W targets times source leaves are at most the body pairs; a share has 64 source leaves or more, a unit 32
+    // targets, so W bounds both, and the 32-bit sums are right unless it is 1.4e11 and more: then they are counted anew.
+    const uint64_t W = ctx->p2p_inter + ctx->n;
+    const bool bounded = W / 32 <= 0xffffffffull && W / 2048 + ctx->n / 32 + dp / 64 + ctx->nleaves <= 0x7fffffffull &&
+                         ctx->p2p_parts_max == 0xffffffffull;
+    uint64_t units = sizes.z, parts = sizes.w;
+    for (uint32_t grain = bounded ? P2P_GRAIN : 0;;) {  // (0: not counted yet)
         cudaError_t e = cudaErrorMemoryAllocation;
-        if (units <= 0x7fffffffull && parts <= ctx->p2p_parts_max) {
+        if (grain && units <= 0x7fffffffull && parts <= ctx->p2p_parts_max) {
             e = ctx->p2p_ucell.ensure(std::max<size_t>(units, 1));
             if (e == cudaSuccess) e = ctx->p2p_part.ensure(std::max<size_t>(parts, 1));
         }
-        ctx->p2p_grain = grain;
         ctx->p2p_nunits = (uint32_t)units;
         if (e == cudaSuccess) break;
-        if (grain == P2P_WHOLE || e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "alloc p2p scratch");
+        if (grain == P2P_WHOLE || (grain && e != cudaErrorMemoryAllocation)) return cuda_fail(ctx, e, "alloc p2p scratch");
         ctx->budget.over = false;
-        grain = grain < (1u << 20) ? 8 * grain : P2P_WHOLE;
+        grain = !grain ? P2P_GRAIN : grain < (1u << 20) ? 8 * grain : P2P_WHOLE;
         unsigned long long* t = lists.totals + 4;
         CK(cudaMemsetAsync(t, 0, 2 * sizeof(*t), s), "memset");
         launch_near_sizes(s, nc, ctx->c_count.p, grain, lists);
@@ -734,7 +740,7 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
 // the near field's work units, as walk_impl left them
 P2pUnits near_units(fmmx_ctx* ctx) {
     return P2pUnits{ctx->p2p_uoff.p, ctx->p2p_ucell.p, ctx->p2p_soff.p, ctx->p2p_part.p, ctx->p2p_next.p,
-                    ctx->p2p_nunits, ctx->p2p_grain};
+                    ctx->p2p_nunits};
 }
 
 // Mixed form, near field: FP32 + double-single P2P on the second stream.

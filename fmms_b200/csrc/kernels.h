@@ -56,7 +56,7 @@ struct WalkLists {
     uint32_t* down_head;
     uint8_t* redone;
     uint4* sizes;                // ncells + 1
-    // pairs examined, body interactions, directed M2L and P2P entries, near-field work units and partial sums
+    // pairs examined, body interactions, directed M2L and P2P entries; k_near_sizes: work units, partial sums
     unsigned long long* totals;
 };
 
@@ -178,7 +178,6 @@ struct P2pUnits {
     double4* part;
     unsigned* next;  // work counter, zero at launch
     uint32_t nunits;  // below 2^31: the counter passes it by one per warp
-    uint32_t grain;   // see p2p_shares
 };
 
 // Work units of the near field, a warp each: up to P2P_NT targets of a leaf
@@ -219,6 +218,10 @@ __host__ __device__ __forceinline__ uint4 near_sizes(uint32_t m2l, uint32_t p2p,
 // units and partial sums of the leaves for another grain: sizes[c].z, .w and their sums totals[4], [5]
 // (both zero before)
 void launch_near_sizes(cudaStream_t s, int ncells, const uint32_t* count, uint32_t grain, WalkLists Ls);
+// shares of leaf c of nt bodies
+__device__ __forceinline__ uint32_t p2p_shares_of(const P2pUnits& U, int c, uint32_t nt) {
+    return (U.uoff[c + 1] - U.uoff[c]) / ((nt + P2P_NT - 1) / P2P_NT);
+}
 void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2pUnits U, double* ax, double* ay,
                         double* az, double* pot);
 void launch_p2p_f64(int nsm, cudaStream_t s, DirList L, int ncells, CellsView cv, P2pUnits U, const double* x,

@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS, 4) k_p2p_mixed(DirList L, Cel
         const int c = U.ucell[u];
         const uint32_t lb = L.seg_begin[c], len = L.seg_end[c] - lb;
         const uint32_t tf = cv.first[c], tn = cv.count[c];
-        const uint32_t ns_all = p2p_shares(tn, len, U.grain);
+        const uint32_t ns_all = p2p_shares_of(U, c, tn);
         const uint32_t k = u - U.uoff[c], share = k % ns_all, t0 = (k / ns_all) * P2P_NT;
         const uint32_t beg = lb + (uint32_t)((uint64_t)len * share / ns_all);
         const uint32_t end = lb + (uint32_t)((uint64_t)len * (share + 1) / ns_all);

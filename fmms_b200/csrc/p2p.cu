@@ -22,7 +22,7 @@ __global__ void k_p2p_combine(int ncells, DirList L, CellsView cv, P2pUnits U, d
     for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += warps) {
         if (U.soff[c + 1] == U.soff[c]) continue;
         const uint32_t tn = cv.count[c], tf = cv.first[c];
-        const uint32_t nu = p2p_shares(tn, L.seg_end[c] - L.seg_begin[c], U.grain);
+        const uint32_t nu = p2p_shares_of(U, c, tn);
         const double4* pp = U.part + U.soff[c];
         for (uint32_t i = lane; i < tn; i += 32) {
             double4 s = pp[i];
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(32 * P2PD_WARPS, 5) k_p2p_f64(DirList L, Cells
         const int c = U.ucell[u];
         const uint32_t lb = L.seg_begin[c], len = L.seg_end[c] - lb;
         const uint32_t tf = cv.first[c], tn = cv.count[c];
-        const uint32_t ns_all = p2p_shares(tn, len, U.grain);
+        const uint32_t ns_all = p2p_shares_of(U, c, tn);
         const uint32_t k = u - U.uoff[c], share = k % ns_all, t0 = (k / ns_all) * P2P_NT;
         const uint32_t beg = lb + (uint32_t)((uint64_t)len * share / ns_all);
         const uint32_t end = lb + (uint32_t)((uint64_t)len * (share + 1) / ns_all);

@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
     const int ncell = RING ? lcnt : min((int)*heavy.count, lcnt);
     const int32_t* cells = RING ? level_cells : heavy.list;
     uint32_t res_next = 0, res_end = 0;  // reserved chunks
-    unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0, nunits = 0, nparts = 0;  // thread sums (n*: thread 0)
+    unsigned long long pops = 0, inter = 0, nm2l = 0, np2p = 0;  // thread sums (n*: thread 0)
     // the unused rest of the reservation (fewer than `batch` chunks): nobody's
     auto give_back = [&]() {
         const uint32_t id = res_next + (uint32_t)tid;
@@ -493,10 +493,7 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
             Ls.down_n[c] = ld.n;
             Ls.down_head[c] = ld.head;
             Ls.redone[c] = RING ? 0 : 1;
-            const uint4 sz = near_sizes(lm.n, lp.n, tn, P2P_GRAIN);
-            nunits += sz.z;
-            nparts += sz.w;
-            Ls.sizes[c] = sz;
+            Ls.sizes[c] = near_sizes(lm.n, lp.n, tn, P2P_GRAIN);
         }
     }
     give_back();
@@ -510,8 +507,6 @@ __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict
         if (inter) atomicAdd(Ls.totals + 1, inter);
         if (nm2l) atomicAdd(Ls.totals + 2, nm2l);
         if (np2p) atomicAdd(Ls.totals + 3, np2p);
-        if (nunits) atomicAdd(Ls.totals + 4, nunits);
-        if (nparts) atomicAdd(Ls.totals + 5, nparts);
     }
 }
 
