@@ -97,6 +97,16 @@ struct CellsView {
 // grid-stride and persistent kernels are multiples of it)
 inline int g_nsm = 148;
 
+// Allows a kernel whose shared memory depends on the order as much as any order
+// needs. The limit belongs to the device and the kernel, not to the launch, so it
+// has to be the same whoever sets it: contexts of other orders launch from other
+// threads.
+#define FMMX_SMEM_MOST (200 * 1024)
+template <class Kernel>
+static inline cudaError_t allow_smem(Kernel* kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FMMX_SMEM_MOST);
+}
+
 // blocks for n items at `block` threads, at most cap (default 32 per SM; the
 // kernels stride over the rest)
 static inline unsigned grid_for(size_t n, int block, unsigned cap = 0) {

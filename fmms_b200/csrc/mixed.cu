@@ -408,14 +408,12 @@ void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, C
                          const double* ell, const double* x, const double* y, const double* z, const double* m, int p,
                          zf* mom, unsigned* arrive) {
     const int H = (p + 1) * (p + 2) / 2, F2 = (p + 1) * (p + 1);
-    // (the limits are the same whatever p, so that contexts of other orders on other threads cannot lower them)
-    const size_t most = 200 * 1024;
-    cudaFuncSetAttribute(k_p2m_mixed<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    cudaFuncSetAttribute(k_p2m_mixed<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    cudaFuncSetAttribute(k_m2m_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    allow_smem(k_p2m_mixed<float>);
+    allow_smem(k_p2m_mixed<double>);
+    allow_smem(k_m2m_mixed);
     auto warps = [&](size_t col) {  // per block: as many as its columns leave room for, 1 .. 4
         int w = 4;
-        while (w > 1 && w * col > most) w >>= 1;
+        while (w > 1 && w * col > FMMX_SMEM_MOST) w >>= 1;
         return w;
     };
     const size_t cf = (size_t)32 * H * sizeof(zf), cd = (size_t)32 * H * sizeof(zd);
@@ -574,14 +572,12 @@ void launch_l2l_mixed(bool fp64, unsigned grid, cudaStream_t s, const int32_t* l
     const unsigned blocks = std::max(1u, std::min(grid, (unsigned)((lcnt + L2LB_WARPS - 1) / L2LB_WARPS)));
     if (fp64) {
         const size_t sm = l2l_smem<double>(p);
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_l2l_mixed<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k_l2l_mixed<double>);
         k_l2l_mixed<double><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
                                                                loc);
     } else {
         const size_t sm = l2l_smem<float>(p);
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_l2l_mixed<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k_l2l_mixed<float>);
         k_l2l_mixed<float><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
                                                                loc);
     }

@@ -43,3 +43,35 @@ def test_two_streams_give_the_same_bits(precision, mac):
         out.append((r.accel, r.pot))
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("precision,orders", [("plain", (12, 8)), ("plain", (20, 14)), ("mixed", (16, 14))])
+def test_contexts_of_other_orders_on_other_threads(precision, orders):
+    """Two host threads, each with a context of its own order: a kernel's shared
+    memory limit belongs to the device, so neither thread may lower it between
+    the other's setting and its launch. Every evaluation succeeds with the bits
+    it gives alone."""
+    import threading
+
+    import fmms_b200 as fx
+
+    mass, pos = fx.gen_plummer(600, seed=5)
+    kw = dict(mac="theta", theta=0.6, softening=1e-3, precision=precision)
+    alone = {p: fx.Fmm(mass, pos, p, 0.0, 8, **kw).run().accel for p in orders}
+    errors = []
+
+    def work(p):
+        try:
+            g = fx.Fmm(mass, pos, p, 0.0, 8, **kw)
+            for _ in range(400):
+                if not np.array_equal(g.run().accel, alone[p]):
+                    errors.append((p, "other bits"))
+        except Exception as e:  # noqa: BLE001
+            errors.append((p, str(e)))
+
+    threads = [threading.Thread(target=work, args=(p,)) for p in orders * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:4]
