@@ -716,12 +716,14 @@ __device__ __forceinline__ void p2p_pair(const float4 a, const float4 b, float2 
 }
 
 // The pair with the target's own body at half h (0 or 1) of it: that half
-// becomes a massless body one unit away (no term).
+// becomes a massless body 1 + |x| away (no term). One unit alone is lost in the
+// rounding where |x| is 2^24 and more (positions in metres): r = 0, 0 times infinity.
 __device__ __forceinline__ void mask_self(float4& a, float4& b, int h, float x, float y, float z) {
+    const float away = x + (1.f + fabsf(x));
     if (h == 0) {
-        a.x = x + 1.f; a.z = y; b.x = z; b.z = 0.f;
+        a.x = away; a.z = y; b.x = z; b.z = 0.f;
     } else {
-        a.y = x + 1.f; a.w = y; b.y = z; b.w = 0.f;
+        a.y = away; a.w = y; b.y = z; b.w = 0.f;
     }
 }
 

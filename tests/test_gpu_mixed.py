@@ -132,3 +132,21 @@ def test_mixed_p2p_giant_leaf_and_tiles(tile):
         assert np.percentile(e, 99) < 1e-5 and np.max(e) < 1e-4, (np.percentile(e, 99), np.max(e))
         pe = np.abs(res.pot[part] - ref.pot[part]) / np.abs(ref.pot[part])
         assert np.max(pe) < 1e-5, np.max(pe)
+
+
+@pytest.mark.parametrize("unit", [1e-9, 1e3, 1e9])
+def test_unsoftened_near_field_in_any_unit(unit):
+    """No softening, positions in other units (leaves of 1e8 and more across:
+    metres): a target's own body gives no term. Accelerations scale with 1/unit^2;
+    the sums are FP32 in groups, so the units agree to 1e-5 as a whole, as long as
+    a pair's m/r^3 is a normal FP32 number (here 2e-4 / (10 unit)^3 > 1.2e-38: unit
+    below 2.5e10)."""
+    import fmms_b200 as fx
+
+    mass, pos = fx.gen_plummer(5000, seed=3)
+    kw = dict(mac="theta", theta=0.5, precision="mixed")
+    ref = fx.Fmm(mass, pos, 6, 0.0, 64, **kw).run()
+    r = fx.Fmm(mass, pos * unit, 6, 0.0, 64, **kw).run()
+    assert np.isfinite(r.accel).all() and np.isfinite(r.pot).all()
+    assert np.linalg.norm(r.accel * unit**2 - ref.accel) <= 1e-5 * np.linalg.norm(ref.accel)
+    assert np.linalg.norm(r.pot * unit - ref.pot) <= 1e-5 * np.linalg.norm(ref.pot)
