@@ -13,12 +13,13 @@ namespace fmmx {
 
 #define DIR_BLOCK 128
 
-// Splits of the sources for nt targets: 32, and more where there are too few
-// target blocks to fill the GPU (a warp's worth of sources each at least);
-// nsplit * nt stays within 32 x 4096 or, for more targets, 32 nt.
+// Splits of the sources for nt targets: 32 (whatever n), and up to 1024 where
+// there are too few target blocks to give every SM eight, as long as each has a
+// block's worth of sources; nsplit * nt stays within 32 x 4096 or, for more
+// targets, 32 nt.
 int direct_splits(size_t n, size_t nt) {
     const size_t blocks = (nt + DIR_BLOCK - 1) / DIR_BLOCK;
-    const size_t want = 8 * 148 / blocks, room = (size_t)32 * 4096 / (nt < 4096 ? nt : 4096);
+    const size_t want = 8 * (size_t)g_nsm / blocks, room = (size_t)32 * 4096 / (nt < 4096 ? nt : 4096);
     size_t s = want < room ? want : room;
     const size_t by_n = (n + DIR_BLOCK - 1) / DIR_BLOCK;
     if (s > by_n) s = by_n;

@@ -545,9 +545,9 @@ fmmx_status build_impl(fmmx_ctx* ctx, size_t n, const double* d_pos, const doubl
     } else {
         for (int L = nlev - 1; L >= 0; --L) {
             const int cnt = ctx->lvl_count[L];
-            k_geometry_level<<<grid_for(cnt, 128), 128, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt,
-                                                                view_mut(ctx), ctx->x.p, ctx->y.p, ctx->z.p,
-                                                                ctx->m.p, ctx->cfg.center_mode);
+            k_geometry_ritter<<<grid_for(cnt, 128), 128, 0, s>>>(ctx->level_cells.p, ctx->lvl_start[L], cnt,
+                                                                 view_mut(ctx), ctx->x.p, ctx->y.p, ctx->z.p,
+                                                                 ctx->m.p);
         }
         k_pack_geo<<<grid_for(nc, 256), 256, 0, s>>>(nc, view_mut(ctx), ctx->c_geo.p);
         LCOUNT(nlev);
@@ -612,13 +612,12 @@ fmmx_status walk_impl(fmmx_ctx* ctx, cudaStream_t s) {
     const size_t tb = scan_u32x4_temp(nc + 1);
     CK(ctx->cub_tmp.ensure(tb), "alloc scan");
     MacParams mp;
-    mp.mode = ctx->cfg.mac_mode;
     mp.p = ctx->cfg.p;
     mp.eps = ctx->cfg.mac_eps;
     mp.theta = ctx->cfg.theta;
     mp.gap = ctx->cfg.soft_gap * ctx->cfg.softening;
     const CellsView cv = view(ctx);
-    const bool dehnen = mp.mode == FMMX_MAC_DEHNEN;
+    const bool dehnen = ctx->cfg.mac_mode == FMMX_MAC_DEHNEN;
     if (dehnen) {
         CK(ctx->mac_rows.ensure((size_t)nc * (mp.p + 2)), "alloc walk");
         k_mac_rows<<<grid_for(nc, 128), 128, 0, s>>>(nc, cv, mp.p, ctx->pows.p, ctx->fmin.p, ctx->mac_rows.p);
@@ -743,7 +742,7 @@ P2pUnits near_units(fmmx_ctx* ctx) {
                     ctx->p2p_nunits};
 }
 
-// Mixed form, near field: FP32 + double-single P2P on the second stream.
+// Mixed form, near field: FP32 P2P with FP64 sums on the second stream.
 fmmx_status near_mixed(fmmx_ctx* ctx, const DirList& lp, bool tm) {
     cudaStream_t s2 = ctx->cfg.overlap ? ctx->stream2 : ctx->stream;
     const int nc = ctx->nc;
@@ -774,7 +773,7 @@ fmmx_status far_mixed(fmmx_ctx* ctx, const DirList& lm, double* d_acc, double* d
     CK(cudaMemsetAsync(ctx->loc_f.p, 0, (size_t)nc * half_stride(p) * sizeof(zf), s), "memset");
     if (ctx->n_m2l > 0) {
         if (p > kRotwMaxP) return fail(ctx, FMMX_INVALID_ARG, "mixed precision supports p <= 16");
-        int* work = nullptr;  // preemptible: one block per destination cell
+        int* work = nullptr;  // preemptible: short blocks instead of persistent ones
         if (!ctx->cfg.preemptible) {
             CK(ctx->work.ensure(1), "alloc");
             CK(cudaMemsetAsync(ctx->work.p, 0, sizeof(int), s), "memset");
@@ -920,7 +919,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
     if (tm) CK(cudaEventRecord(ev[5], s2), "event");
 
     // (the lists' pointers are taken after the walk, which may reallocate them)
-    const DirList lp{nullptr, ctx->p2p_src.p, ctx->p2p_off.p, ctx->p2p_off.p + 1, 32};
+    const DirList lp{ctx->p2p_src.p, ctx->p2p_off.p, ctx->p2p_off.p + 1};
     if (mixed) {
         fmmx_status ms = near_mixed(ctx, lp, tm);
         if (ms != FMMX_OK) return ms;
@@ -935,7 +934,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         CK(cudaEventRecord(ctx->fork[2], s2), "event");
     }
     if (!reuse) CK(cudaStreamWaitEvent(s, ctx->fork[1], 0), "join");  // the M2L reads its list
-    const DirList lm{nullptr, ctx->m2l_src.p, ctx->m2l_off.p, ctx->m2l_off.p + 1, 32};
+    const DirList lm{ctx->m2l_src.p, ctx->m2l_off.p, ctx->m2l_off.p + 1};
     if (mixed) {
         fmmx_status ms = far_mixed(ctx, lm, d_acc, d_pot, tm);
         if (ms != FMMX_OK) return ms;
@@ -946,7 +945,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         const unsigned g = std::min<unsigned>(nc, 16u * (unsigned)ctx->nsm);
         const M2lChoice ch = m2l_choice(ctx->cfg);
         if (ch == M2L_ROT_WARP) {
-            int* work = nullptr;  // preemptible: one block per destination cell
+            int* work = nullptr;  // preemptible: short blocks instead of persistent ones
             if (!ctx->cfg.preemptible) {
                 CK(ctx->work.ensure(1), "alloc");
                 CK(cudaMemsetAsync(ctx->work.p, 0, sizeof(int), s), "memset");

@@ -28,7 +28,6 @@ struct CellsMut {
 };
 
 struct MacParams {
-    int mode;  // fmmx_mac_mode
     int p;
     double eps;
     double theta;
@@ -60,16 +59,12 @@ struct WalkLists {
     unsigned long long* totals;
 };
 
-// Segmented directed interaction list: for destination cell c, sources
-// src(key(i)) for i in [seg_begin[c], seg_end[c]), in the walk's order.
+// Directed interaction list: for destination cell c, the sources src[seg_begin[c]
+// .. seg_end[c]), in the walk's order.
 struct DirList {
-    const uint64_t* keys;    // entries (dst << shift) | src, or null
-    const uint32_t* keys32;  // 32-bit entries (then keys is null); with shift = 32 the entries are the sources
+    const uint32_t* src;
     const uint32_t* seg_begin;
     const uint32_t* seg_end;
-    int shift;
-    __host__ __device__ uint64_t key(size_t i) const { return keys32 ? (uint64_t)keys32[i] : keys[i]; }
-    __host__ __device__ uint32_t src(uint64_t key) const { return (uint32_t)(key & ((1ull << shift) - 1)); }
 };
 
 // tree_exact.cu
@@ -99,8 +94,8 @@ __global__ void k_cell_emit(const uint64_t* keys, uint32_t n, const uint64_t* of
 #define GEO_WARPS 4
 __global__ void k_geometry_com(int nc, CellsMut cells, const double* x, const double* y, const double* z,
                                const double* m, unsigned* arrive, double4* geo);
-__global__ void k_geometry_level(const int32_t* level_cells, int lstart, int lcnt, CellsMut cells, const double* x,
-                                 const double* y, const double* z, const double* m, int center_mode);
+__global__ void k_geometry_ritter(const int32_t* level_cells, int lstart, int lcnt, CellsMut cells, const double* x,
+                                  const double* y, const double* z, const double* m);
 // bodies per round of the exact P2M (the lanes of a warp build that many Υ tables at once)
 __host__ __device__ inline int p2m_round(int p) { return p <= 12 ? 32 : (p <= 16 ? 16 : 8); }
 __host__ __device__ size_t upward_exact_smem_per_warp(int p);

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(32 * W, (rotw_warps_per_sm<T, P>() / W))
     Z* col = sbuf + lane;           // this lane's column: entry e at col[32 e]
     Z* pha = sbuf + 32 * H + lane;  // e^{imα}, m = 1..P (where not in registers)
     Z* phb = pha + 32 * P;          // e^{imβ}
-    const uint32_t* __restrict__ srcs = L.keys32;
+    const uint32_t* __restrict__ srcs = L.src;
     auto clear = [&]() {
 #pragma unroll 4
         for (int e = 0; e < H; ++e) col[32 * e] = mk<T>(T(0), T(0));

@@ -800,8 +800,9 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS, 4) k_p2p_mixed(DirList L, Cel
         const float2 nx0 = make_float2(-x0, -x0), ny0 = make_float2(-y0, -y0), nz0 = make_float2(-z0, -z0);
         const float2 nx1 = make_float2(-x1, -x1), ny1 = make_float2(-y1, -y1), nz1 = make_float2(-z1, -z1);
         double a0x = 0, a0y = 0, a0z = 0, p0 = 0, a1x = 0, a1y = 0, a1z = 0, p1 = 0;
-        // FP32 partial sums, added into the FP64 sums once they hold
-        // P2PM_FLUSH source pairs (and at the end)
+        // FP32 partial sums, added into the FP64 sums after the tile with which
+        // they reach P2PM_FLUSH source pairs (and at the end): at most P2PM_FLUSH - 1
+        // pairs and a tile's share, half of its pairs or less (R >= 2)
         float2 q0x{0, 0}, q0y{0, 0}, q0z{0, 0}, q0p{0, 0}, q1x{0, 0}, q1y{0, 0}, q1z{0, 0}, q1p{0, 0};
         int held = 0;
         auto flush = [&]() {
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS, 4) k_p2p_mixed(DirList L, Cel
 #pragma unroll
             for (int h = 0; h < P2PW_CHUNK / 32; ++h) {
                 const int q = lane + 32 * h;
-                src[h] = q < ns ? (int)L.keys32[sc + q] : -1;
+                src[h] = q < ns ? (int)L.src[sc + q] : -1;
             }
 #pragma unroll
             for (int h = 0; h < P2PW_CHUNK / 32; ++h) {

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32 * P2PD_WARPS, 5) k_p2p_f64(DirList L, Cells
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 const int q = lane + 32 * h;
-                src[h] = q < ns ? (int)L.keys32[sc + q] : -1;
+                src[h] = q < ns ? (int)L.src[sc + q] : -1;
             }
 #pragma unroll
             for (int h = 0; h < H; ++h) {

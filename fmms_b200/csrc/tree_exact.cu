@@ -526,60 +526,35 @@ __device__ void ritter(const Items& it, double cen[3]) {
     }
 }
 
-// Octree::geometry, tree.rs:152-227, one level at a time from the deepest, a
-// thread per cell: the Ritter spheres (each a serial scan of its items), whose
-// centres of mass k_geometry_com does not serve.
-__global__ void k_geometry_level(const int32_t* __restrict__ level_cells, int lstart, int lcnt, CellsMut cells,
-                                 const double* __restrict__ x, const double* __restrict__ y,
-                                 const double* __restrict__ z, const double* __restrict__ m, int center_mode) {
+// Octree::geometry with Ritter centres, tree.rs:152-227, one level at a time from
+// the deepest, a thread per cell (each sphere is a serial scan of its items;
+// centres of mass: k_geometry_com).
+__global__ void k_geometry_ritter(const int32_t* __restrict__ level_cells, int lstart, int lcnt, CellsMut cells,
+                                  const double* __restrict__ x, const double* __restrict__ y,
+                                  const double* __restrict__ z, const double* __restrict__ m) {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < lcnt; j += gridDim.x * blockDim.x) {
         const int c = level_cells[lstart + j];
         double mass = 0.0, cen[3], rho = 0.0;
         if (cells.leaf[c]) {
             const uint32_t f = cells.first[c], e = f + cells.count[c];
             for (uint32_t k = f; k < e; ++k) mass += m[k];
-            if (center_mode == FMMX_CENTER_COM) {
-                double com[3] = {0.0, 0.0, 0.0};
-                for (uint32_t k = f; k < e; ++k) {
-                    com[0] += m[k] * x[k];
-                    com[1] += m[k] * y[k];
-                    com[2] += m[k] * z[k];
-                }
-                cen[0] = com[0] / mass;
-                cen[1] = com[1] / mass;
-                cen[2] = com[2] / mass;
-            } else {
-                LeafItems it{x, y, z, f, e - f};
-                ritter(it, cen);
-            }
+            LeafItems it{x, y, z, f, e - f};
+            ritter(it, cen);
             for (uint32_t k = f; k < e; ++k) rho = fmax(rho, dist3(x[k], y[k], z[k], cen[0], cen[1], cen[2]));
         } else {
-            const int32_t* ch = cells.child + 8 * c;
+            const int32_t* ch = cells.child + 8 * (size_t)c;
+            ChildItems it;
+            it.nitems = 0;
             for (int o = 0; o < 8; ++o)
-                if (ch[o] >= 0) mass += cells.mass[ch[o]];
-            if (center_mode == FMMX_CENTER_COM) {
-                double com[3] = {0.0, 0.0, 0.0};
-                for (int o = 0; o < 8; ++o) {
-                    int q = ch[o];
-                    if (q < 0) continue;
-                    com[0] += cells.mass[q] * cells.cx[q];
-                    com[1] += cells.mass[q] * cells.cy[q];
-                    com[2] += cells.mass[q] * cells.cz[q];
+                if (ch[o] >= 0) {
+                    mass += cells.mass[ch[o]];
+                    it.ids[it.nitems++] = ch[o];
                 }
-                cen[0] = com[0] / mass;
-                cen[1] = com[1] / mass;
-                cen[2] = com[2] / mass;
-            } else {
-                ChildItems it;
-                it.nitems = 0;
-                for (int o = 0; o < 8; ++o)
-                    if (ch[o] >= 0) it.ids[it.nitems++] = ch[o];
-                it.cx = cells.cx;
-                it.cy = cells.cy;
-                it.cz = cells.cz;
-                it.rho = cells.rho;
-                ritter(it, cen);
-            }
+            it.cx = cells.cx;
+            it.cy = cells.cy;
+            it.cz = cells.cz;
+            it.rho = cells.rho;
+            ritter(it, cen);
             for (int o = 0; o < 8; ++o) {
                 int q = ch[o];
                 if (q < 0) continue;
@@ -878,7 +853,7 @@ __global__ void k_upward_exact(const int32_t* __restrict__ level_cells, int lsta
 // the Υ tables of the (up to 8) child offsets and each child's convolution
 // sums s_o[e] (8 dim independent chains) are computed side by side; then
 // every coefficient adds its children's sums in octant order, as m2m_cell
-// (moments.rs:56-90) does one child after the other. Power and fmin as in
+// (moments.rs:56-90) does one child after the other. Power as in
 // k_upward_exact. Shared memory: 16 dim complex.
 __global__ void __launch_bounds__(M2M_EXACT_WIDE) k_m2m_exact_block(const int32_t* __restrict__ level_cells, int lstart,
                                                          int lcnt, CellsView cells, int p, zd* __restrict__ moments,

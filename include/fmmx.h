@@ -80,7 +80,8 @@ typedef struct fmmx_config {
     void* stream;      /* cudaStream_t to run on, or NULL for a private stream */
     int p2p_tile;      /* source bodies a block of the mixed P2P stages at a time: 256 (any value up to it), 512
                           or 1024; 0 = 512 */
-    int preemptible;   /* 1: the M2L runs one short block per destination cell instead of persistent warps,
+    int preemptible;   /* 1: the M2L runs short blocks (one destination cell each, up to eight at high order) instead of
+                          persistent warps,
                           so kernels on higher-priority streams start between its blocks (serving lanes);
                           0 (default): persistent warps, the faster form for one evaluation at a time */
     double soft_gap;   /* extension, with softening > 0: a cell pair is accepted for M2L only if its bodies are
