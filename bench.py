@@ -398,11 +398,11 @@ class _NullCtx:
 
 
 # DRAM bytes (read + write) per directed M2L translation, from one ncu capture of
-# the M2L launch at N = 262144 (uniform cube, p = 10, theta 0.5, leaf 64: 5,809,554
+# the M2L launch at N = 262144 (uniform cube, p = 10, theta 0.5, leaf 64: 5,879,670
 # directed translations); the expansions are L2-resident, so the traffic grows
 # with the translation count.
-M2L_DRAM_BYTES_PER_TRANSLATION = {("mixed", 10): (34.537728e6 + 0.07424e6) / 5809554,
-                                  ("plain", 10): (84.023808e6 + 21.590272e6) / 5809554}
+M2L_DRAM_BYTES_PER_TRANSLATION = {("mixed", 10): (34.797056e6 + 0.011008e6) / 5879670,
+                                  ("plain", 10): (61.145344e6 + 17.89952e6) / 5879670}
 
 
 def roofline(args, cfg, r, precision, dev):

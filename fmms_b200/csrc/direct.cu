@@ -2,8 +2,9 @@
 // reference (direct.rs:6-31 one-sided, and the sampled error of
 // crates/bench/src/main.rs:34-78). Sources are split across blockIdx.y; each
 // split writes its partial sums and k_direct_reduce adds them in split order,
-// so the result is deterministic. Bound by the FP64 pipe (a square root and a
-// division per pair, instead of the one reciprocal root, took half the time).
+// so the result is deterministic. Bound by the latency of the FP64 chains and the
+// FP64 pipe (4,096 targets of 2^18 bodies: issue 57 %, FP64 pipe 55 %, 1.9 ms; with a
+// square root and a division per pair, instead of one reciprocal root, 3.0 ms).
 #include <mutex>
 
 #include "common.cuh"

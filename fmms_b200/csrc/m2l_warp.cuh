@@ -390,7 +390,11 @@ constexpr size_t rotw_smem_per_warp() {
 
 // Resident warps per SM: what the columns leave room for in 224 KB of shared
 // memory (1 KB per block is the system's), and as many as the registers allow
-// without spilling the expansion.
+// without spilling the expansion. FP32 keeps it, with the phases and two degrees'
+// temporaries, in 128 registers up to P = 6 (16 warps), in 168 up to P = 10 (12
+// warps) and in 255 above (8 warps; 9 of 224: P = 12 2.24 ms against 1.84). FP64
+// uses 166 registers at P = 4 (12 warps) and 246 and more from P = 5 (8 warps);
+// from P = 10 it spills at 255.
 template <typename T, int P>
 constexpr int rotw_warps_per_sm() {
     const int by_smem = (int)(224 * 1024 / (rotw_smem_per_warp<T, P>() + 1024));
@@ -484,7 +488,10 @@ __device__ __forceinline__ void rotw_fwd(const TRegs<T, P>& t, const PhRegs<T, P
 // its tables in constant memory: FP32 p = 8 0.88, 10 1.82, 12 4.90, 14 8.70;
 // FP64 p = 6 1.64, 8 3.76, 10 6.14, 12 17.9, 14 38.9 ms. The FP32 form is
 // bound by issue and instruction latency (12 warps per SM, 168 registers), the
-// FP64 form by latency at 3 to 8 warps per SM (shared memory for the columns).
+// FP64 form by latency at 2 to 8 warps per SM (shared memory for the columns).
+// FP64 p = 14 takes twice p = 13 (17.1 and 8.6 ms): two warps of columns fit instead
+// of three, half again as much is spilled (1.6 KB a thread), and two warps in step
+// share each fetch between them instead of three (no_instruction 1.8 per issue).
 template <typename T, int P, bool SCALED, bool FULL_LAYOUT, int W>
 __global__ void __launch_bounds__(32 * W, (rotw_warps_per_sm<T, P>() / W))
     k_m2l_rotw(DirList L, int ncells, CellsView cv, const T* __restrict__ scale, const cplx<T>* __restrict__ mom,

@@ -164,7 +164,8 @@ __global__ void k_moments_to_mixed(int nc, int p, const zd* __restrict__ full, c
 // adds m Υ into its own column of shared memory; the columns are summed at the
 // end, lane e taking entry e from its own column on (distinct banks). A =
 // double for the leaves of the top three levels (`top`), float below. Bound by
-// shared memory and latency. (A 128-thread block per leaf, a thread per column
+// latency at the 9 warps per SM that the columns leave room for (p = 10: issue
+// 39 %, shared-memory pipe 15 %). (A 128-thread block per leaf, a thread per column
 // and body group, took 0.31 ms for 32,768 leaves of 32 bodies at p = 10.)
 template <typename A>
 __global__ void __launch_bounds__(128) k_p2m_mixed(const int32_t* __restrict__ list, int nc, bool top,
@@ -274,8 +275,8 @@ __device__ __forceinline__ void ups_column_full(A x, A y, A z, A r2, int p, int 
 // a product is two loads and four FMAs; then a thread per (child, entry) sums that
 // child's contribution and the children are added in octant order. A = double on
 // the top three levels, float below. Bound by latency: the products of a cell
-// (13,700 at p = 10) take a few hundred instructions a thread. arrive: one zero
-// per cell. (With P2M in the same kernel and a launch per level: N = 1e3, 7
+// (13,700 at p = 10) take a few hundred instructions a thread between barriers
+// (issue 44 %, 8.4 barrier stalls per issue). arrive: one zero per cell. (With P2M in the same kernel and a launch per level: N = 1e3, 7
 // levels, 0.15 ms; N = 2^20 uniform 0.70 ms.)
 #define M2M_BLOCK 512
 #define M2M_SCAN 32  // cells a block looks over at a time for its starting points
@@ -588,8 +589,8 @@ void launch_l2l_mixed(bool fp64, unsigned grid, cudaStream_t s, const int32_t* l
 // recursion in k) and contracted on the fly. The orders +l and -l of a real field
 // contribute equally to Ψ_0^0 and Ψ_1^0, and to Ψ_1^1 through L_{k+1,l+1} and
 // L_{k+1,l-1}, so only l >= 0 is run through; L_{k,l} is the last step's
-// L_{k+1,l}. Bound by issue (N = 2^20, p = 10: 0.25 ms with both signs written
-// out).
+// L_{k+1,l}. Bound by issue, 69 % of the time, and the loads of the locals
+// (N = 2^20, p = 10: 0.13 ms; 0.25 with both signs written out).
 __global__ void k_l2p_mixed(size_t n, const int32_t* __restrict__ body_leaf, const uint32_t* __restrict__ order,
                             CellsView cv, const double* __restrict__ ell, int p, const zf* __restrict__ loc,
                             const double* __restrict__ x, const double* __restrict__ y,

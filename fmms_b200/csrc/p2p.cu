@@ -74,8 +74,9 @@ void launch_p2p_combine(cudaStream_t s, int ncells, DirList L, CellsView cv, P2p
 // groups of G = ceil(nt / 2) lanes over the targets, R = 32 / G groups over the
 // source bodies of each tile, reduced in group order at the end. A table gives
 // each source body's leaf, and the next tile's loads are in flight while a tile
-// is computed. Bound by the FP64 pipe (about 20 FP64 instructions per
-// interaction, the reciprocal square root half of them).
+// is computed. Bound by the FP64 pipe, 66 % busy at 15 bodies per leaf (about 20
+// FP64 instructions per interaction, the reciprocal square root half of them), and
+// the latency of its chains (N = 2^18: 1.37 ms; a block per leaf took 2.20).
 #define P2PD_CHUNK 128
 #define P2PD_MAP 2048
 #define P2PD_TILE 64

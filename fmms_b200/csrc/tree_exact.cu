@@ -932,8 +932,10 @@ __global__ void __launch_bounds__(M2M_EXACT_WIDE) k_m2m_exact_block(const int32_
 // themselves, so every body's sum is the reference's, term by term. A cell's
 // record goes onto the stack with it (eight lanes read eight children at once),
 // and a leaf's bodies are read side by side into shared memory: one L2 round trip
-// per expansion or leaf instead of several per body and cell. Bound by those round
-// trips and by the FP64 divisions. (A thread per body with its own stack took
+// per expansion or leaf instead of several per body and cell. Bound by the latency
+// of the dependent FP64 terms, a division each, and then by those round trips
+// (10^5 bodies: 15 warps per SM, issue 47 %, FP64 pipe 28 %; stalls 4.1 wait, 1.4
+// long scoreboard per issue). (A thread per body with its own stack took
 // 0.90 ms for 16,384 bodies and 1.58 ms for a cuspy profile of 10^5.)
 #define FPRE_STACK (8 * FMMX_NLEVELS + 32)
 struct FpreWarp {

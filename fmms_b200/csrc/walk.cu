@@ -17,7 +17,7 @@
 // alone: no list has to be sorted or scattered. (The walk used to append mutual
 // pairs with atomics, a frontier at a time, and a counting sort and segment sorts
 // made the lists. Walk and lists alone on the device: N = 2^22, 64 clusters,
-// 14.4 + 47 -> 21.1 + 2.5 ms; uniform 2^20 0.41 + 0.99 -> 0.44 + 0.07; 10^3
+// 14.4 + 47 -> 21.3 + 2.5 ms; uniform 2^20 0.41 + 0.99 -> 0.44 + 0.07; 10^3
 // bodies 0.145 + 0.22 -> 0.13 + 0.01.)
 //
 // The sources of a cell are taken in blocks of WK_BLOCK inherited entries; of a
@@ -239,9 +239,11 @@ __device__ __forceinline__ unsigned long long pack4(uint32_t a, uint32_t b, uint
 // disjoint subtrees, so as many as there are leaves always suffice).
 // list_mode: the cells are heavy.list[0 .. *heavy.count), else the level's. A cell
 // whose queue is full, or (W = 1) that has taken `limit` sources, is left to
-// the heavy list. Bound by the L2 round trips of a step (the sources' records,
-// then the children of those that split) at shallow levels, by issue where a
-// level has many cells.
+// the heavy list. Bound at shallow levels by the steps' barriers and L2 round
+// trips (the sources' records, then the children of those that split: issue 20
+// to 40 % of the time); where a level has many cells by issue with the theta
+// criterion (53 to 55 %, 17 to 22 warps per SM) and by round trips with Dehnen's
+// (26 to 29 %, 8 to 11 warps of 128 registers).
 template <bool DEHNEN, int W, int RING>
 __global__ void __launch_bounds__(32 * W) k_walk_level(const int32_t* __restrict__ level_cells, int lcnt, CellsView cv,
                                                        const int32_t* __restrict__ parent, MacParams mp,

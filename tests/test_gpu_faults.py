@@ -61,8 +61,8 @@ def test_over_budget_in_evaluate():
 
 
 def test_walk_overflow_retry_gives_the_same_bits(monkeypatch):
-    """Walk buffers of 64 pairs (FMMX_TEST_WALK_CAPACITY): the walk overflows
-    and is redone with larger buffers until it fits; the lists, and so every
+    """A pool of 64 list entries, two chunks (FMMX_TEST_WALK_CAPACITY): the walk
+    overflows and is redone with a larger one until it fits; the lists, and so every
     result bit, are those of a context sized for the tree."""
     mass, pos, _ = fx().gen_plummer_ic(30_000, 1.0, 1.0, 20.0, 8)
     kw = dict(mac="theta", theta=0.5, softening=1e-3)
