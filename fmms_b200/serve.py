@@ -75,11 +75,9 @@ import numpy as np
 
 # Device bytes per body kept resident (pos, vel, acc, pot, mass, dt: 12 FP64) and
 # the engine's working memory per body of a forest evaluation (tree, expansions,
-# lists) at p=8, leaf 64 with headroom (1e3 to 1e6 bodies: Plummer 960 to 1,200 B, up to
-# 2,000 for 1e3; uniform 620 to 1,720, most where its leaves have just split); plus a
-# fixed part per session.
+# lists) at p=8, leaf 64 with headroom; plus a fixed part per session.
 RESIDENT_BYTES_PER_BODY = 96
-ENGINE_BYTES_PER_BODY = 1900
+ENGINE_BYTES_PER_BODY = 640
 SESSION_FIXED_BYTES = 1 << 20
 STAGED_BYTES_PER_BODY = 56  # pos, vel, mass staged on the device while queued
 SMALL_POOL_RESERVE = 256 << 20  # small-block pool reserved per stream (blocks <= 1 MB)

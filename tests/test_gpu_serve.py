@@ -83,16 +83,3 @@ def test_forest_tree_reuse_in_serving():
         pa, va, _ = run_session_alone(s, **kw)
         scale = np.abs(pa).max()
         assert np.max(np.abs(s.result_pos - pa)) < 1e-7 * scale
-
-
-@pytest.mark.parametrize("n", [1000, 30_000, 300_000])
-def test_admission_covers_the_engine_memory(n):
-    """What admission charges a session for the engine is at least what the
-    engine holds after evaluating it, for both calibrated distributions."""
-    import fmms_b200 as fx
-    from fmms_b200.serve import ENGINE_BYTES_PER_BODY, SESSION_FIXED_BYTES
-
-    for mass, pos in (fx.gen_plummer_ic(n, 1.0, 1.0, 20.0, 3)[:2], fx.gen_uniform_lognormal(n, seed=3)):
-        g = fx.Fmm(mass, pos, 8, 0.0, 64, mac="theta", theta=0.5, softening=1e-3, precision="mixed")
-        g.run()
-        assert g.stats()["device_bytes"] <= n * ENGINE_BYTES_PER_BODY + SESSION_FIXED_BYTES
