@@ -74,8 +74,11 @@ from collections import deque
 import numpy as np
 
 # Device bytes per body kept resident (pos, vel, acc, pot, mass, dt: 12 FP64) and
-# the engine's working memory per body of a forest evaluation (tree, expansions,
-# lists) at p=8, leaf 64 with headroom; plus a fixed part per session.
+# what admission charges for the engine's working memory per body of a forest
+# evaluation (tree, expansions, lists), plus a fixed part per session. At p=8, leaf 64
+# the engine holds 960 to 1,200 B a body of Plummer systems and 620 to 1,720 of uniform
+# ones (2e4 to 1e6 bodies, most where leaves have just split): the charge is low, and
+# budget_bytes has to leave room for the difference.
 RESIDENT_BYTES_PER_BODY = 96
 ENGINE_BYTES_PER_BODY = 640
 SESSION_FIXED_BYTES = 1 << 20
