@@ -97,13 +97,14 @@ struct CellsView {
 // grid-stride and persistent kernels are multiples of it)
 inline int g_nsm = 148;
 
-// Allows a kernel whose shared memory depends on the order as much as any order
-// needs. The limit belongs to the device and the kernel, not to the launch, so it
+// Allows a kernel that needs `need` bytes of shared memory, depending on the order,
+// as much as any order needs (up to 48 KB nothing has to be allowed). The limit belongs to the device and the kernel, not to the launch, so it
 // has to be the same whoever sets it: contexts of other orders launch from other
 // threads.
 #define FMMX_SMEM_MOST (200 * 1024)
 template <class Kernel>
-static inline cudaError_t allow_smem(Kernel* kern) {
+static inline cudaError_t allow_smem(Kernel* kern, size_t need) {
+    if (need <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FMMX_SMEM_MOST);
 }
 

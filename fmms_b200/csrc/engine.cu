@@ -877,8 +877,8 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
         const int warps = 2;  // the P2M tables take 35 KB of shared memory per warp at p = 10
         const size_t smem = (size_t)warps * upward_exact_smem_per_warp(p);
         const size_t smem_b = 16 * (size_t)dim * sizeof(zd);
-        CK(allow_smem(k_upward_exact), "attr");
-        CK(allow_smem(k_m2m_exact_block), "attr");
+        CK(allow_smem(k_upward_exact, smem), "attr");
+        CK(allow_smem(k_m2m_exact_block, smem_b), "attr");
         // the leaves' P2M (a warp per leaf), then level by level the internal
         // cells' M2M (a block per cell, a wide one where a level has few)
         k_upward_exact<<<std::min<unsigned>((nc + warps - 1) / warps, 16u * (unsigned)ctx->nsm), 32 * warps, smem, s>>>(
@@ -954,7 +954,7 @@ fmmx_status evaluate_impl(fmmx_ctx* ctx, const double* d_pos, const double* d_ma
             CK(launch_rotw_f64(p, lm, nc, cv, ctx->moments.p, ctx->locals.p, work, ctx->nsm, s), "m2l");
         } else if (ch == M2L_ROT_BLOCK) {
             const size_t smem = m2l_rot_smem_bytes(p);
-            CK(allow_smem(k_m2l_rot_f64), "attr");
+            CK(allow_smem(k_m2l_rot_f64, smem), "attr");
             k_m2l_rot_f64<<<g, 128, smem, s>>>(lm, nc, cv, p, ctx->moments.p, ctx->locals.p, ctx->swap_dev.p);
         } else {
             const size_t smem = 2 * (size_t)dim * sizeof(zd);

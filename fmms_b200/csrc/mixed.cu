@@ -409,9 +409,6 @@ void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, C
                          const double* ell, const double* x, const double* y, const double* z, const double* m, int p,
                          zf* mom, unsigned* arrive) {
     const int H = (p + 1) * (p + 2) / 2, F2 = (p + 1) * (p + 1);
-    allow_smem(k_p2m_mixed<float>);
-    allow_smem(k_p2m_mixed<double>);
-    allow_smem(k_m2m_mixed);
     auto warps = [&](size_t col) {  // per block: as many as its columns leave room for, 1 .. 4
         int w = 4;
         while (w > 1 && w * col > FMMX_SMEM_MOST) w >>= 1;
@@ -419,10 +416,13 @@ void launch_upward_mixed(cudaStream_t s, const int32_t* top, int ntop, int nc, C
     };
     const size_t cf = (size_t)32 * H * sizeof(zf), cd = (size_t)32 * H * sizeof(zd);
     const int wf = warps(cf), wd = warps(cd);
+    allow_smem(k_p2m_mixed<float>, wf * cf);
+    allow_smem(k_p2m_mixed<double>, wd * cd);
     k_p2m_mixed<double><<<grid_for(ntop, wd), 32 * wd, wd * cd, s>>>(top, ntop, true, cv, ell, x, y, z, m, p, mom);
     if (nc > ntop)
         k_p2m_mixed<float><<<grid_for(nc, wf), 32 * wf, wf * cf, s>>>(nullptr, nc, false, cv, ell, x, y, z, m, p, mom);
     const size_t sm = 8 * (size_t)(F2 + H) * sizeof(zd) + 8 * (size_t)F2 * sizeof(zf);
+    allow_smem(k_m2m_mixed, sm);
     if (nc > 1)
         k_m2m_mixed<<<grid_for(nc, M2M_SCAN), M2M_BLOCK, sm, s>>>(nc, cv, parent, ell, p, mom, arrive);
 }
@@ -573,12 +573,12 @@ void launch_l2l_mixed(bool fp64, unsigned grid, cudaStream_t s, const int32_t* l
     const unsigned blocks = std::max(1u, std::min(grid, (unsigned)((lcnt + L2LB_WARPS - 1) / L2LB_WARPS)));
     if (fp64) {
         const size_t sm = l2l_smem<double>(p);
-        allow_smem(k_l2l_mixed<double>);
+        allow_smem(k_l2l_mixed<double>, sm);
         k_l2l_mixed<double><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
                                                                loc);
     } else {
         const size_t sm = l2l_smem<float>(p);
-        allow_smem(k_l2l_mixed<float>);
+        allow_smem(k_l2l_mixed<float>, sm);
         k_l2l_mixed<float><<<blocks, L2LB_WARPS * 32, sm, s>>>(level_cells, lstart, lcnt, cv, parent, ell, p, sched,
                                                                loc);
     }
